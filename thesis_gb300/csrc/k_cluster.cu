@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "host.hpp"
+#include "reg2d_body.cuh"
 
 namespace st {
 
@@ -467,6 +468,71 @@ __global__ void __launch_bounds__(kClusterThreads)
     }
 }
 
+// Batches of small 2-D grids on single CTAs (clusters of one): each grid in
+// the registers of one CTA (reg2d_body.cuh), one CTA per SM, job indices from
+// *queue.
+constexpr int kRegThreads = 384;
+
+// Grids whose two border bands differ, which one register state cannot hold.
+__device__ __noinline__ void reg2d_general(const ClusterJob &j) {
+    const float *src = j.a;
+    float *dst = j.b;
+    for (int it = 0; it < j.iters; ++it) {
+        sweep_rows2d<1>(src, dst, 0, 0, j.ny, j);
+        __syncthreads();
+        const float *t = src;
+        src = dst;
+        dst = const_cast<float *>(t);
+    }
+}
+
+template <int LW, int RW>
+__device__ __forceinline__ void reg2d_job(const ClusterJob &j, Reg2dHalo<kRegThreads> &halo) {
+    if (j.nx % 4) reg2d_sweeps<LW, RW, kRegThreads, true>(j.a, j.b, j.nx, j.ny, j.px, j.iters, halo);
+    else reg2d_sweeps<LW, RW, kRegThreads, false>(j.a, j.b, j.nx, j.ny, j.px, j.iters, halo);
+}
+
+__global__ void __launch_bounds__(kRegThreads, 1)
+    k_reg2d(const ClusterJob *__restrict__ jobs, int njobs, unsigned *queue) {
+    __shared__ Reg2dHalo<kRegThreads> halo;
+    __shared__ int s_job;
+    for (;;) {
+        if (threadIdx.x == 0) s_job = (int)atomicAdd(queue, 1u);
+        __syncthreads();
+        const int jid = s_job;
+        __syncthreads();
+        if (jid >= njobs) break;
+        const ClusterJob j = jobs[jid];
+        if (!reg2d_borders_equal(j.a, j.b, j.nx, j.ny, j.px)) {
+            reg2d_general(j);
+            continue;
+        }
+        if (j.px <= 64) {  // 24 blocks of rows, two per warp
+            const int rows = (j.ny - 1 + 23) / 24;
+            if (rows <= 3) reg2d_job<16, 3>(j, halo);
+            else if (rows <= 4) reg2d_job<16, 4>(j, halo);
+            else if (rows <= 6) reg2d_job<16, 6>(j, halo);
+            else if (rows <= 8) reg2d_job<16, 8>(j, halo);
+            else reg2d_job<16, 11>(j, halo);
+        } else {  // 12 blocks
+            const int rows = (j.ny - 1 + 11) / 12;
+            if (rows <= 6) reg2d_job<32, 6>(j, halo);
+            else if (rows <= 7) reg2d_job<32, 7>(j, halo);
+            else if (rows <= 8) reg2d_job<32, 8>(j, halo);
+            else if (rows <= 9) reg2d_job<32, 9>(j, halo);
+            else if (rows <= 10) reg2d_job<32, 10>(j, halo);
+            else reg2d_job<32, 11>(j, halo);
+        }
+    }
+}
+
+// The grids k_reg2d takes: R = 1, JACOBI, at most 133 rows of up to 128 cells,
+// or 265 of up to 64 (11 rows per block).
+static bool reg2d_takes(const ClusterJob &j) {
+    return j.dims == 2 && j.radius == 1 && !j.legacy &&
+           ((j.px <= 64 && j.ny <= 265) || (j.px <= 128 && j.ny <= 133));
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -666,6 +732,8 @@ struct BatchHeader {
     int njobs;
     int cluster_size;
     int clusters;
+    int reg_jobs;        // of the njobs, the last ones: grids of k_reg2d
+    unsigned reg_queue;
 };
 
 // A job too large for a cluster's shared memory: swept by the whole GPU
@@ -1146,10 +1214,16 @@ extern "C" int stencil_batch_prepare_engine(const stencil_batch_job *jobs, int n
     std::vector<int> order(nc);
     for (int i = 0; i < nc; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work[x] > work[y]; });
+    // On clusters of one CTA the small 2-D grids go to k_reg2d, a launch of
+    // its own, last in the table.
+    auto in_regs = [&](int i) { return csize == 1 && reg2d_takes(table[i]); };
+    const auto reg0 = std::stable_partition(order.begin(), order.end(), [&](int i) { return !in_regs(i); });
     std::vector<ClusterJob> sorted(nc);
     for (int i = 0; i < nc; ++i) sorted[i] = table[order[i]];
     BatchHeader &h = plan.h;
     h.queue = 0;
+    h.reg_queue = 0;
+    h.reg_jobs = (int)(order.end() - reg0);
     h.njobs = nc;
     h.cluster_size = csize;
     h.clusters = max_active_clusters(csize);
@@ -1183,9 +1257,18 @@ extern "C" int stencil_batch_launch(const void *d_workspace, stencil_stream_t st
     if (h.njobs) {
         const size_t hb = (sizeof(BatchHeader) + 255) & ~(size_t)255;
         const ClusterJob *table = reinterpret_cast<const ClusterJob *>(static_cast<const char *>(d_workspace) + hb);
-        unsigned *queue = reinterpret_cast<unsigned *>(const_cast<void *>(d_workspace));
-        int rc = launch_cluster_jobs(table, h.njobs, queue, std::min(h.clusters, h.njobs), h.cluster_size, s);
-        if (rc) return rc;
+        BatchHeader *dh = reinterpret_cast<BatchHeader *>(const_cast<void *>(d_workspace));
+        const int nc = h.njobs - h.reg_jobs;
+        if (h.reg_jobs) {
+            ST_CUDA(cudaMemsetAsync(&dh->reg_queue, 0, sizeof(unsigned), s));
+            k_reg2d<<<std::min(h.reg_jobs, num_sms()), kRegThreads, 0, s>>>(table + nc, h.reg_jobs,
+                                                                               &dh->reg_queue);
+            ST_CUDA(cudaGetLastError());
+        }
+        if (nc) {
+            int rc = launch_cluster_jobs(table, nc, &dh->queue, std::min(h.clusters, nc), h.cluster_size, s);
+            if (rc) return rc;
+        }
     }
     for (const BatchPlan::Phase &ph : plan.phases) {
         if (ph.queue.size() == 1) {
@@ -1263,7 +1346,7 @@ extern "C" int stencil_batch_launches(const void *d_workspace, int *kernel_launc
     BatchPlan plan;
     if (!recall(d_workspace, &plan))
         return fail(STENCIL_EINVAL, "workspace was not prepared by stencil_batch_prepare");
-    *kernel_launches = (plan.h.njobs ? 1 : 0) + (int)plan.streamed.size() + (plan.nstaged ? 2 : 0);
+    *kernel_launches = (plan.h.njobs > plan.h.reg_jobs ? 1 : 0) + (plan.h.reg_jobs ? 1 : 0) + (int)plan.streamed.size() + (plan.nstaged ? 2 : 0);
     return STENCIL_OK;
 }
 
