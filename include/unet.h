@@ -64,13 +64,14 @@ UNET_API int unet_conv3x3_wgrad(const unet_act *x, const unet_act *dy, float *dw
  * same dilation. */
 UNET_API int unet_conv3x3_wgrad_dil(const unet_act *x, const unet_act *dy, float *dw, float *db,
                                     int dilation, stencil_stream_t stream);
-/* Bytes of device workspace the tcgen05 weight gradient needs for these
- * views: channel-major copies of x (three, shifted by -dilation, 0 and
- * +dilation columns) and of dy: (3 x->c + dy->c) * n * h * w * 2. */
+/* Bytes of the device workspace that engine 1 below asks for:
+ * (3 x->c + dy->c) * n * h * w * 2. */
 UNET_API int unet_wgrad_workspace_bytes(const unet_act *x, const unet_act *dy, size_t *bytes);
 /* The weight gradient on a chosen engine: 1 = tcgen05 (TMEM accumulator,
- * TMA-fed operands; needs w % 32 == 0 and a 256-byte aligned workspace of
- * unet_wgrad_workspace_bytes), 2 = mma.sync, 0 = tcgen05 where it applies.
+ * TMA-fed operands; asks for w % 32 == 0 and a 256-byte aligned workspace of
+ * unet_wgrad_workspace_bytes, which it no longer uses), 2 = mma.sync, 0 =
+ * tcgen05 for any width (workspace may be NULL) where the channels are
+ * multiples of 32 and the dilation is below about 20, else mma.sync.
  * Same accumulation contract as unet_conv3x3_wgrad_dil (FP32 atomics). */
 UNET_API int unet_conv3x3_wgrad_engine(const unet_act *x, const unet_act *dy, float *dw, float *db,
                                        int dilation, int engine, void *workspace,

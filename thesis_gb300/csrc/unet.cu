@@ -539,95 +539,150 @@ constexpr int tma_smem_bytes() {
 
 // ---------------------------------------------------------------------------
 // Weight gradient on tcgen05:
-//   dW[co][tap][ci] += sum_p dy[p][co] x[p + tap][ci]
-// as per-tap GEMMs D[co][ci] (M = 128 output channels, N = BN input
-// channels) with K = pixels in 32-pixel chunks (a run of one image row),
-// accumulated in TMEM over the CTA's slice of the pixels and added to dW
-// with FP32 atomics.  Both operands must be K-major (pixels contiguous), so
-// dy and x are first transposed into channel-major copies (k_to_cmajor) in
-// the caller's workspace; a chunk is then one 4-D tensor-map box per operand
-// (the x box shifted by the tap, out-of-bounds zeros = the padding), 64-byte
-// swizzle, the same UMMA descriptors as the forward kernel.  Warps: 0-3
-// epilogue, 4 TMA producer, 5 MMA issuer.
+//   dW[co][tap][ci] += sum_p dy[p][co] x[p + tap][ci],  db[co] += sum_p dy[p][co]
+// as GEMMs with K = pixels, both operands MN-major: channels are innermost in
+// the NHWC views, so a TMA box of 32 channels x a run of pixels of one image
+// row (64-byte swizzle) is an operand as it lands, with no transposed copy.
+// One CTA owns 32 input channels, up to 128 output channels and the three taps
+// of one column shift, and marches down image rows: each input row is loaded
+// once, shifted by -dil, 0 or +dil columns (out-of-bounds zeros are the
+// padding), into a ring of rows; output row y multiplies dy's row with the
+// input rows y - dil, y and y + dil, which are dil ring slots apart: three of
+// the four 32-row blocks of an M = 128 instruction (the fourth reads what lies
+// behind them; its result rows are not used).  The ring's first 2 * dil slots
+// are loaded a second time behind its end, so that the three rows always lie
+// in line.  The accumulator [(tap row, ci)][co] in tensor memory ends in FP32
+// atomics on dW, coalesced over ci.  In the CTAs of the middle shift and the
+// first channel block the idle epilogue warps sum dy's rows for the bias while
+// they are in shared memory.
+// What bounds it: shared-memory reads of the operands (5 to 8 KB per
+// instruction of K = 16) and the latency of one issuing thread, which is why
+// ring positions are counted and never divided (a division per slot made every
+// row cost 3500 cycles).
+// Warps: 0-3 bias and epilogue, 4 and 6 TMA producers (x, dy), 5 MMA issuer.
 // ---------------------------------------------------------------------------
-// out[c][p] = view[p shifted by dx columns][c], zero where the shifted
-// column leaves the image (32 x 32 tiles through shared memory; W % 32 == 0,
-// so a 32-pixel tile lies in one image row).  The shift is applied here, not
-// by the tensor map, because a TMA box may only start at a 16-byte aligned
-// innermost coordinate and the pixels are the innermost dimension.
-__global__ void __launch_bounds__(256) k_to_cmajor(Act a, bf16 *__restrict__ out, long long P, int W, int dx) {
-    // tile: 64 pixels x 32 channels; 16-byte loads (8 channels of a pixel)
-    // and 16-byte stores (8 pixels of a channel)
-    __shared__ __align__(16) bf16 t[32][64 + 8];
-    const long long p0 = (long long)blockIdx.x * 64;
-    const int c0 = blockIdx.y * 32;
-    const int tid = threadIdx.x;
-    {
-        const int r = tid >> 2, q = tid & 3;
-        const long long p = p0 + r;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (p < P) {
-            const int ws = (int)(p % W) + dx;
-            if (ws >= 0 && ws < W)
-                v = *reinterpret_cast<const uint4 *>(a.p + (p + dx) * a.cs + a.co + c0 + 8 * q);
-        }
-        const bf16 *e = reinterpret_cast<const bf16 *>(&v);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t[8 * q + k][r] = e[k];
-    }
-    __syncthreads();
-    {
-        const int c = tid >> 3, q = tid & 7;
-        const long long p = p0 + 8 * q;
-        if (p + 8 <= P) {
-            *reinterpret_cast<uint4 *>(out + (long long)(c0 + c) * P + p) =
-                *reinterpret_cast<const uint4 *>(&t[c][8 * q]);
-        } else {
-            for (int k = 0; k < 8 && p + k < P; ++k) out[(long long)(c0 + c) * P + p + k] = t[c][8 * q + k];
-        }
-    }
+struct WgradRows {
+    int cin, cout, n, H, W, dil;
+    int wp;          // pixels of a row segment (a multiple of 16, at most 128)
+    int rows;        // row segments in all
+    int slices;      // CTAs that share them
+    int nx, nd;      // ring slots of input rows (without the repeated ones) and of dy rows
+    int dslot;       // bytes of a dy slot
+};
+
+__device__ __forceinline__ uint64_t umma_desc_mn64(uint32_t saddr, uint32_t block_bytes) {
+    // MN-major, 64-byte swizzle: 32-element blocks block_bytes apart, groups
+    // of 8 K rows 512 bytes apart, version 1
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(block_bytes >> 4) << 16) |
+           ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
 
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0,
-                                            int c1, int c2, int c3, int c4) {
+// One issuing thread, uniform code: the whole warp runs the loop, so that the
+// compiler keeps addresses, coordinates and descriptors in uniform registers
+// (where TMA and MMA instructions take them), and only the instructions
+// themselves are predicated on the elected lane.  In a branch of one lane
+// every operand is moved to a uniform register first: about 90 cycles an MMA
+// and 200 a TMA load, on the weight gradient of 128 x 128 x 32 channels.
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
+}
+
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
+__device__ __forceinline__ void tc_commit_if(uint32_t on, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-        "r"(c4)
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(on)
         : "memory");
 }
 
-template <int BN>
-__global__ void __launch_bounds__(192)
-    k_wgrad_tma(const __grid_constant__ CUtensorMap gmap, const __grid_constant__ CUtensorMap xmap,
-                float *__restrict__ dw, int cin, int cout, int H, int W, int dil, int chunks_per_cta,
-                long long nchunks) {
-    extern __shared__ __align__(1024) unsigned char wg_smem[];
-    constexpr int A_BYTES = BM * BK * 2;
-    constexpr int B_BYTES = BN * BK * 2;
-    constexpr int STAGE = A_BYTES + B_BYTES;
+__device__ __forceinline__ void mma_f16_if(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+        "r"(acc), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void expect_tx_if(uint32_t on, uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+        "r"(bytes), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
+                                               int c1, int c2, int c3) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %7, 0;\n\t"
+        "@p cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
+                                               int c1, int c2, int c3, int c4) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %8, 0;\n\t"
+        "@p cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(on)
+        : "memory");
+}
+
+// mbar_wait_bounded of a whole warp; its lanes agree on the outcome.
+__device__ __forceinline__ bool warp_wait_bounded(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+
+// A ring position: slot, and the parity of the slot's current use.
+struct RingPos {
+    int slot = 0;
+    uint32_t parity = 0;
+    __device__ __forceinline__ void next(int n) {
+        if (++slot == n) {
+            slot = 0;
+            parity ^= 1;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(224, 2)
+    k_wgrad_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
+                 float *__restrict__ dw, float *__restrict__ db, WgradRows p) {
+    extern __shared__ __align__(1024) unsigned char wr_smem[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
-        (reinterpret_cast<uintptr_t>(wg_smem) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(base + TMA_STAGES * STAGE);
-    uint64_t *empty = full + TMA_STAGES;
-    uint64_t *accd = empty + TMA_STAGES;
+        (reinterpret_cast<uintptr_t>(wr_smem) + 1023) & ~static_cast<uintptr_t>(1023));
+    const int tile = p.wp * 64, dil = p.dil, nx = p.nx, nd = p.nd;
+    unsigned char *xring = base, *dring = base + (size_t)(nx + 3 * dil) * tile;
+    uint64_t *xfull = reinterpret_cast<uint64_t *>(dring + (size_t)nd * p.dslot);
+    uint64_t *xempty = xfull + nx, *dfull = xempty + nx, *dempty = dfull + nd;
+    uint64_t *accd = dempty + nd;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(accd + 1);
     int *bad = reinterpret_cast<int *>(tslot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int co0 = blockIdx.x * BM, ci0 = blockIdx.y * BN;
-    const int tap = blockIdx.z % 9;
-    const long long k0 = (long long)(blockIdx.z / 9) * chunks_per_cta;
-    const int KB = (int)min((long long)chunks_per_cta, nchunks - k0);
-    const int dy = (tap / 3 - 1) * dil;
-    const int rowchunks = W / BK;  // 32-pixel chunks per image row
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+    const int shift = blockIdx.y % 3, ci0 = blockIdx.y / 3 * 32, co0 = blockIdx.z * 128;
+    const int ncols = min(128, p.cout - co0), nb = ncols / 32;
+    const bool bias = db != nullptr && blockIdx.y == 1;
+    const int r0 = (int)((long long)p.rows * blockIdx.x / gridDim.x);
+    const int r1 = (int)((long long)p.rows * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t tcols = ncols <= 32 ? 32 : ncols <= 64 ? 64 : 128;
 
     if (tid == 0) {
-        prefetch_tensormap(&gmap);
         prefetch_tensormap(&xmap);
-        for (int s = 0; s < TMA_STAGES; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
+        prefetch_tensormap(&gmap);
+        for (int s = 0; s < nx; ++s) {
+            mbar_init(&xfull[s], 1);
+            mbar_init(&xempty[s], 1);
+        }
+        for (int s = 0; s < nd; ++s) {
+            mbar_init(&dfull[s], 1);
+            mbar_init(&dempty[s], bias ? 5 : 1);
         }
         mbar_init(accd, 1);
         *bad = 0;
@@ -635,69 +690,126 @@ __global__ void __launch_bounds__(192)
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(BN) : "memory");
+                     "r"(tcols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-
-    if (warp == 4) {
-        if (lane == 0) {
-            for (int k = 0; k < KB; ++k) {
-                const int st = k % TMA_STAGES;
-                if (k >= TMA_STAGES && !mbar_wait_bounded(&empty[st], ((k / TMA_STAGES) - 1) & 1)) {
-                    *bad = 1;
-                    break;
+    // Row segment r: segment column, image and row; a run of segments that
+    // stays in one image's column is processed as one march.
+    if (warp == 4 || warp == 6) {
+        // warp 4 loads the input rows, warp 6 dy's
+        const bool in = warp == 4;
+        const uint32_t on = elect_lane(), ring = smem_u32(in ? xring : dring), full = smem_u32(in ? xfull : dfull);
+        uint64_t *empty = in ? xempty : dempty;
+        const int slots = in ? nx : nd, halo = in ? dil : 0;
+        RingPos q;
+        bool ok = true, wrap = false;  // wrap: the slots have been used before
+        for (int r = r0; r < r1 && ok;) {
+            const int img = r / p.H, y0 = r - img * p.H, y1 = min(p.H, y0 + (r1 - r));
+            const int im = img % p.n, w0 = img / p.n * p.wp, xw = w0 + (shift - 1) * dil;
+            for (int row = y0 - halo; row < y1 + halo; ++row) {
+                if (wrap && !warp_wait_bounded(&empty[q.slot], q.parity ^ 1)) { ok = false; break; }
+                const uint32_t bar = full + 8 * q.slot;
+                if (in) {
+                    const bool twice = q.slot < 2 * dil;
+                    expect_tx_if(on, bar, twice ? 2 * tile : tile);
+                    tma_load_4d_if(on, ring + q.slot * tile, &xmap, bar, ci0, xw, row, im);
+                    if (twice) tma_load_4d_if(on, ring + (nx + q.slot) * tile, &xmap, bar, ci0, xw, row, im);
+                } else {
+                    if (bias) fence_proxy_async();  // the bias warps' reads of the slot before the TMA write
+                    expect_tx_if(on, bar, p.dslot);
+                    tma_load_5d_if(on, ring + q.slot * p.dslot, &gmap, bar, 0, w0, co0 / 32, row, im);
                 }
-                const long long ch = k0 + k;  // chunk = (n, h, 32-pixel run of the row)
-                const int wc = (int)(ch % rowchunks);
-                const long long r = ch / rowchunks;
-                const int h = (int)(r % H), n = (int)(r / H);
-                unsigned char *a = base + st * STAGE;
-                mbar_arrive_expect_tx(&full[st], STAGE);
-                tma_load_4d(a, &gmap, &full[st], wc * BK, h, n, co0);
-                // x copy shifted by this tap's column offset (index tap % 3), row shift by coordinate
-                tma_load_5d(a + A_BYTES, &xmap, &full[st], wc * BK, h + dy, n, ci0, tap % 3);
+                q.next(slots);
+                wrap |= q.slot == 0;
             }
+            r += y1 - y0;
         }
+        if (!ok && on) *bad = 1;
     } else if (warp == 5) {
-        if (lane == 0) {
-            constexpr uint32_t IDESC = umma_idesc<BN>();
-            for (int k = 0; k < KB; ++k) {
-                const int st = k % TMA_STAGES;
-                if (!mbar_wait_bounded(&full[st], (k / TMA_STAGES) & 1)) {
-                    *bad = 1;
-                    break;
-                }
+        // D FP32, A and B BF16, both MN-major, N = ncols, M = 128
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                               ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        const uint64_t adesc = umma_desc_mn64(smem_u32(xring), dil * tile), bdesc = umma_desc_mn64(smem_u32(dring), tile);
+        const uint32_t astep = tile >> 4, bstep = p.dslot >> 4, ks = p.wp / 16;
+        const uint32_t on = elect_lane(), xe = smem_u32(xempty), de = smem_u32(dempty);
+        RingPos got, d;  // the next input row to wait for; dy
+        int first = 0;   // slot of input row y - dil
+        uint32_t acc = 0;
+        bool ok = true;
+        for (int r = r0; r < r1 && ok;) {
+            const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
+            for (int i = -2 * dil; i < np; ++i) {
+                if (!warp_wait_bounded(&xfull[got.slot], got.parity)) { ok = false; break; }
+                got.next(nx);
+                if (i < 0) continue;
+                if (!warp_wait_bounded(&dfull[d.slot], d.parity)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t a = smem_u32(base + st * STAGE), b = a + A_BYTES;
-#pragma unroll
-                for (int j = 0; j < BK / 16; ++j) {
-                    const uint64_t ad = umma_desc_sw64(a + j * 32), bd = umma_desc_sw64(b + j * 32);
-                    const uint32_t acc = (k > 0 || j > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(IDESC), "r"(acc)
-                        : "memory");
+                const uint64_t a = adesc + first * astep, b = bdesc + d.slot * bstep;
+#pragma unroll 4
+                for (uint32_t k = 0; k < ks; ++k) {
+                    mma_f16_if(on, tmem, a + k * 64, b + k * 64, idesc, acc);
+                    acc = 1;
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&empty[st]))
-                             : "memory");
+                tc_commit_if(on, de + 8 * d.slot);
+                tc_commit_if(on, xe + 8 * first);
+                d.next(nd);
+                if (++first == nx) first = 0;
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(accd))
-                         : "memory");
+            if (!ok) break;
+            for (int i = 0; i < 2 * dil; ++i) {
+                tc_commit_if(on, xe + 8 * first);
+                if (++first == nx) first = 0;
+            }
+            r += np;
         }
+        if (!ok && on) *bad = 1;
+        tc_commit_if(on, smem_u32(accd));  // arrives once every MMA issued above has completed
     } else {
+        if (bias) {
+            // thread -> 8 channels (a 16-byte chunk) of every 32nd pixel
+            float s[4][8] = {};
+            const int c = tid & 3;
+            RingPos d;
+            for (int r = r0; r < r1; ++r) {
+                if (!mbar_wait_bounded(&dfull[d.slot], d.parity)) break;
+                const unsigned char *t = dring + d.slot * p.dslot;
+                for (int px = tid >> 2; px < p.wp; px += 32) {
+                    const int off = px * 64 + ((c ^ ((px >> 1) & 3)) << 4);  // 64-byte swizzle
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (k >= nb) break;
+                        const uint4 v = *reinterpret_cast<const uint4 *>(t + k * tile + off);
+                        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float2 f = __bfloat1622float2(h[e]);
+                            s[k][2 * e] += f.x;
+                            s[k][2 * e + 1] += f.y;
+                        }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&dempty[d.slot]);
+                d.next(nd);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    for (int o = 4; o < 32; o <<= 1) s[k][e] += __shfl_xor_sync(0xffffffffu, s[k][e], o);
+                    if (k < nb && lane < 4) atomicAdd(db + co0 + 32 * k + 8 * c + e, s[k][e]);
+                }
+        }
         const bool done = mbar_wait_bounded(accd, 0);
         tc_fence_after();
-        if (done && KB > 0 && !*reinterpret_cast<volatile int *>(bad)) {
-            const int co = co0 + warp * 32 + lane;
-#pragma unroll
-            for (int c = 0; c < BN; c += 8) {
+        if (warp < 3 && done && r1 > r0 && !*reinterpret_cast<volatile int *>(bad)) {
+            // warp = tap row, lane = input channel
+            float *d = dw + ((long long)co0 * 9 + warp * 3 + shift) * p.cin + ci0 + lane;
+            for (int c = 0; c < ncols; c += 8) {
                 uint32_t r[8];
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -705,11 +817,8 @@ __global__ void __launch_bounds__(192)
                       "=r"(r[7])
                     : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (co < cout) {
-                    float *d = dw + ((long long)co * 9 + tap) * cin + ci0 + c;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) atomicAdd(d + e, __uint_as_float(r[e]));
-                }
+                for (int e = 0; e < 8; ++e) atomicAdd(d + (long long)(c + e) * 9 * p.cin, __uint_as_float(r[e]));
             }
         }
     }
@@ -717,7 +826,7 @@ __global__ void __launch_bounds__(192)
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols) : "memory");
     }
 }
 
@@ -1356,52 +1465,74 @@ extern "C" int unet_flip_weights(const void *w, void *wt, int cout, int cin, ste
     return cuda_fail(cudaGetLastError(), "flip launch");
 }
 
-template <int BN>
-int launch_wgrad_tma(const unet_act *x, const unet_act *dy, float *dw, int dil, void *ws, cudaStream_t s) {
+namespace {
+
+// The row-marching weight gradient's plan for a layer; false where the rows
+// of one march do not fit shared memory in segments of 16 pixels (dilations
+// beyond about 20).  Two CTAs share an SM where the rings allow it.
+constexpr int WR_SMEM = 110 * 1024, WR_SMEM_MAX = 220 * 1024;
+bool wgrad_rows_plan(const unet_act *x, const unet_act *dy, int dil, WgradRows *p) {
+    if (x->c % 32 || dy->c % 32 || (long long)x->n * x->h * ((x->w + 15) / 16) >= (1LL << 31)) return false;
+    const int nb = std::min(dy->c, 128) / 32;
+    for (int budget : {WR_SMEM, WR_SMEM_MAX})
+        for (int wp : {128, 64, 32, 16}) {
+            // the shortest segment that covers a row, else the longest that fits
+            if (wp > 16 && wp / 2 >= x->w) continue;
+            wp = std::min(wp, (x->w + 15) / 16 * 16);
+            const int nd = wp * nb > 256 ? 3 : 4, dslot = nb * wp * 64, tile = wp * 64;
+            const int nx = std::min(16, (budget - nd * dslot) / tile - 3 * dil);
+            if (nx < 2 * dil + 2) continue;
+            *p = {x->c, dy->c, x->n, x->h, x->w, dil, wp, (x->w + wp - 1) / wp * x->n * x->h, 1, nx, nd, dslot};
+            // Slices of the rows.  The tensor core truncates: a sum of k
+            // steps of 16 pixels ends about 1.5e-8 k below its exact value
+            // (measured, positive activations), so few slices cost accuracy
+            // and many cost atomics.  About two CTAs per SM for the nine taps
+            // of a 128 x 128 (widths that are multiples of 32) or four for
+            // those of a 64 x 64 channel block.
+            const long long px = (long long)x->n * x->h * x->w;
+            long long blocks, splits, least;  // least pixels of a slice
+            if (x->w % 32 == 0) {
+                blocks = (dy->c + 127) / 128 * (x->c % 128 == 0 ? x->c / 128 : x->c % 64 == 0 ? x->c / 64 : x->c / 32);
+                splits = (2LL * num_sms() + 9 * blocks - 1) / (9 * blocks), least = 512;
+            } else {
+                blocks = (long long)((dy->c + 63) / 64) * ((x->c + 63) / 64);
+                splits = (4LL * num_sms() + 9 * blocks - 1) / (9 * blocks), least = 32;
+            }
+            const long long per = std::max(least, (px + splits - 1) / splits);
+            p->slices = (int)std::max(1LL, std::min((long long)p->rows, (px + per - 1) / per));
+            return true;
+        }
+    return false;
+}
+
+int launch_wgrad_rows(const unet_act *x, const unet_act *dy, float *dw, float *db, const WgradRows &p,
+                      cudaStream_t s) {
     static bool attr[64] = {false};
-    constexpr int SMEM = TMA_STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * TMA_STAGES + 1) * 8 + 16 + 1024;
     const int dev = current_device();
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-        ST_CUDA(cudaFuncSetAttribute(k_wgrad_tma<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        ST_CUDA(cudaFuncSetAttribute(k_wgrad_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, WR_SMEM_MAX + 2048));
         attr[dev] = true;
     }
-    const int cin = x->c, cout = dy->c, H = x->h, W = x->w, N = x->n;
-    const long long P = (long long)N * H * W;
-    // workspace: x as three channel-major copies shifted by -dil, 0, +dil
-    // columns, then dy channel-major
-    bf16 *xT = static_cast<bf16 *>(ws);
-    bf16 *gT = xT + 3LL * cin * P;
-    for (int k = 0; k < 3; ++k)
-        k_to_cmajor<<<dim3((unsigned)((P + 63) / 64), cin / 32), 256, 0, s>>>(
-            to_act(*x), xT + (long long)k * cin * P, P, W, (k - 1) * dil);
-    k_to_cmajor<<<dim3((unsigned)((P + 63) / 64), cout / 32), 256, 0, s>>>(to_act(*dy), gT, P, W, 0);
-    ST_CUDA(cudaGetLastError());
-    CUtensorMap gm, xm;
-    const unsigned long long p2 = (unsigned long long)P * 2;
-    const unsigned long long gd[4] = {(unsigned long long)W, (unsigned long long)H, (unsigned long long)N,
-                                      (unsigned long long)cout};
-    const unsigned long long st[4] = {(unsigned long long)W * 2, (unsigned long long)W * H * 2, p2,
-                                      p2 * (unsigned long long)cin};
-    const unsigned gb[4] = {(unsigned)BK, 1u, 1u, (unsigned)BM};
-    int rc = make_tensor_map_general(&gm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, gT, gd, st, gb,
-                                     CU_TENSOR_MAP_SWIZZLE_64B);
+    CUtensorMap xm, gm;
+    typedef unsigned long long u64;
+    const u64 W = p.W, H = p.H, N = p.n, xc = 2ull * x->c_stride, gc = 2ull * dy->c_stride;
+    const u64 xd[4] = {(u64)p.cin, W, H, N}, xs[3] = {xc, xc * W, xc * W * H};
+    const unsigned xb[4] = {32u, (unsigned)p.wp, 1u, 1u};
+    int rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, static_cast<const bf16 *>(x->ptr) + x->c_off,
+                                     xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
-    const unsigned long long xd[5] = {(unsigned long long)W, (unsigned long long)H, (unsigned long long)N,
-                                      (unsigned long long)cin, 3ull};
-    const unsigned xb[5] = {(unsigned)BK, 1u, 1u, (unsigned)BN, 1u};
-    rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, xT, xd, st, xb,
-                                 CU_TENSOR_MAP_SWIZZLE_64B);
+    // dy's channels in blocks of 32: one box holds every block of a row
+    const u64 gd[5] = {32, W, (u64)p.cout / 32, H, N}, gs[4] = {gc, 64, gc * W, gc * W * H};
+    const unsigned gb[5] = {32u, (unsigned)p.wp, (unsigned)(p.dslot / (p.wp * 64)), 1u, 1u};
+    rc = make_tensor_map_general(&gm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, static_cast<const bf16 *>(dy->ptr) + dy->c_off,
+                                 gd, gs, gb, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
-    const long long nchunks = P / BK;
-    const int tiles = ((cout + BM - 1) / BM) * (cin / BN) * 9;
-    long long splits = (2LL * num_sms() + tiles - 1) / tiles;
-    long long per = (nchunks + splits - 1) / splits;
-    if (per < 16) per = 16;
-    splits = (nchunks + per - 1) / per;
-    dim3 grid((unsigned)((cout + BM - 1) / BM), (unsigned)(cin / BN), (unsigned)(9 * splits));
-    k_wgrad_tma<BN><<<grid, 192, SMEM, s>>>(gm, xm, dw, cin, cout, H, W, dil, (int)per, nchunks);
+    const int smem = (p.nx + 3 * p.dil) * p.wp * 64 + p.nd * p.dslot + 1024 + (2 * (p.nx + p.nd) + 1) * 8 + 16;
+    k_wgrad_rows<<<dim3(p.slices, 3 * (p.cin / 32), (p.cout + 127) / 128), 224, smem, s>>>(xm, gm, dw, db, p);
     return cuda_fail(cudaGetLastError(), "wgrad (tcgen05) launch");
 }
+
+}  // namespace
 
 extern "C" int unet_wgrad_workspace_bytes(const unet_act *x, const unet_act *dy, size_t *bytes) {
     CHECK_VIEW(x);
@@ -1425,18 +1556,9 @@ extern "C" int unet_conv3x3_wgrad_engine(const unet_act *x, const unet_act *dy, 
                       workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
     if (engine == 1 && !fits)
         return fail(STENCIL_EINVAL, "tcgen05 weight gradient needs W %% 32 == 0 and a %zu-byte workspace", need);
-    if (engine == 0) engine = fits ? 1 : 2;
-    if (engine == 1) {
-        const int cin = x->c;
-        int rc = cin % 128 == 0 ? launch_wgrad_tma<128>(x, dy, dw, dilation, workspace, STREAM(s))
-                 : cin % 64 == 0 ? launch_wgrad_tma<64>(x, dy, dw, dilation, workspace, STREAM(s))
-                                 : launch_wgrad_tma<32>(x, dy, dw, dilation, workspace, STREAM(s));
-        if (rc || !db) return rc;
-        const long long P = (long long)x->n * x->h * x->w;
-        dim3 g2((unsigned)std::min<long long>(1024, (P + 255) / 256), (dy->c + 31) / 32);
-        k_bias_grad<<<g2, 256, 0, STREAM(s)>>>(to_act(*dy), db);
-        return cuda_fail(cudaGetLastError(), "bias grad launch");
-    }
+    // tcgen05 wherever the rows of a march fit shared memory
+    WgradRows p;
+    if (engine != 2 && wgrad_rows_plan(x, dy, dilation, &p)) return launch_wgrad_rows(x, dy, dw, db, p, STREAM(s));
     return unet_conv3x3_wgrad_dil(x, dy, dw, db, dilation, s);
 }
 
