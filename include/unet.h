@@ -46,8 +46,8 @@ UNET_API int unet_conv3x3_fwd_dil(const unet_act *x, const void *w, const float 
                                   const unet_act *y, int relu, int dilation, stencil_stream_t stream);
 /* The same convolution on a chosen engine: 1 = tcgen05 (5th-generation tensor
  * cores, FP32 accumulator in tensor memory), 2 = warp-level mma.sync, 0 = the
- * library's default.  Both engines take the same views and weights and agree
- * up to the FP32 summation order before the BF16 rounding. */
+ * library's default (1).  Both engines take the same views and weights and
+ * accumulate in the same order. */
 UNET_API int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const float *b,
                                      const unet_act *y, int relu, int dilation, int engine,
                                      stencil_stream_t stream);

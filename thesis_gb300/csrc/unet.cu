@@ -1,13 +1,14 @@
 // unet.cu -- kernels of the learned-warm-start U-Net (include/unet.h).
 //
 // Convolutions are implicit GEMMs on the BF16 tensor cores with FP32
-// accumulation (warp-level mma.sync.m16n8k16; operands staged in shared
-// memory by cp.async, fragments loaded with ldmatrix):
+// accumulation:
 //   forward / data gradient:  M = pixels, N = output channels, K = 9 x input
-//     channels (taps outer, 32-channel chunks inner), zero padding by
-//     cp.async zero-fill;
-//   weight gradient:          M = output channels, N = input channels, K =
-//     pixels (split across blocks, FP32 atomics), one tap per grid slice.
+//     channels (taps outer, channels inner), zero padding;
+//   weight gradient:          M = input channels of three taps, N = output
+//     channels, K = pixels (split across CTAs, FP32 atomics).
+// The default engine is tcgen05 (TMA-fed, TMEM accumulators); the mma.sync one
+// (cp.async-fed, ldmatrix) is kept as an engine a caller may choose and serves
+// weight gradients that the other does not take.
 // Everything else (pooling, upsampling, ReLU gradient, head, loss, Adam,
 // features) is bandwidth-bound element-wise work on 16-byte vectors.
 #include <cuda_bf16.h>
@@ -170,32 +171,14 @@ __global__ void __launch_bounds__(128)
 // ---------------------------------------------------------------------------
 // 3x3 convolution, forward / data gradient, on the 5th-generation tensor
 // cores: tcgen05.mma (kind::f16, BF16 operands, FP32 accumulator in tensor
-// memory), issued by one thread, completion tracked by tcgen05.commit on an
-// mbarrier per shared-memory stage.
+// memory), completion tracked by tcgen05.commit on mbarriers.
 //   D[128 pixels x BN channels] (TMEM, BN columns) += A[128 x 16] B[BN x 16]^T
-// per instruction; K runs over (tap, 32-channel chunk), two instructions per
-// chunk.  A (the shifted input pixels, zero outside the image) and B (the
-// weights of one tap and chunk) are staged by cp.async into a ring of
-// TC_STAGES buffers in the canonical K-major layout without swizzle: 8-row x
-// 16-byte core matrices, 128 bytes apart along K (leading byte offset) and
-// 512 bytes apart along M/N (stride byte offset).  The epilogue reads the
-// accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = pixels),
-// adds the bias, applies ReLU and stores BF16.  Every mbarrier wait is
-// bounded; a CTA that gives up waits (bounded) for its issued MMAs and frees
-// its TMEM.
+// per instruction; K runs over taps, then channels.  A is the shifted input
+// pixels (zero outside the image), B the weights of one tap.  The epilogue
+// reads the accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 =
+// pixels), adds the bias, applies ReLU and stores BF16.  Every mbarrier wait
+// is bounded.
 // ---------------------------------------------------------------------------
-// shared-memory stages: more for wide tiles, fewer (more resident CTAs) for narrow ones
-template <int BN>
-__host__ __device__ constexpr int tc_stages() { return BN >= 128 ? 6 : (BN >= 64 ? 4 : 3); }
-constexpr int TC_A_BYTES = BM * BK * 2;  // 8 KiB per stage
-
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-    // start address, leading byte offset 128 (K), stride byte offset 512
-    // (M/N), descriptor version 1, no swizzle
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) |
-           ((uint64_t)(512 >> 4) << 32) | (1ull << 46);
-}
-
 template <int BN>
 __device__ __forceinline__ constexpr uint32_t umma_idesc() {
     // D FP32, A and B BF16, both K-major, N = BN, M = 128
@@ -205,229 +188,141 @@ __device__ __forceinline__ constexpr uint32_t umma_idesc() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-template <int BN>
-__global__ void __launch_bounds__(160)
-    k_conv3x3_tc(Act x, const bf16 *__restrict__ w, const float *__restrict__ bias, Act y, int relu,
-                 int dil) {
-    // warps 0-3: cp.async producers, then the epilogue (TMEM lanes 32w..32w+31);
-    // warp 4: one thread issues the MMAs
-    extern __shared__ __align__(1024) unsigned char tc_smem[];
-    constexpr int B_BYTES = BN * BK * 2;
-    constexpr int TC_STAGES = tc_stages<BN>();
-    constexpr int LAG = TC_STAGES - 2;  // chunks in flight per producer before it signals
-    unsigned char *base = reinterpret_cast<unsigned char *>(
-        (reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~static_cast<uintptr_t>(1023));
-    unsigned char *As = base;
-    unsigned char *Bs = base + TC_STAGES * TC_A_BYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(Bs + TC_STAGES * B_BYTES);
-    uint64_t *done = full + TC_STAGES;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + TC_STAGES);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long P = (long long)x.n * x.h * x.w;
-    const long long m0 = (long long)blockIdx.x * BM;
-    const int n0 = blockIdx.y * BN;
-    const int cin = x.c, cout = y.c;
-    const int nc = cin / BK, KB = 9 * nc;
-
-    if (tid == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) {
-            mbar_init(&full[s], 128);
-            mbar_init(&done[s], 1);
-        }
-        fence_mbar_init();
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(BN) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    bool ok = true;
-
-    if (warp < 4) {
-        // ---------------- producers ----------------
-        int a_n[4], a_y[4], a_x[4];
-        bool a_ok[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = (tid + 128 * i) >> 2;
-            const long long p = m0 + row;
-            a_ok[i] = p < P;
-            const long long pp = a_ok[i] ? p : 0;
-            a_x[i] = (int)(pp % x.w);
-            a_y[i] = (int)((pp / x.w) % x.h);
-            a_n[i] = (int)(pp / ((long long)x.w * x.h));
-        }
-        int signalled = 0;  // chunks whose copies this thread has reported complete
-        for (int k = 0; k < KB; ++k) {
-            const int st = k % TC_STAGES;
-            // the MMAs of chunk k - TC_STAGES read this stage last
-            if (k >= TC_STAGES && !mbar_wait_bounded(&done[st], ((k - TC_STAGES) / TC_STAGES) & 1)) {
-                ok = false;
-                break;
-            }
-            const int tap = k / nc, c0 = (k % nc) * BK;
-            const int dy = (tap / 3 - 1) * dil, dx = (tap % 3 - 1) * dil;
-            unsigned char *a = As + st * TC_A_BYTES;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int idx = tid + 128 * i, row = idx >> 2, part = idx & 3;
-                const int yy = a_y[i] + dy, xx = a_x[i] + dx;
-                const bool v = a_ok[i] && yy >= 0 && yy < x.h && xx >= 0 && xx < x.w;
-                const bf16 *src = x.p + (((long long)a_n[i] * x.h + (v ? yy : 0)) * x.w + (v ? xx : 0)) * x.cs +
-                                  x.co + c0 + part * 8;
-                cp_async16(a + (row >> 3) * 512 + part * 128 + (row & 7) * 16, src, v);
-            }
-            unsigned char *b = Bs + st * B_BYTES;
-#pragma unroll
-            for (int i = 0; i < (BN * 4) / 128; ++i) {
-                const int idx = tid + 128 * i, row = idx >> 2, part = idx & 3;
-                const int co = n0 + row;
-                const bool v = co < cout;
-                const bf16 *src = w + ((long long)(v ? co : 0) * 9 + tap) * cin + c0 + part * 8;
-                cp_async16(b + (row >> 3) * 512 + part * 128 + (row & 7) * 16, src, v);
-            }
-            cp_async_commit();
-            if (k >= LAG) {
-                // chunk k - LAG has landed: make it visible to the async proxy, report it
-                asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                mbar_arrive(&full[(k - LAG) % TC_STAGES]);
-                signalled = k - LAG + 1;
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (ok)
-            for (int k = signalled; k < KB; ++k) mbar_arrive(&full[k % TC_STAGES]);
-    } else if (lane == 0) {
-        // ---------------- MMA issuer ----------------
-        constexpr uint32_t IDESC = umma_idesc<BN>();
-        int issued = 0;
-        for (int k = 0; k < KB; ++k) {
-            const int st = k % TC_STAGES;
-            if (!mbar_wait_bounded(&full[st], (k / TC_STAGES) & 1)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t a = smem_u32(As + st * TC_A_BYTES), b = smem_u32(Bs + st * B_BYTES);
-#pragma unroll
-            for (int j = 0; j < BK / 16; ++j) {
-                const uint64_t ad = umma_desc(a + j * 256), bd = umma_desc(b + j * 256);
-                const uint32_t acc = (k > 0 || j > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(IDESC), "r"(acc)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&done[st]))
-                         : "memory");
-            issued = k + 1;
-        }
-        // every issued MMA has completed once the last commit has arrived
-        if (issued > 0 &&
-            !mbar_wait_bounded(&done[(issued - 1) % TC_STAGES], ((issued - 1) / TC_STAGES) & 1))
-            ok = false;
-        if (issued < KB) ok = false;
-    }
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
-    tc_fence_after();
-    if (ok && warp < 4) {
-        const long long p = m0 + warp * 32 + lane;
-#pragma unroll
-        for (int c = 0; c < BN; c += 8) {
-            uint32_t r[8];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                  "=r"(r[7])
-                : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int co = n0 + c;
-            if (p < P && co < cout) {
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    v[e] = __uint_as_float(r[e]) + (bias ? bias[co + e] : 0.f);
-                    if (relu) v[e] = fmaxf(v[e], 0.f);
-                }
-                uint4 q;
-                __nv_bfloat162 h0 = __floats2bfloat162_rn(v[0], v[1]), h1 = __floats2bfloat162_rn(v[2], v[3]);
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(v[4], v[5]), h3 = __floats2bfloat162_rn(v[6], v[7]);
-                q.x = *reinterpret_cast<uint32_t *>(&h0);
-                q.y = *reinterpret_cast<uint32_t *>(&h1);
-                q.z = *reinterpret_cast<uint32_t *>(&h2);
-                q.w = *reinterpret_cast<uint32_t *>(&h3);
-                *reinterpret_cast<uint4 *>(y.p + p * y.cs + y.co + co) = q;
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
-    }
+// One issuing thread, uniform code: the whole warp runs the loop, so that the
+// compiler keeps addresses, coordinates and descriptors in uniform registers
+// (where TMA and MMA instructions take them), and only the instructions
+// themselves are predicated on the elected lane.  In a branch of one lane
+// every operand is moved to a uniform register first: about 90 cycles an MMA
+// and 200 a TMA load, on the weight gradient of 128 x 128 x 32 channels.
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
 }
 
-// ---------------------------------------------------------------------------
-// The same convolution with TMA-fed operands (grids whose 128-pixel tiles are
-// whole image rows or 128-pixel runs of one row: W a power of two, or a
-// multiple of 128).  One thread streams each K chunk as two tensor-map loads
-// -- a 4-D box of 32 channels x the tile's pixels shifted by the tap (its
-// out-of-bounds cells arrive as zeros, which is the convolution's padding)
-// and a 3-D box of the weights -- with 64-byte swizzle, which is the layout
-// the UMMA descriptors below describe; one thread issues the MMAs; 4 warps
-// run the epilogue.  Warps: 0-3 epilogue, 4 TMA producer, 5 MMA issuer.
-// ---------------------------------------------------------------------------
-constexpr int TMA_STAGES = 6;
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 
-__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr) {
-    // K-major, 64-byte swizzle: 8-row groups 512 bytes apart, version 1
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) |
-           (1ull << 46) | (4ull << 61);
-}
-
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0,
-                                            int c1, int c2, int c3) {
+__device__ __forceinline__ void tc_commit_if(uint32_t on, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(on)
         : "memory");
 }
 
-template <int BN>
+__device__ __forceinline__ void mma_f16_if(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+        "r"(acc), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void expect_tx_if(uint32_t on, uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+        "r"(bytes), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
+                                               int c1, int c2) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "@p cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
+                                               int c1, int c2, int c3) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %7, 0;\n\t"
+        "@p cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(on)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
+                                               int c1, int c2, int c3, int c4) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %8, 0;\n\t"
+        "@p cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(on)
+        : "memory");
+}
+
+// mbar_wait_bounded of a whole warp; its lanes agree on the outcome.
+__device__ __forceinline__ bool warp_wait_bounded(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+
+// A ring position: slot, and the parity of the slot's current use.
+struct RingPos {
+    int slot = 0;
+    uint32_t parity = 0;
+    __device__ __forceinline__ void next(int n) {
+        if (++slot == n) {
+            slot = 0;
+            parity ^= 1;
+        }
+    }
+};
+
+// ---------------------------------------------------------------------------
+// Tiles fed by TMA.  A tile is 128 pixels, 128 /
+// tile_w rows of tile_w columns of one image.  One warp streams each K chunk
+// as two tensor-map loads -- a 4-D box of BC channels x the tile's pixels
+// shifted by the tap (its out-of-bounds cells arrive as zeros, which is the
+// convolution's padding and fills tiles that reach past the image) and a 3-D
+// box of the weights -- with a swizzle of BC channels (64 or 128 bytes), which
+// is the layout the UMMA descriptors below describe; one warp issues the
+// MMAs; 4 warps run the epilogue.  Warps: 0-3 epilogue, 4 TMA producer, 5 MMA
+// issuer.  K runs over taps, then channels, in either form.
+// What bounds it: TMA, at about three cycles per box row of 64 or 128 bytes
+// (the input nine times, the weights once per tile), hence 64 channels a row
+// where the layer has them; and, with few tiles, the latency of the K chain.
+// ---------------------------------------------------------------------------
+// K-major descriptor of BC-channel rows (64- or 128-byte swizzle): 8-row
+// groups 8 rows apart, version 1.
+template <int BC>
+__device__ __forceinline__ uint64_t umma_desc_k(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(BC * 16 >> 4) << 32) | (1ull << 46) |
+           ((BC == 64 ? 2ull : 4ull) << 61);
+}
+
+struct ConvTiles {
+    int cin, H, W, tile_w, tiles_x, tiles_y, relu, dil, stages;
+};
+
+template <int BN, int BC>
 __global__ void __launch_bounds__(192)
     k_conv3x3_tma(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-                  const float *__restrict__ bias, Act y, int cin, int H, int W, int tile_w, int relu,
-                  int dil) {
+                  const float *__restrict__ bias, Act y, ConvTiles p) {
     extern __shared__ __align__(1024) unsigned char tm_smem[];
-    constexpr int B_BYTES = BN * BK * 2;
-    constexpr int STAGE = TC_A_BYTES + B_BYTES;
+    constexpr int A_BYTES = BM * BC * 2, STAGE = A_BYTES + BN * BC * 2;
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(tm_smem) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(base + TMA_STAGES * STAGE);
-    uint64_t *empty = full + TMA_STAGES;
-    uint64_t *accd = empty + TMA_STAGES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(base + p.stages * STAGE);
+    uint64_t *empty = full + p.stages;
+    uint64_t *accd = empty + p.stages;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(accd + 1);
     int *bad = reinterpret_cast<int *>(tslot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long m0 = (long long)blockIdx.x * BM;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int n0 = blockIdx.y * BN;
-    const int nc = cin / BK, KB = 9 * nc;
-    // tile origin: image n, row h0, column w0 (tile = 128 / tile_w rows of tile_w pixels)
-    const int n = (int)(m0 / ((long long)H * W));
-    const int h0 = (int)((m0 / W) % H), w0 = (int)(m0 % W);
+    const int nc = p.cin / BC;
+    // tile origin: image n, row h0, column w0
+    const int tx = blockIdx.x % p.tiles_x, t = blockIdx.x / p.tiles_x;
+    const int n = t / p.tiles_y, h0 = t % p.tiles_y * (BM / p.tile_w), w0 = tx * p.tile_w;
 
     if (tid == 0) {
         prefetch_tensormap(&xmap);
         prefetch_tensormap(&wmap);
-        for (int s = 0; s < TMA_STAGES; ++s) {
+        for (int s = 0; s < p.stages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -446,57 +341,51 @@ __global__ void __launch_bounds__(192)
     const uint32_t tmem = *tslot;
 
     if (warp == 4) {
-        if (lane == 0) {
-            for (int k = 0; k < KB; ++k) {
-                const int st = k % TMA_STAGES;
-                if (k >= TMA_STAGES && !mbar_wait_bounded(&empty[st], ((k / TMA_STAGES) - 1) & 1)) {
-                    *bad = 1;
-                    break;
-                }
-                const int tap = k / nc, c0 = (k % nc) * BK;
-                const int dy = (tap / 3 - 1) * dil, dx = (tap % 3 - 1) * dil;
-                unsigned char *a = base + st * STAGE;
-                mbar_arrive_expect_tx(&full[st], STAGE);
-                tma_load_4d(a, &xmap, &full[st], c0, w0 + dx, h0 + dy, n);
-                tma_load_3d(a + TC_A_BYTES, &wmap, &full[st], c0, tap, n0);
+        const uint32_t on = elect_lane(), ring = smem_u32(base), fb = smem_u32(full);
+        RingPos q;
+        bool ok = true, wrap = false;  // wrap: the stages have been used before
+        for (int tap = 0; tap < 9 && ok; ++tap) {
+            const int dy = (tap / 3 - 1) * p.dil, dx = (tap % 3 - 1) * p.dil;
+            for (int c = 0; c < nc; ++c) {
+                if (wrap && !warp_wait_bounded(&empty[q.slot], q.parity ^ 1)) { ok = false; break; }
+                const uint32_t a = ring + q.slot * STAGE, bar = fb + 8 * q.slot;
+                expect_tx_if(on, bar, STAGE);
+                tma_load_4d_if(on, a, &xmap, bar, c * BC, w0 + dx, h0 + dy, n);
+                tma_load_3d_if(on, a + A_BYTES, &wmap, bar, c * BC, tap, n0);
+                q.next(p.stages);
+                wrap |= q.slot == 0;
             }
         }
+        if (!ok && on) *bad = 1;
     } else if (warp == 5) {
-        if (lane == 0) {
-            constexpr uint32_t IDESC = umma_idesc<BN>();
-            for (int k = 0; k < KB; ++k) {
-                const int st = k % TMA_STAGES;
-                if (!mbar_wait_bounded(&full[st], (k / TMA_STAGES) & 1)) {
-                    *bad = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a = smem_u32(base + st * STAGE), b = a + TC_A_BYTES;
+        constexpr uint32_t IDESC = umma_idesc<BN>();
+        const uint32_t on = elect_lane(), eb = smem_u32(empty);
+        const uint64_t ad0 = umma_desc_k<BC>(smem_u32(base)), bd0 = umma_desc_k<BC>(smem_u32(base) + A_BYTES);
+        RingPos q;
+        bool ok = true;
+        uint32_t acc = 0;
+        for (int k = 0; k < 9 * nc; ++k) {
+            if (!warp_wait_bounded(&full[q.slot], q.parity)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t off = q.slot * (STAGE >> 4);
 #pragma unroll
-                for (int j = 0; j < BK / 16; ++j) {
-                    const uint64_t ad = umma_desc_sw64(a + j * 32), bd = umma_desc_sw64(b + j * 32);
-                    const uint32_t acc = (k > 0 || j > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(IDESC), "r"(acc)
-                        : "memory");
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&empty[st]))
-                             : "memory");
+            for (int j = 0; j < BC / 16; ++j) {
+                mma_f16_if(on, tmem, ad0 + off + 2 * j, bd0 + off + 2 * j, IDESC, acc);
+                acc = 1;
             }
-            // arrives once every MMA issued above has completed
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(accd))
-                         : "memory");
+            tc_commit_if(on, eb + 8 * q.slot);
+            q.next(p.stages);
         }
+        if (!ok && on) *bad = 1;
+        tc_commit_if(on, smem_u32(accd));  // arrives once every MMA issued above has completed
     } else {
-        // epilogue warps 0-3: TMEM lanes 32w .. 32w+31 = pixels m0 + 32w + lane
+        // epilogue warps 0-3: TMEM lanes 32w .. 32w+31 = the tile's pixels 32w + lane
         const bool done = mbar_wait_bounded(accd, 0);
         tc_fence_after();
         if (done && !*reinterpret_cast<volatile int *>(bad)) {
-            const long long p = m0 + warp * 32 + lane;
+            const int m = warp * 32 + lane, row = h0 + m / p.tile_w, col = w0 + m % p.tile_w;
+            const bool in = row < p.H && col < p.W;
+            bf16 *out = y.p + (((long long)n * p.H + row) * p.W + col) * y.cs + y.co + n0;
 #pragma unroll
             for (int c = 0; c < BN; c += 8) {
                 uint32_t r[8];
@@ -506,12 +395,11 @@ __global__ void __launch_bounds__(192)
                       "=r"(r[7])
                     : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int co = n0 + c;
                 float v[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    v[e] = __uint_as_float(r[e]) + (bias ? bias[co + e] : 0.f);
-                    if (relu) v[e] = fmaxf(v[e], 0.f);
+                    v[e] = __uint_as_float(r[e]) + (bias ? bias[n0 + c + e] : 0.f);
+                    if (p.relu) v[e] = fmaxf(v[e], 0.f);
                 }
                 uint4 q;
                 __nv_bfloat162 h0v = __floats2bfloat162_rn(v[0], v[1]), h1v = __floats2bfloat162_rn(v[2], v[3]);
@@ -520,7 +408,7 @@ __global__ void __launch_bounds__(192)
                 q.y = *reinterpret_cast<uint32_t *>(&h1v);
                 q.z = *reinterpret_cast<uint32_t *>(&h2v);
                 q.w = *reinterpret_cast<uint32_t *>(&h3v);
-                *reinterpret_cast<uint4 *>(y.p + p * y.cs + y.co + co) = q;
+                if (in) *reinterpret_cast<uint4 *>(out + c) = q;
             }
         }
     }
@@ -532,9 +420,189 @@ __global__ void __launch_bounds__(192)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same convolution for few channels on wide images (rows longer than 64
+// pixels; all the weights of up to 128 output channels in shared memory): one
+// CTA marches down the rows of 128-pixel columns.  Each input row is loaded
+// once with its column halo into a ring of rows; a tap's A operand is the
+// row's slot started dx pixels (rows of 64 bytes) later, so a row serves all
+// nine taps, where the tiled form loads it nine times and the weights once
+// per tile.  Accumulators alternate between two TMEM buffers, so that the
+// epilogue of one row runs under the MMAs of the next.  What bounds it: the
+// operand reads of the MMAs (5 KB of shared memory each for 32 output
+// channels) and HBM.  Warps: 0-3 epilogue, 4 TMA producer, 5 MMA issuer.
+// ---------------------------------------------------------------------------
+struct ConvMarch {
+    int cin, H, W, n, relu, dil;
+    int rows;      // row tiles in all
+    int slots;     // ring slots, each one row of every 32-channel chunk
+    int rowbytes;  // bytes of one chunk's row in a slot
+};
+
 template <int BN>
-constexpr int tma_smem_bytes() {
-    return TMA_STAGES * (TC_A_BYTES + BN * BK * 2) + (2 * TMA_STAGES + 1) * 8 + 16 + 1024;
+__global__ void __launch_bounds__(192)
+    k_conv3x3_march(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+                    const float *__restrict__ bias, Act y, ConvMarch p) {
+    extern __shared__ __align__(1024) unsigned char mc_smem[];
+    constexpr int WT = BN * BK * 2;  // weights of one tap and chunk
+    constexpr uint32_t TCOLS = BN <= 32 ? 64 : BN <= 64 ? 128 : 256;
+    unsigned char *wsm = reinterpret_cast<unsigned char *>(
+        (reinterpret_cast<uintptr_t>(mc_smem) + 1023) & ~static_cast<uintptr_t>(1023));
+    const int nc = p.cin / BK, slot = nc * p.rowbytes, dil = p.dil;
+    unsigned char *ring = wsm + 9 * nc * WT;
+    uint64_t *full = reinterpret_cast<uint64_t *>(ring + p.slots * slot);
+    uint64_t *empty = full + p.slots, *wfull = empty + p.slots, *accf = wfull + 1, *acce = accf + 2;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+    const int n0 = blockIdx.y * BN;
+    const int r0 = (int)((long long)p.rows * blockIdx.x / gridDim.x);
+    const int r1 = (int)((long long)p.rows * (blockIdx.x + 1) / gridDim.x);
+
+    if (tid == 0) {
+        prefetch_tensormap(&xmap);
+        prefetch_tensormap(&wmap);
+        for (int s = 0; s < p.slots; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(wfull, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&accf[s], 1);
+            mbar_init(&acce[s], 4);
+        }
+        fence_mbar_init();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(TCOLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    // Row tile r: column segment, image and row; a run of tiles that stays in
+    // one image's column is one march.
+    if (warp == 4) {
+        const uint32_t on = elect_lane(), rs = smem_u32(ring), ws = smem_u32(wsm), fb = smem_u32(full);
+        const uint32_t rowtx = nc * (128 + 2 * dil) * BK * 2;
+        expect_tx_if(on, smem_u32(wfull), 9 * nc * WT);
+        for (int k = 0; k < 9 * nc; ++k)
+            tma_load_3d_if(on, ws + k * WT, &wmap, smem_u32(wfull), k % nc * BK, k / nc, n0);
+        RingPos q;
+        bool ok = true, wrap = false;  // wrap: the slots have been used before
+        for (int r = r0; r < r1 && ok;) {
+            const int img = r / p.H, y0 = r - img * p.H, y1 = min(p.H, y0 + (r1 - r));
+            const int im = img % p.n, w0 = img / p.n * 128 - dil;
+            for (int row = y0 - dil; row < y1 + dil; ++row) {
+                if (wrap && !warp_wait_bounded(&empty[q.slot], q.parity ^ 1)) { ok = false; break; }
+                const uint32_t bar = fb + 8 * q.slot;
+                expect_tx_if(on, bar, rowtx);
+                for (int c = 0; c < nc; ++c)
+                    tma_load_4d_if(on, rs + q.slot * slot + c * p.rowbytes, &xmap, bar, c * BK, w0, row, im);
+                q.next(p.slots);
+                wrap |= q.slot == 0;
+            }
+            r += y1 - y0;
+        }
+    } else if (warp == 5) {
+        constexpr uint32_t IDESC = umma_idesc<BN>();
+        const uint32_t on = elect_lane(), eb = smem_u32(empty), afb = smem_u32(accf);
+        const uint64_t ad0 = umma_desc_k<BK>(smem_u32(ring)), bd0 = umma_desc_k<BK>(smem_u32(wsm));
+        RingPos got, acc;
+        int first = 0;  // slot of input row y - dil
+        bool ok = warp_wait_bounded(wfull, 0), again = false;
+        for (int r = r0; r < r1 && ok;) {
+            const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
+            for (int i = -2 * dil; i < np; ++i) {
+                if (!warp_wait_bounded(&full[got.slot], got.parity)) { ok = false; break; }
+                got.next(p.slots);
+                if (i < 0) continue;
+                if (again && !warp_wait_bounded(&acce[acc.slot], acc.parity ^ 1)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d = tmem + acc.slot * (TCOLS / 2);
+                uint64_t b = bd0;
+                int s = first;
+                uint32_t more = 0;
+                for (int ty = 0; ty < 3; ++ty) {
+                    const uint64_t arow = ad0 + s * (slot >> 4);
+                    for (int dx = 0; dx < 3; ++dx) {
+                        uint64_t a = arow + dx * dil * (BK * 2 / 16);
+                        for (int c = 0; c < nc; ++c, a += p.rowbytes >> 4, b += WT >> 4) {
+                            mma_f16_if(on, d, a, b, IDESC, more);
+                            mma_f16_if(on, d, a + 2, b + 2, IDESC, 1);
+                            more = 1;
+                        }
+                    }
+                    s += dil;
+                    if (s >= p.slots) s -= p.slots;
+                }
+                tc_commit_if(on, afb + 8 * acc.slot);
+                tc_commit_if(on, eb + 8 * first);
+                acc.next(2);
+                again |= acc.slot == 0;
+                if (++first == p.slots) first = 0;
+            }
+            if (!ok) break;
+            for (int i = 0; i < 2 * dil; ++i) {
+                tc_commit_if(on, eb + 8 * first);
+                if (++first == p.slots) first = 0;
+            }
+            r += np;
+        }
+    } else {
+        RingPos acc;
+        for (int r = r0; r < r1; ++r) {
+            if (!warp_wait_bounded(&accf[acc.slot], acc.parity)) break;
+            tc_fence_after();
+            const int img = r / p.H, row = r - img * p.H, col = img / p.n * 128 + warp * 32 + lane;
+            const bool in = col < p.W;
+            bf16 *out = y.p + (((long long)(img % p.n) * p.H + row) * p.W + col) * y.cs + y.co + n0;
+            const uint32_t t = tmem + ((uint32_t)(warp * 32) << 16) + acc.slot * (TCOLS / 2);
+#pragma unroll
+            for (int c = 0; c < BN; c += 32) {
+                uint32_t v[32];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                    "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
+                    "[%32];"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                      "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+                      "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+                      "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                    : "r"(t + c));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (c + 32 >= BN) {  // read: the buffer may be written again
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acce[acc.slot]);
+                }
+#pragma unroll
+                for (int g = 0; g < 32; g += 8) {
+                    uint4 q;
+                    uint32_t *h = reinterpret_cast<uint32_t *>(&q);
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        float a0 = __uint_as_float(v[g + e]) + (bias ? bias[n0 + c + g + e] : 0.f);
+                        float a1 = __uint_as_float(v[g + e + 1]) + (bias ? bias[n0 + c + g + e + 1] : 0.f);
+                        if (p.relu) a0 = fmaxf(a0, 0.f), a1 = fmaxf(a1, 0.f);
+                        const __nv_bfloat162 b2 = __floats2bfloat162_rn(a0, a1);
+                        h[e / 2] = *reinterpret_cast<const uint32_t *>(&b2);
+                    }
+                    if (in) *reinterpret_cast<uint4 *>(out + c + g) = q;
+                }
+            }
+            acc.next(2);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -576,81 +644,6 @@ __device__ __forceinline__ uint64_t umma_desc_mn64(uint32_t saddr, uint32_t bloc
     return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(block_bytes >> 4) << 16) |
            ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
-
-// One issuing thread, uniform code: the whole warp runs the loop, so that the
-// compiler keeps addresses, coordinates and descriptors in uniform registers
-// (where TMA and MMA instructions take them), and only the instructions
-// themselves are predicated on the elected lane.  In a branch of one lane
-// every operand is moved to a uniform register first: about 90 cycles an MMA
-// and 200 a TMA load, on the weight gradient of 128 x 128 x 32 channels.
-__device__ __forceinline__ uint32_t elect_lane() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p;
-}
-
-__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
-
-__device__ __forceinline__ void tc_commit_if(uint32_t on, uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
-        "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_f16_if(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-        "r"(acc), "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void expect_tx_if(uint32_t on, uint32_t bar, uint32_t bytes) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
-        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
-        "r"(bytes), "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_4d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                               int c1, int c2, int c3) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %7, 0;\n\t"
-        "@p cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_5d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                               int c1, int c2, int c3, int c4) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %8, 0;\n\t"
-        "@p cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(on)
-        : "memory");
-}
-
-// mbar_wait_bounded of a whole warp; its lanes agree on the outcome.
-__device__ __forceinline__ bool warp_wait_bounded(uint64_t *bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
-}
-
-// A ring position: slot, and the parity of the slot's current use.
-struct RingPos {
-    int slot = 0;
-    uint32_t parity = 0;
-    __device__ __forceinline__ void next(int n) {
-        if (++slot == n) {
-            slot = 0;
-            parity ^= 1;
-        }
-    }
-};
 
 __global__ void __launch_bounds__(224, 2)
     k_wgrad_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
@@ -828,11 +821,6 @@ __global__ void __launch_bounds__(224, 2)
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols) : "memory");
     }
-}
-
-template <int BN>
-constexpr int tc_smem_bytes() {
-    return tc_stages<BN>() * (TC_A_BYTES + BN * BK * 2) + 2 * tc_stages<BN>() * 8 + 16 + 1024;
 }
 
 // ---------------------------------------------------------------------------
@@ -1350,62 +1338,118 @@ using namespace st;
     do { int rc_ = check_act(v, #v); if (rc_) return rc_; } while (0)
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 
-template <int BN>
-int launch_conv_tc(const Act &xa, const bf16 *wb, const float *b, const Act &ya, int relu, int dil,
-                   long long P, cudaStream_t s) {
-    static bool attr[64] = {false};
-    const int dev = current_device();
-    if (dev >= 0 && dev < 64 && !attr[dev]) {
-        ST_CUDA(cudaFuncSetAttribute(k_conv3x3_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     tc_smem_bytes<BN>()));
-        attr[dev] = true;
-    }
-    dim3 grid((unsigned)((P + BM - 1) / BM), ya.c / BN);
-    k_conv3x3_tc<BN><<<grid, 160, tc_smem_bytes<BN>(), s>>>(xa, wb, b, ya, relu, dil);
-    return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05) launch");
-}
-
-// Tile shape for the TMA engine: 128 pixels = whole rows (W < 128, a power of
-// two dividing 128, H a multiple of 128 / W) or a 128-pixel run of one row
-// (W a multiple of 128); 0 if neither.
+// Columns of a 128-pixel tile (its rows: 128 over that) that cover an H x W
+// image with the fewest tiles.
 int tma_tile_w(int H, int W) {
-    if (W >= 128) return W % 128 == 0 ? 128 : 0;
-    if (128 % W == 0 && H % (128 / W) == 0) return W;
-    return 0;
+    int best = 128, count = 1 << 30;
+    for (int tw : {128, 64, 32, 16, 8}) {
+        const int th = BM / tw, n = ((W + tw - 1) / tw) * ((H + th - 1) / th);
+        if (n < count) count = n, best = tw;
+    }
+    return best;
 }
 
-template <int BN>
+template <int BN, int BC>
 int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil,
-                    int tile_w, cudaStream_t s) {
+                    cudaStream_t s) {
+    constexpr int STAGE = (BM + BN) * BC * 2, SMEM_MAX = 200 * 1024;
     static bool attr[64] = {false};
     const int dev = current_device();
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-        ST_CUDA(cudaFuncSetAttribute(k_conv3x3_tma<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     tma_smem_bytes<BN>()));
+        ST_CUDA(cudaFuncSetAttribute(k_conv3x3_tma<BN, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     SMEM_MAX + 2048));
         attr[dev] = true;
     }
-    const int cin = x->c, cout = ya.c;
+    const int cin = x->c, cout = ya.c, tw = tma_tile_w(x->h, x->w), th = BM / tw;
     CUtensorMap xm, wm;
     const unsigned long long cs2 = (unsigned long long)x->c_stride * 2;
     const unsigned long long xd[4] = {(unsigned long long)cin, (unsigned long long)x->w,
                                       (unsigned long long)x->h, (unsigned long long)x->n};
     const unsigned long long xs[3] = {cs2, cs2 * x->w, cs2 * x->w * x->h};
-    const unsigned xb[4] = {(unsigned)BK, (unsigned)tile_w, (unsigned)(BM / tile_w), 1u};
+    const unsigned xb[4] = {(unsigned)BC, (unsigned)tw, (unsigned)th, 1u};
     const bf16 *xbase = static_cast<const bf16 *>(x->ptr) + x->c_off;
-    int rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, xbase, xd, xs, xb,
-                                     CU_TENSOR_MAP_SWIZZLE_64B);
+    const CUtensorMapSwizzle swz = BC == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+    int rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, xbase, xd, xs, xb, swz);
     if (rc) return rc;
     const unsigned long long wd[3] = {(unsigned long long)cin, 9ull, (unsigned long long)cout};
     const unsigned long long ws[2] = {(unsigned long long)cin * 2, 9ull * cin * 2};
-    const unsigned wbx[3] = {(unsigned)BK, 1u, (unsigned)BN};
-    rc = make_tensor_map_general(&wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, wb, wd, ws, wbx,
-                                 CU_TENSOR_MAP_SWIZZLE_64B);
+    const unsigned wbx[3] = {(unsigned)BC, 1u, (unsigned)BN};
+    rc = make_tensor_map_general(&wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, wb, wd, ws, wbx, swz);
     if (rc) return rc;
-    const long long P = (long long)x->n * x->h * x->w;
-    dim3 grid((unsigned)(P / BM), cout / BN);
-    k_conv3x3_tma<BN><<<grid, 192, tma_smem_bytes<BN>(), s>>>(xm, wm, b, ya, cin, x->h, x->w, tile_w,
-                                                              relu, dil);
+    ConvTiles p = {cin, x->h, x->w, tw, (x->w + tw - 1) / tw, (x->h + th - 1) / th, relu, dil, 0};
+    const dim3 grid((unsigned)((long long)p.tiles_x * p.tiles_y * x->n), cout / BN);
+    // a lone CTA per SM gets a deep ring; otherwise several share the SM, the
+    // more the fewer channels a tile has (64^2, 64 -> 64: 41 us with two stages,
+    // 48 with four; 32^2, 384 -> 128: 66 us with two, 53 with three)
+    const int budget = (long long)grid.x * grid.y <= num_sms() ? SMEM_MAX : BN == 128 ? 100 * 1024 : 48 * 1024;
+    p.stages = std::max(2, std::min(9 * cin / BC, std::min(8, budget / STAGE)));
+    const int smem = p.stages * STAGE + (2 * p.stages + 1) * 8 + 16 + 1024;
+    k_conv3x3_tma<BN, BC><<<grid, 192, smem, s>>>(xm, wm, b, ya, p);
     return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05, TMA) launch");
+}
+
+template <int BN>
+int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil,
+                    cudaStream_t s) {
+    return x->c % 64 == 0 ? launch_conv_tma<BN, 64>(x, wb, b, ya, relu, dil, s)
+                          : launch_conv_tma<BN, 32>(x, wb, b, ya, relu, dil, s);
+}
+
+// Whether the marching form takes the layer, and its plan: rows of more than
+// 64 pixels (a tile is 128 pixels of one row), two row tiles per SM or more,
+// and weights plus 2 * dil + 2 rows in shared memory.  Six slots let three
+// CTAs share an SM at 32 -> 32 channels (39 us against 43 with eight slots and
+// two CTAs); with 96 outputs one CTA with eight slots is faster than two (93 /
+// 103 us).
+constexpr int CM_SMEM = 200 * 1024;
+template <int BN>
+bool conv_march_plan(const unet_act *x, int relu, int dil, ConvMarch *p) {
+    if (x->w <= 64 || dil > 32) return false;
+    const int nc = x->c / BK, rowbytes = ((128 + 2 * dil) * BK * 2 + 1023) / 1024 * 1024;
+    const int slots = std::min(BN <= 64 ? 6 : 8, (CM_SMEM - 9 * nc * BN * BK * 2) / (nc * rowbytes));
+    if (slots < 2 * dil + 2) return false;
+    const long long rows = (long long)x->n * x->h * ((x->w + 127) / 128);
+    if (rows < 2LL * num_sms() || rows >= (1LL << 31)) return false;
+    *p = {x->c, x->h, x->w, x->n, relu, dil, (int)rows, slots, rowbytes};
+    return true;
+}
+
+template <int BN>
+int launch_conv_march(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const ConvMarch &p,
+                      cudaStream_t s) {
+    static bool attr[64] = {false};
+    const int dev = current_device();
+    if (dev >= 0 && dev < 64 && !attr[dev]) {
+        ST_CUDA(cudaFuncSetAttribute(k_conv3x3_march<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM + 2048));
+        attr[dev] = true;
+    }
+    typedef unsigned long long u64;
+    CUtensorMap xm, wm;
+    const u64 cs2 = 2ull * x->c_stride, cin = x->c;
+    const u64 xd[4] = {cin, (u64)x->w, (u64)x->h, (u64)x->n}, xs[3] = {cs2, cs2 * x->w, cs2 * x->w * x->h};
+    const unsigned xb[4] = {(unsigned)BK, (unsigned)(128 + 2 * p.dil), 1u, 1u};
+    int rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, static_cast<const bf16 *>(x->ptr) + x->c_off,
+                                     xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc) return rc;
+    const u64 wd[3] = {cin, 9, (u64)ya.c}, ws[2] = {cin * 2, 9 * cin * 2};
+    const unsigned wbx[3] = {(unsigned)BK, 1u, (unsigned)BN};
+    rc = make_tensor_map_general(&wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, wb, wd, ws, wbx, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc) return rc;
+    const int nc = p.cin / BK;
+    const int smem = 9 * nc * BN * BK * 2 + p.slots * nc * p.rowbytes + 1024 + (2 * p.slots + 5) * 8 + 16;
+    const int per_sm = std::max(1, std::min(512 / (BN <= 32 ? 64 : BN <= 64 ? 128 : 256), (227 * 1024) / (smem + 1024)));
+    const int ctas = std::max(1, std::min(p.rows, per_sm * num_sms() / (ya.c / BN)));
+    k_conv3x3_march<BN><<<dim3(ctas, ya.c / BN), 192, smem, s>>>(xm, wm, b, ya, p);
+    return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05, rows) launch");
+}
+
+template <int BN>
+int launch_conv(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil, cudaStream_t s) {
+    ConvMarch m;
+    if (conv_march_plan<BN>(x, relu, dil, &m)) return launch_conv_march<BN>(x, wb, b, ya, m, s);
+    // tiles of at most 128 channels whose number divides the layer's
+    if constexpr (BN == 96) return launch_conv_tma<32>(x, wb, b, ya, relu, dil, s);
+    else return launch_conv_tma<BN>(x, wb, b, ya, relu, dil, s);
 }
 
 extern "C" int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const float *b,
@@ -1421,22 +1465,19 @@ extern "C" int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const f
     const long long P = (long long)x->n * x->h * x->w;
     const Act xa = to_act(*x), ya = to_act(*y);
     const bf16 *wb = static_cast<const bf16 *>(w);
-    // default: tcgen05 with TMA-fed operands wherever the tiles allow it
-    // (measured 1.5-3.4x the mma.sync engine on every U-Net layer: 199 vs 129
-    // TFLOP/s at 128^2 x 32 -> 32, 759 vs 222 at 32^2 x 384 -> 128); the
-    // cp.async-fed tcgen05 form is slower than mma.sync (operand staging
-    // bound), so other shapes use mma.sync
-    if (engine == 0) engine = (tma_tile_w(x->h, x->w) && P % BM == 0) ? 1 : 2;
-    if (engine == 1) {
-        const int tw = tma_tile_w(x->h, x->w);
-        if (tw && P % BM == 0) {
-            if (y->c % 128 == 0) return launch_conv_tma<128>(x, wb, b, ya, relu, dilation, tw, STREAM(s));
-            if (y->c % 64 == 0) return launch_conv_tma<64>(x, wb, b, ya, relu, dilation, tw, STREAM(s));
-            return launch_conv_tma<32>(x, wb, b, ya, relu, dilation, tw, STREAM(s));
-        }
-        if (y->c % 128 == 0) return launch_conv_tc<128>(xa, wb, b, ya, relu, dilation, P, STREAM(s));
-        if (y->c % 64 == 0) return launch_conv_tc<64>(xa, wb, b, ya, relu, dilation, P, STREAM(s));
-        return launch_conv_tc<32>(xa, wb, b, ya, relu, dilation, P, STREAM(s));
+    // tcgen05 with TMA-fed operands for every shape (bit for bit the mma.sync
+    // engine's results, 1.6 to 5 times as fast on the U-Net's layers); the
+    // marching form where it fits and its row tiles fill the GPU more than
+    // once (64 x 128^2, us, marching / tiled / mma.sync: 32 -> 32 channels 39 /
+    // 74 / 149, 96 -> 32 96 / 146 / 349, 32 -> 96 93 / 231 / 425; one 128^2
+    // image 8 / 7 / 12)
+    if (engine != 2) {
+        if (y->c == 32) return launch_conv<32>(x, wb, b, ya, relu, dilation, STREAM(s));
+        if (y->c == 96) return launch_conv<96>(x, wb, b, ya, relu, dilation, STREAM(s));
+        if (y->c == 64) return launch_conv<64>(x, wb, b, ya, relu, dilation, STREAM(s));
+        if (y->c % 128 == 0) return launch_conv<128>(x, wb, b, ya, relu, dilation, STREAM(s));
+        if (y->c % 64 == 0) return launch_conv_tma<64>(x, wb, b, ya, relu, dilation, STREAM(s));
+        return launch_conv_tma<32>(x, wb, b, ya, relu, dilation, STREAM(s));
     }
     if (y->c % 64 == 0) {
         dim3 grid((unsigned)((P + BM - 1) / BM), y->c / 64);
