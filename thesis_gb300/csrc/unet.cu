@@ -620,22 +620,30 @@ __global__ void __launch_bounds__(192)
 // behind them; its result rows are not used).  The ring's first 2 * dil slots
 // are loaded a second time behind its end, so that the three rows always lie
 // in line.  The accumulator [(tap row, ci)][co] in tensor memory ends in FP32
-// atomics on dW, coalesced over ci.  In the CTAs of the middle shift and the
-// first channel block the idle epilogue warps sum dy's rows for the bias while
-// they are in shared memory.
-// What bounds it: shared-memory reads of the operands (5 to 8 KB per
-// instruction of K = 16) and the latency of one issuing thread, which is why
-// ring positions are counted and never divided (a division per slot made every
-// row cost 3500 cycles).
-// Warps: 0-3 bias and epilogue, 4 and 6 TMA producers (x, dy), 5 MMA issuer.
+// atomics on dW, coalesced over ci.  In the CTAs of the first channel block the
+// idle epilogue warps sum every third row of dy for the bias while it is in
+// shared memory (all rows in the CTAs of one shift made those the slowest: 119
+// us against 86 on 64 x 128^2, 32 -> 32 channels; rows shared out over all
+// channel blocks' CTAs cost more in atomics on the few bias words).
+// A step loads rs input rows and the rs rows of dy that they complete (about
+// 128 pixels by two 32-channel blocks), with one barrier to wait for and one
+// commit, since a wait and a commit cost the issuing warp some 200 cycles.
+// What bounds it: the issue of eight MMAs per 128 pixels of a row (5 to 8 KB
+// of operands each) behind those, and the few slices of the widest layers.
+// Ring positions are counted and never divided (a division per slot made every
+// row cost 3500 cycles).  Measured and not kept: dy by cp.async or through
+// registers from the idle warps (64 x 128^2, 32 -> 32 channels: 281 and 270 us
+// where both operands by TMA took 127).
+// Warps: 0-3 bias and epilogue, 4 TMA producer, 5 MMA issuer.
 // ---------------------------------------------------------------------------
 struct WgradRows {
     int cin, cout, n, H, W, dil;
-    int wp;          // pixels of a row segment (a multiple of 16, at most 128)
+    int wp, rs;      // a step: rs rows of segments of wp pixels (a multiple of 16, at most 128)
     int rows;        // row segments in all
     int slices;      // CTAs that share them
-    int nx, nd;      // ring slots of input rows (without the repeated ones) and of dy rows
-    int dslot;       // bytes of a dy slot
+    int stages;      // steps in flight
+    int lag;         // steps between a row's arrival and its last use
+    int dslot;       // bytes of a step of dy
 };
 
 __device__ __forceinline__ uint64_t umma_desc_mn64(uint32_t saddr, uint32_t block_bytes) {
@@ -645,23 +653,24 @@ __device__ __forceinline__ uint64_t umma_desc_mn64(uint32_t saddr, uint32_t bloc
            ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
 
-__global__ void __launch_bounds__(224, 2)
+__global__ void __launch_bounds__(192, 2)
     k_wgrad_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
                  float *__restrict__ dw, float *__restrict__ db, WgradRows p) {
     extern __shared__ __align__(1024) unsigned char wr_smem[];
+    __shared__ float bsum[4][128];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(wr_smem) + 1023) & ~static_cast<uintptr_t>(1023));
-    const int tile = p.wp * 64, dil = p.dil, nx = p.nx, nd = p.nd;
-    unsigned char *xring = base, *dring = base + (size_t)(nx + 3 * dil) * tile;
-    uint64_t *xfull = reinterpret_cast<uint64_t *>(dring + (size_t)nd * p.dslot);
-    uint64_t *xempty = xfull + nx, *dfull = xempty + nx, *dempty = dfull + nd;
-    uint64_t *accd = dempty + nd;
+    const int tile = p.wp * 64, dil = p.dil, rs = p.rs, nst = p.stages, nx = nst + p.lag;
+    unsigned char *xring = base, *dring = base + (size_t)((nx + p.lag) * rs + dil) * tile;
+    uint64_t *full = reinterpret_cast<uint64_t *>(dring + (size_t)nst * p.dslot);
+    uint64_t *empty = full + nst, *accd = empty + nst;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(accd + 1);
     int *bad = reinterpret_cast<int *>(tslot + 1);
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int shift = blockIdx.y % 3, ci0 = blockIdx.y / 3 * 32, co0 = blockIdx.z * 128;
     const int ncols = min(128, p.cout - co0), nb = ncols / 32;
-    const bool bias = db != nullptr && blockIdx.y == 1;
+    const int drow = p.dslot / rs;  // bytes of a row of dy
+    const bool bias = db != nullptr && ci0 == 0;
     const int r0 = (int)((long long)p.rows * blockIdx.x / gridDim.x);
     const int r1 = (int)((long long)p.rows * (blockIdx.x + 1) / gridDim.x);
     const uint32_t tcols = ncols <= 32 ? 32 : ncols <= 64 ? 64 : 128;
@@ -669,13 +678,9 @@ __global__ void __launch_bounds__(224, 2)
     if (tid == 0) {
         prefetch_tensormap(&xmap);
         prefetch_tensormap(&gmap);
-        for (int s = 0; s < nx; ++s) {
-            mbar_init(&xfull[s], 1);
-            mbar_init(&xempty[s], 1);
-        }
-        for (int s = 0; s < nd; ++s) {
-            mbar_init(&dfull[s], 1);
-            mbar_init(&dempty[s], bias ? 5 : 1);
+        for (int s = 0; s < nst; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], bias ? 5 : 1);
         }
         mbar_init(accd, 1);
         *bad = 0;
@@ -691,32 +696,29 @@ __global__ void __launch_bounds__(224, 2)
     tc_fence_after();
     const uint32_t tmem = *tslot;
     // Row segment r: segment column, image and row; a run of segments that
-    // stays in one image's column is processed as one march.
-    if (warp == 4 || warp == 6) {
-        // warp 4 loads the input rows, warp 6 dy's
-        const bool in = warp == 4;
-        const uint32_t on = elect_lane(), ring = smem_u32(in ? xring : dring), full = smem_u32(in ? xfull : dfull);
-        uint64_t *empty = in ? xempty : dempty;
-        const int slots = in ? nx : nd, halo = in ? dil : 0;
+    // stays in one image's column (output rows y0 .. y1 - 1) is one march.
+    // Its step g brings input rows y0 - dil + g * rs ... and dy's rows that
+    // these complete, y0 - 2 * dil + g * rs ..., of which the ones in the
+    // march are used.
+    if (warp == 4) {
+        const uint32_t on = elect_lane(), xs = smem_u32(xring), ds = smem_u32(dring), fb = smem_u32(full);
         RingPos q;
-        bool ok = true, wrap = false;  // wrap: the slots have been used before
+        int xslot = 0;
+        bool ok = true, wrap = false;  // wrap: the stages have been used before
         for (int r = r0; r < r1 && ok;) {
             const int img = r / p.H, y0 = r - img * p.H, y1 = min(p.H, y0 + (r1 - r));
             const int im = img % p.n, w0 = img / p.n * p.wp, xw = w0 + (shift - 1) * dil;
-            for (int row = y0 - halo; row < y1 + halo; ++row) {
+            for (int row = y0 - dil; row < y1 + dil; row += rs) {
                 if (wrap && !warp_wait_bounded(&empty[q.slot], q.parity ^ 1)) { ok = false; break; }
-                const uint32_t bar = full + 8 * q.slot;
-                if (in) {
-                    const bool twice = q.slot < 2 * dil;
-                    expect_tx_if(on, bar, twice ? 2 * tile : tile);
-                    tma_load_4d_if(on, ring + q.slot * tile, &xmap, bar, ci0, xw, row, im);
-                    if (twice) tma_load_4d_if(on, ring + (nx + q.slot) * tile, &xmap, bar, ci0, xw, row, im);
-                } else {
-                    if (bias) fence_proxy_async();  // the bias warps' reads of the slot before the TMA write
-                    expect_tx_if(on, bar, p.dslot);
-                    tma_load_5d_if(on, ring + q.slot * p.dslot, &gmap, bar, 0, w0, co0 / 32, row, im);
-                }
-                q.next(slots);
+                if (bias) fence_proxy_async();  // the bias warps' reads of the slot before the TMA write
+                const uint32_t bar = fb + 8 * q.slot;
+                const bool twice = xslot < p.lag;
+                expect_tx_if(on, bar, p.dslot + (twice ? 2 : 1) * rs * tile);
+                tma_load_4d_if(on, xs + xslot * rs * tile, &xmap, bar, ci0, xw, row, im);
+                tma_load_5d_if(on, ds + q.slot * p.dslot, &gmap, bar, 0, w0, co0 / 32, row - dil, im);
+                if (twice) tma_load_4d_if(on, xs + (nx + xslot) * rs * tile, &xmap, bar, ci0, xw, row, im);
+                if (++xslot == nx) xslot = 0;
+                q.next(nst);
                 wrap |= q.slot == 0;
             }
             r += y1 - y0;
@@ -727,35 +729,31 @@ __global__ void __launch_bounds__(224, 2)
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
         const uint64_t adesc = umma_desc_mn64(smem_u32(xring), dil * tile), bdesc = umma_desc_mn64(smem_u32(dring), tile);
-        const uint32_t astep = tile >> 4, bstep = p.dslot >> 4, ks = p.wp / 16;
-        const uint32_t on = elect_lane(), xe = smem_u32(xempty), de = smem_u32(dempty);
-        RingPos got, d;  // the next input row to wait for; dy
-        int first = 0;   // slot of input row y - dil
+        const uint32_t astep = tile >> 4, ks = p.wp / 16, on = elect_lane(), fb = smem_u32(empty);
+        RingPos q;
+        int xslot = 0;
         uint32_t acc = 0;
         bool ok = true;
         for (int r = r0; r < r1 && ok;) {
             const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
-            for (int i = -2 * dil; i < np; ++i) {
-                if (!warp_wait_bounded(&xfull[got.slot], got.parity)) { ok = false; break; }
-                got.next(nx);
-                if (i < 0) continue;
-                if (!warp_wait_bounded(&dfull[d.slot], d.parity)) { ok = false; break; }
+            int first = xslot * rs;  // ring row of input row y - dil
+            for (int i = -2 * dil; i < np; i += rs) {
+                if (!warp_wait_bounded(&full[q.slot], q.parity)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t a = adesc + first * astep, b = bdesc + d.slot * bstep;
+                uint64_t b = bdesc + q.slot * (p.dslot >> 4);
+                for (int j = i; j < i + rs; ++j, b += drow >> 4) {
+                    if (j < 0 || j >= np) continue;
+                    const uint64_t a = adesc + first * astep;
 #pragma unroll 4
-                for (uint32_t k = 0; k < ks; ++k) {
-                    mma_f16_if(on, tmem, a + k * 64, b + k * 64, idesc, acc);
-                    acc = 1;
+                    for (uint32_t k = 0; k < ks; ++k) {
+                        mma_f16_if(on, tmem, a + k * 64, b + k * 64, idesc, acc);
+                        acc = 1;
+                    }
+                    if (++first == nx * rs) first = 0;
                 }
-                tc_commit_if(on, de + 8 * d.slot);
-                tc_commit_if(on, xe + 8 * first);
-                d.next(nd);
-                if (++first == nx) first = 0;
-            }
-            if (!ok) break;
-            for (int i = 0; i < 2 * dil; ++i) {
-                tc_commit_if(on, xe + 8 * first);
-                if (++first == nx) first = 0;
+                tc_commit_if(on, fb + 8 * q.slot);
+                if (++xslot == nx) xslot = 0;
+                q.next(nst);
             }
             r += np;
         }
@@ -763,39 +761,57 @@ __global__ void __launch_bounds__(224, 2)
         tc_commit_if(on, smem_u32(accd));  // arrives once every MMA issued above has completed
     } else {
         if (bias) {
-            // thread -> 8 channels (a 16-byte chunk) of every 32nd pixel
+            // thread -> 8 channels (a 16-byte chunk) of every 32nd pixel of
+            // this CTA's share of the rows
             float s[4][8] = {};
             const int c = tid & 3;
-            RingPos d;
-            for (int r = r0; r < r1; ++r) {
-                if (!mbar_wait_bounded(&dfull[d.slot], d.parity)) break;
-                const unsigned char *t = dring + d.slot * p.dslot;
-                for (int px = tid >> 2; px < p.wp; px += 32) {
-                    const int off = px * 64 + ((c ^ ((px >> 1) & 3)) << 4);  // 64-byte swizzle
+            const unsigned char *own = dring + (tid >> 2) * 64 + ((c ^ ((tid >> 3) & 3)) << 4);  // 64-byte swizzle
+            RingPos q;
+            bool ok = true;
+            for (int r = r0; r < r1 && ok;) {
+                const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
+                for (int i = -2 * dil; i < np; i += rs) {
+                    if (!warp_wait_bounded(&full[q.slot], q.parity)) { ok = false; break; }
+                    for (int j = max(i, 0); j < min(i + rs, np); ++j) {
+                        if ((y0 + j) % 3 != shift) continue;
+                        const unsigned char *t = own + q.slot * p.dslot + (j - i) * drow;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (k >= nb) break;
-                        const uint4 v = *reinterpret_cast<const uint4 *>(t + k * tile + off);
-                        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+                        for (int k = 0; k < 4; ++k) {
+                            if (k >= nb) break;
+                            uint4 v[4];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 f = __bfloat1622float2(h[e]);
-                            s[k][2 * e] += f.x;
-                            s[k][2 * e + 1] += f.y;
+                            for (int u = 0; u < 4; ++u) {
+                                v[u] = make_uint4(0, 0, 0, 0);
+                                if ((tid >> 2) + 32 * u < p.wp)
+                                    v[u] = *reinterpret_cast<const uint4 *>(t + k * tile + u * 2048);
+                            }
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v[u]);
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float2 f = __bfloat1622float2(h[e]);
+                                    s[k][2 * e] += f.x;
+                                    s[k][2 * e + 1] += f.y;
+                                }
+                            }
                         }
                     }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[q.slot]);
+                    q.next(nst);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&dempty[d.slot]);
-                d.next(nd);
+                r += np;
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     for (int o = 4; o < 32; o <<= 1) s[k][e] += __shfl_xor_sync(0xffffffffu, s[k][e], o);
-                    if (k < nb && lane < 4) atomicAdd(db + co0 + 32 * k + 8 * c + e, s[k][e]);
+                    if (lane < 4) bsum[warp][32 * k + 8 * c + e] = s[k][e];
                 }
+            named_barrier_and(1, 128, true);  // the four warps' sums, then one atomic per channel
+            if (tid < ncols) atomicAdd(db + co0 + tid, (bsum[0][tid] + bsum[1][tid]) + (bsum[2][tid] + bsum[3][tid]));
         }
         const bool done = mbar_wait_bounded(accd, 0);
         tc_fence_after();
@@ -1511,7 +1527,7 @@ namespace {
 // The row-marching weight gradient's plan for a layer; false where the rows
 // of one march do not fit shared memory in segments of 16 pixels (dilations
 // beyond about 20).  Two CTAs share an SM where the rings allow it.
-constexpr int WR_SMEM = 110 * 1024, WR_SMEM_MAX = 220 * 1024;
+constexpr int WR_SMEM = 107 * 1024, WR_SMEM_MAX = 218 * 1024;
 bool wgrad_rows_plan(const unet_act *x, const unet_act *dy, int dil, WgradRows *p) {
     if (x->c % 32 || dy->c % 32 || (long long)x->n * x->h * ((x->w + 15) / 16) >= (1LL << 31)) return false;
     const int nb = std::min(dy->c, 128) / 32;
@@ -1520,10 +1536,11 @@ bool wgrad_rows_plan(const unet_act *x, const unet_act *dy, int dil, WgradRows *
             // the shortest segment that covers a row, else the longest that fits
             if (wp > 16 && wp / 2 >= x->w) continue;
             wp = std::min(wp, (x->w + 15) / 16 * 16);
-            const int nd = wp * nb > 256 ? 3 : 4, dslot = nb * wp * 64, tile = wp * 64;
-            const int nx = std::min(16, (budget - nd * dslot) / tile - 3 * dil);
-            if (nx < 2 * dil + 2) continue;
-            *p = {x->c, dy->c, x->n, x->h, x->w, dil, wp, (x->w + wp - 1) / wp * x->n * x->h, 1, nx, nd, dslot};
+            const int rs = std::max(1, 256 / (wp * nb)), tile = wp * 64, lag = (2 * dil + rs - 1) / rs;
+            const int dslot = rs * nb * tile, fixed = (2 * lag * rs + dil) * tile;
+            const int stages = std::min(8, (budget - fixed) / (dslot + rs * tile));
+            if (stages < 3) continue;
+            *p = {x->c, dy->c, x->n, x->h, x->w, dil, wp, rs, (x->w + wp - 1) / wp * x->n * x->h, 1, stages, lag, dslot};
             // Slices of the rows.  The tensor core truncates: a sum of k
             // steps of 16 pixels ends about 1.5e-8 k below its exact value
             // (measured, positive activations), so few slices cost accuracy
@@ -1558,18 +1575,19 @@ int launch_wgrad_rows(const unet_act *x, const unet_act *dy, float *dw, float *d
     typedef unsigned long long u64;
     const u64 W = p.W, H = p.H, N = p.n, xc = 2ull * x->c_stride, gc = 2ull * dy->c_stride;
     const u64 xd[4] = {(u64)p.cin, W, H, N}, xs[3] = {xc, xc * W, xc * W * H};
-    const unsigned xb[4] = {32u, (unsigned)p.wp, 1u, 1u};
+    const unsigned xb[4] = {32u, (unsigned)p.wp, (unsigned)p.rs, 1u};
     int rc = make_tensor_map_general(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, static_cast<const bf16 *>(x->ptr) + x->c_off,
                                      xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
-    // dy's channels in blocks of 32: one box holds every block of a row
+    // dy's channels in blocks of 32: one box holds every block of a step
     const u64 gd[5] = {32, W, (u64)p.cout / 32, H, N}, gs[4] = {gc, 64, gc * W, gc * W * H};
-    const unsigned gb[5] = {32u, (unsigned)p.wp, (unsigned)(p.dslot / (p.wp * 64)), 1u, 1u};
+    const unsigned gb[5] = {32u, (unsigned)p.wp, (unsigned)(p.dslot / (p.rs * p.wp * 64)), (unsigned)p.rs, 1u};
     rc = make_tensor_map_general(&gm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, static_cast<const bf16 *>(dy->ptr) + dy->c_off,
                                  gd, gs, gb, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
-    const int smem = (p.nx + 3 * p.dil) * p.wp * 64 + p.nd * p.dslot + 1024 + (2 * (p.nx + p.nd) + 1) * 8 + 16;
-    k_wgrad_rows<<<dim3(p.slices, 3 * (p.cin / 32), (p.cout + 127) / 128), 224, smem, s>>>(xm, gm, dw, db, p);
+    const int xrows = (p.stages + 2 * p.lag) * p.rs + p.dil;
+    const int smem = xrows * p.wp * 64 + p.stages * p.dslot + 1024 + (2 * p.stages + 1) * 8 + 16;
+    k_wgrad_rows<<<dim3(p.slices, 3 * (p.cin / 32), (p.cout + 127) / 128), 192, smem, s>>>(xm, gm, dw, db, p);
     return cuda_fail(cudaGetLastError(), "wgrad (tcgen05) launch");
 }
 
