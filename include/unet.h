@@ -55,6 +55,12 @@ UNET_API int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const flo
  * convolution, so that dx = unet_conv3x3_fwd(dy, wt, NULL, dx, 0). */
 UNET_API int unet_flip_weights(const void *w, void *wt, int cout, int cin,
                                stencil_stream_t stream);
+/* The data gradient through a ReLU: dx = conv3x3(dy, wt) (flipped weights, taps
+ * `dilation` apart) where gate > 0, else 0; gate has dx's shape (the layer's
+ * input, itself a ReLU's output).  Equals the convolution without bias and
+ * then unet_relu_bwd(dx, gate). */
+UNET_API int unet_conv3x3_dgrad_relu(const unet_act *dy, const void *wt, const unet_act *gate,
+                                     const unet_act *dx, int dilation, stencil_stream_t stream);
 /* dw[co][ky][kx][ci] += sum_p dy[p][co] * x[p + (ky-1, kx-1)][ci] (FP32, atomics);
  * db[co] += sum_p dy[p][co] if db != NULL. */
 UNET_API int unet_conv3x3_wgrad(const unet_act *x, const unet_act *dy, float *dw, float *db,
@@ -82,9 +88,18 @@ UNET_API int unet_relu_bwd(const unet_act *g, const unet_act *y, stencil_stream_
 UNET_API int unet_maxpool2_fwd(const unet_act *x, const unet_act *y, stencil_stream_t stream);
 UNET_API int unet_maxpool2_bwd(const unet_act *x, const unet_act *y, const unet_act *dy,
                                const unet_act *dx, stencil_stream_t stream);
+/* The pooling gradient, plus a skip connection's gradient, through the ReLU
+ * whose output x was pooled: unet_maxpool2_bwd(x, y, dy, dx), unet_add(dx,
+ * skip) and unet_relu_bwd(dx, x) in one pass. */
+UNET_API int unet_maxpool2_bwd_skip_relu(const unet_act *x, const unet_act *y, const unet_act *dy,
+                                         const unet_act *skip, const unet_act *dx,
+                                         stencil_stream_t stream);
 /* Nearest-neighbour x2 upsampling and its gradient (sum of the 2x2 block). */
 UNET_API int unet_upsample2_fwd(const unet_act *x, const unet_act *y, stencil_stream_t stream);
 UNET_API int unet_upsample2_bwd(const unet_act *dy, const unet_act *dx, stencil_stream_t stream);
+/* unet_upsample2_bwd(dy, dx) and unet_relu_bwd(dx, gate) in one pass. */
+UNET_API int unet_upsample2_bwd_relu(const unet_act *dy, const unet_act *gate, const unet_act *dx,
+                                     stencil_stream_t stream);
 /* a += b (BF16 views of the same shape). */
 UNET_API int unet_add(const unet_act *a, const unet_act *b, stencil_stream_t stream);
 /* Output head: y[p] = sum_c x[p][c] * w[c] + b[0] (FP32 out, one channel). */
@@ -93,6 +108,9 @@ UNET_API int unet_head_fwd(const unet_act *x, const float *w, const float *b, fl
 /* Head gradient: dx[p][c] = dy[p] * w[c]; dw[c] += sum_p dy[p] x[p][c]; db += sum dy. */
 UNET_API int unet_head_bwd(const unet_act *x, const float *w, const float *dy,
                            const unet_act *dx, float *dw, float *db, stencil_stream_t stream);
+/* The same with dx through the ReLU whose output x is (dx = 0 where x <= 0). */
+UNET_API int unet_head_bwd_relu(const unet_act *x, const float *w, const float *dy,
+                                const unet_act *dx, float *dw, float *db, stencil_stream_t stream);
 /* Input features of n 2-D problems (fields fp32 [n][h][w], border band of
  * width 1 holds the Dirichlet values): channel 0 = the border field (zero
  * interior), 1 = the border mask, 2 = the transfinite (Coons) interpolation of

@@ -57,6 +57,19 @@ struct Act {
 
 Act to_act(const unet_act &a) { return {static_cast<bf16 *>(a.ptr), a.n, a.h, a.w, a.c_stride, a.c_off, a.c}; }
 
+// v where the gate's value is positive, else 0 (the ReLU gradient), for eight
+// BF16 values.
+__device__ __forceinline__ uint4 gate8(uint4 v, uint4 gate) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(&v);
+    const __nv_bfloat162 *g = reinterpret_cast<const __nv_bfloat162 *>(&gate);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = __bfloat1622float2(g[k]);
+        w[k] &= (f.x > 0.f ? 0x0000FFFFu : 0u) | (f.y > 0.f ? 0xFFFF0000u : 0u);
+    }
+    return v;
+}
+
 // ---------------------------------------------------------------------------
 // 3x3 convolution, forward (also the data gradient with flipped weights).
 // Block: 128 threads = 2 x 2 warps; tile BM = 128 pixels x BN output channels,
@@ -302,7 +315,7 @@ struct ConvTiles {
 template <int BN, int BC>
 __global__ void __launch_bounds__(192)
     k_conv3x3_tma(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-                  const float *__restrict__ bias, Act y, ConvTiles p) {
+                  const float *__restrict__ bias, Act y, Act gate, ConvTiles p) {
     extern __shared__ __align__(1024) unsigned char tm_smem[];
     constexpr int A_BYTES = BM * BC * 2, STAGE = A_BYTES + BN * BC * 2;
     unsigned char *base = reinterpret_cast<unsigned char *>(
@@ -385,7 +398,9 @@ __global__ void __launch_bounds__(192)
         if (done && !*reinterpret_cast<volatile int *>(bad)) {
             const int m = warp * 32 + lane, row = h0 + m / p.tile_w, col = w0 + m % p.tile_w;
             const bool in = row < p.H && col < p.W;
-            bf16 *out = y.p + (((long long)n * p.H + row) * p.W + col) * y.cs + y.co + n0;
+            const long long px = ((long long)n * p.H + row) * p.W + col;
+            bf16 *out = y.p + px * y.cs + y.co + n0;
+            const bf16 *gt = gate.p + px * gate.cs + gate.co + n0;
 #pragma unroll
             for (int c = 0; c < BN; c += 8) {
                 uint32_t r[8];
@@ -408,7 +423,10 @@ __global__ void __launch_bounds__(192)
                 q.y = *reinterpret_cast<uint32_t *>(&h1v);
                 q.z = *reinterpret_cast<uint32_t *>(&h2v);
                 q.w = *reinterpret_cast<uint32_t *>(&h3v);
-                if (in) *reinterpret_cast<uint4 *>(out + c) = q;
+                if (in) {
+                    if (gate.p) q = gate8(q, *reinterpret_cast<const uint4 *>(gt + c));
+                    *reinterpret_cast<uint4 *>(out + c) = q;
+                }
             }
         }
     }
@@ -442,7 +460,7 @@ struct ConvMarch {
 template <int BN>
 __global__ void __launch_bounds__(192)
     k_conv3x3_march(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-                    const float *__restrict__ bias, Act y, ConvMarch p) {
+                    const float *__restrict__ bias, Act y, Act gate, ConvMarch p) {
     extern __shared__ __align__(1024) unsigned char mc_smem[];
     constexpr int WT = BN * BK * 2;  // weights of one tap and chunk
     constexpr uint32_t TCOLS = BN <= 32 ? 64 : BN <= 64 ? 128 : 256;
@@ -558,7 +576,9 @@ __global__ void __launch_bounds__(192)
             tc_fence_after();
             const int img = r / p.H, row = r - img * p.H, col = img / p.n * 128 + warp * 32 + lane;
             const bool in = col < p.W;
-            bf16 *out = y.p + (((long long)(img % p.n) * p.H + row) * p.W + col) * y.cs + y.co + n0;
+            const long long px = ((long long)(img % p.n) * p.H + row) * p.W + col;
+            bf16 *out = y.p + px * y.cs + y.co + n0;
+            const bf16 *gt = gate.p + px * gate.cs + gate.co + n0;
             const uint32_t t = tmem + ((uint32_t)(warp * 32) << 16) + acc.slot * (TCOLS / 2);
 #pragma unroll
             for (int c = 0; c < BN; c += 32) {
@@ -591,7 +611,10 @@ __global__ void __launch_bounds__(192)
                         const __nv_bfloat162 b2 = __floats2bfloat162_rn(a0, a1);
                         h[e / 2] = *reinterpret_cast<const uint32_t *>(&b2);
                     }
-                    if (in) *reinterpret_cast<uint4 *>(out + c + g) = q;
+                    if (in) {
+                        if (gate.p) q = gate8(q, *reinterpret_cast<const uint4 *>(gt + c + g));
+                        *reinterpret_cast<uint4 *>(out + c + g) = q;
+                    }
                 }
             }
             acc.next(2);
@@ -1049,8 +1072,10 @@ __global__ void k_pool_fwd(Act x, Act y) {
     }
 }
 
-// dx = dy routed to the first input of each 2x2 block equal to the max (y).
-__global__ void k_pool_bwd(Act x, Act y, Act dy, Act dx) {
+// dx = dy routed to the first input of each 2x2 block equal to the max (y);
+// with a skip gradient (skip.p), that is added (one rounding to BF16, as a sum
+// of two stored gradients) and the result passes where x > 0.
+__global__ void k_pool_bwd(Act x, Act y, Act dy, Act skip, Act dx) {
     const long long n = vec_count(y);
     const int c8n = y.c / 8;
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n;
@@ -1076,6 +1101,17 @@ __global__ void k_pool_bwd(Act x, Act y, Act dy, Act dx) {
                 taken[k] = taken[k] || hit;
                 ob[k] = hit ? gb[k] : __float2bfloat16_rn(0.f);
             }
+            if (skip.p) {
+                const uint4 sv = *reinterpret_cast<const uint4 *>(skip.p + ip * skip.cs + skip.co + c8 * 8);
+                __nv_bfloat162 *op = reinterpret_cast<__nv_bfloat162 *>(&ov);
+                const __nv_bfloat162 *sp = reinterpret_cast<const __nv_bfloat162 *>(&sv);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 a = __bfloat1622float2(op[k]), b = __bfloat1622float2(sp[k]);
+                    op[k] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+                }
+                ov = gate8(ov, xv);
+            }
             *reinterpret_cast<uint4 *>(dx.p + ip * dx.cs + dx.co + c8 * 8) = ov;
         }
     }
@@ -1095,7 +1131,8 @@ __global__ void k_up_fwd(Act x, Act y) {
     }
 }
 
-__global__ void k_up_bwd(Act dy, Act dx) {
+// gate.p: the result passes where the gate is positive.
+__global__ void k_up_bwd(Act dy, Act gate, Act dx) {
     const long long n = vec_count(dx);
     const int c8n = dx.c / 8;
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n;
@@ -1120,6 +1157,7 @@ __global__ void k_up_bwd(Act dy, Act dx) {
         __nv_bfloat162 *op = reinterpret_cast<__nv_bfloat162 *>(&ov);
 #pragma unroll
         for (int k = 0; k < 4; ++k) op[k] = __floats2bfloat162_rn(s[2 * k], s[2 * k + 1]);
+        if (gate.p) ov = gate8(ov, *reinterpret_cast<const uint4 *>(gate.p + p * gate.cs + gate.co + c8 * 8));
         *reinterpret_cast<uint4 *>(dx.p + p * dx.cs + dx.co + c8 * 8) = ov;
     }
 }
@@ -1145,21 +1183,27 @@ __global__ void k_head_fwd(Act x, const float *__restrict__ w, const float *__re
     }
 }
 
-__global__ void k_head_bwd(Act x, const float *__restrict__ w, const float *__restrict__ dy, Act dx,
-                           float *__restrict__ dw, float *__restrict__ db) {
-    // block: 256 threads; thread t owns channel t % x.c partial sums for dw.
+// Head gradient: dx = dy w (where x > 0 with GATE), dw += sum dy x, db += sum
+// dy.  A thread owns 8 channels of every groups-th pixel and keeps their sums
+// in registers; bound by HBM (64 x 128^2 x 32 channels: 502 us with an atomic
+// on shared memory per value, 42 us so).
+template <bool GATE>
+__global__ void __launch_bounds__(256) k_head_bwd(Act x, const float *__restrict__ w, const float *__restrict__ dy, Act dx,
+                                                  float *__restrict__ dw, float *__restrict__ db) {
     __shared__ float sdw[256];
     __shared__ float sdb;
-    if (threadIdx.x < 256) sdw[threadIdx.x] = 0.f;
+    sdw[threadIdx.x] = 0.f;
     if (threadIdx.x == 0) sdb = 0.f;
     __syncthreads();
+    const int c8n = x.c / 8, groups = 256 / c8n, c = (int)threadIdx.x % c8n * 8, grp = (int)threadIdx.x / c8n;
     const long long P = (long long)x.n * x.h * x.w;
-    float mydb = 0.f;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P;
-         p += (long long)gridDim.x * blockDim.x) {
-        const float g = dy[p];
-        mydb += g;
-        for (int c = 0; c < x.c; c += 8) {
+    float wv[8], s[8] = {}, sb = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) wv[k] = w[c + k];
+    if (grp < groups)
+        for (long long p = (long long)blockIdx.x * groups + grp; p < P; p += (long long)gridDim.x * groups) {
+            const float g = dy[p];
+            if (c == 0) sb += g;
             const uint4 xv = *reinterpret_cast<const uint4 *>(x.p + p * x.cs + x.co + c);
             const __nv_bfloat162 *xp = reinterpret_cast<const __nv_bfloat162 *>(&xv);
             uint4 ov;
@@ -1167,16 +1211,20 @@ __global__ void k_head_bwd(Act x, const float *__restrict__ w, const float *__re
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float2 f = __bfloat1622float2(xp[k]);
-                atomicAdd(&sdw[c + 2 * k], g * f.x);
-                atomicAdd(&sdw[c + 2 * k + 1], g * f.y);
-                op[k] = __floats2bfloat162_rn(g * w[c + 2 * k], g * w[c + 2 * k + 1]);
+                s[2 * k] += g * f.x;
+                s[2 * k + 1] += g * f.y;
+                op[k] = __floats2bfloat162_rn(g * wv[2 * k], g * wv[2 * k + 1]);
             }
+            if (GATE) ov = gate8(ov, xv);
             *reinterpret_cast<uint4 *>(dx.p + p * dx.cs + dx.co + c) = ov;
         }
+    if (grp < groups) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) atomicAdd(&sdw[c + k], s[k]);
+        if (c == 0) atomicAdd(&sdb, sb);
     }
-    atomicAdd(&sdb, mydb);
     __syncthreads();
-    if (threadIdx.x < x.c) atomicAdd(&dw[threadIdx.x], sdw[threadIdx.x]);
+    if ((int)threadIdx.x < x.c) atomicAdd(&dw[threadIdx.x], sdw[threadIdx.x]);
     if (threadIdx.x == 0) atomicAdd(db, sdb);
 }
 
@@ -1366,8 +1414,8 @@ int tma_tile_w(int H, int W) {
 }
 
 template <int BN, int BC>
-int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil,
-                    cudaStream_t s) {
+int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate, int relu,
+                    int dil, cudaStream_t s) {
     constexpr int STAGE = (BM + BN) * BC * 2, SMEM_MAX = 200 * 1024;
     static bool attr[64] = {false};
     const int dev = current_device();
@@ -1400,15 +1448,15 @@ int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act
     const int budget = (long long)grid.x * grid.y <= num_sms() ? SMEM_MAX : BN == 128 ? 100 * 1024 : 48 * 1024;
     p.stages = std::max(2, std::min(9 * cin / BC, std::min(8, budget / STAGE)));
     const int smem = p.stages * STAGE + (2 * p.stages + 1) * 8 + 16 + 1024;
-    k_conv3x3_tma<BN, BC><<<grid, 192, smem, s>>>(xm, wm, b, ya, p);
+    k_conv3x3_tma<BN, BC><<<grid, 192, smem, s>>>(xm, wm, b, ya, gate, p);
     return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05, TMA) launch");
 }
 
 template <int BN>
-int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil,
-                    cudaStream_t s) {
-    return x->c % 64 == 0 ? launch_conv_tma<BN, 64>(x, wb, b, ya, relu, dil, s)
-                          : launch_conv_tma<BN, 32>(x, wb, b, ya, relu, dil, s);
+int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate, int relu,
+                    int dil, cudaStream_t s) {
+    return x->c % 64 == 0 ? launch_conv_tma<BN, 64>(x, wb, b, ya, gate, relu, dil, s)
+                          : launch_conv_tma<BN, 32>(x, wb, b, ya, gate, relu, dil, s);
 }
 
 // Whether the marching form takes the layer, and its plan: rows of more than
@@ -1431,8 +1479,8 @@ bool conv_march_plan(const unet_act *x, int relu, int dil, ConvMarch *p) {
 }
 
 template <int BN>
-int launch_conv_march(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const ConvMarch &p,
-                      cudaStream_t s) {
+int launch_conv_march(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate,
+                      const ConvMarch &p, cudaStream_t s) {
     static bool attr[64] = {false};
     const int dev = current_device();
     if (dev >= 0 && dev < 64 && !attr[dev]) {
@@ -1455,17 +1503,29 @@ int launch_conv_march(const unet_act *x, const bf16 *wb, const float *b, const A
     const int smem = 9 * nc * BN * BK * 2 + p.slots * nc * p.rowbytes + 1024 + (2 * p.slots + 5) * 8 + 16;
     const int per_sm = std::max(1, std::min(512 / (BN <= 32 ? 64 : BN <= 64 ? 128 : 256), (227 * 1024) / (smem + 1024)));
     const int ctas = std::max(1, std::min(p.rows, per_sm * num_sms() / (ya.c / BN)));
-    k_conv3x3_march<BN><<<dim3(ctas, ya.c / BN), 192, smem, s>>>(xm, wm, b, ya, p);
+    k_conv3x3_march<BN><<<dim3(ctas, ya.c / BN), 192, smem, s>>>(xm, wm, b, ya, gate, p);
     return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05, rows) launch");
 }
 
 template <int BN>
-int launch_conv(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, int relu, int dil, cudaStream_t s) {
+int launch_conv(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate, int relu, int dil,
+                cudaStream_t s) {
     ConvMarch m;
-    if (conv_march_plan<BN>(x, relu, dil, &m)) return launch_conv_march<BN>(x, wb, b, ya, m, s);
+    if (conv_march_plan<BN>(x, relu, dil, &m)) return launch_conv_march<BN>(x, wb, b, ya, gate, m, s);
     // tiles of at most 128 channels whose number divides the layer's
-    if constexpr (BN == 96) return launch_conv_tma<32>(x, wb, b, ya, relu, dil, s);
-    else return launch_conv_tma<BN>(x, wb, b, ya, relu, dil, s);
+    if constexpr (BN == 96) return launch_conv_tma<32>(x, wb, b, ya, gate, relu, dil, s);
+    else return launch_conv_tma<BN>(x, wb, b, ya, gate, relu, dil, s);
+}
+
+// The tcgen05 convolution; gate.p null: none.
+int conv_tcgen05(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate, int relu, int dil,
+                 cudaStream_t s) {
+    if (ya.c % 128 == 0) return launch_conv<128>(x, wb, b, ya, gate, relu, dil, s);
+    if (ya.c == 96) return launch_conv<96>(x, wb, b, ya, gate, relu, dil, s);
+    if (ya.c == 64) return launch_conv<64>(x, wb, b, ya, gate, relu, dil, s);
+    if (ya.c == 32) return launch_conv<32>(x, wb, b, ya, gate, relu, dil, s);
+    return ya.c % 64 == 0 ? launch_conv_tma<64>(x, wb, b, ya, gate, relu, dil, s)
+                          : launch_conv_tma<32>(x, wb, b, ya, gate, relu, dil, s);
 }
 
 extern "C" int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const float *b,
@@ -1487,14 +1547,7 @@ extern "C" int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const f
     // once (64 x 128^2, us, marching / tiled / mma.sync: 32 -> 32 channels 39 /
     // 74 / 149, 96 -> 32 96 / 146 / 349, 32 -> 96 93 / 231 / 425; one 128^2
     // image 8 / 7 / 12)
-    if (engine != 2) {
-        if (y->c == 32) return launch_conv<32>(x, wb, b, ya, relu, dilation, STREAM(s));
-        if (y->c == 96) return launch_conv<96>(x, wb, b, ya, relu, dilation, STREAM(s));
-        if (y->c == 64) return launch_conv<64>(x, wb, b, ya, relu, dilation, STREAM(s));
-        if (y->c % 128 == 0) return launch_conv<128>(x, wb, b, ya, relu, dilation, STREAM(s));
-        if (y->c % 64 == 0) return launch_conv_tma<64>(x, wb, b, ya, relu, dilation, STREAM(s));
-        return launch_conv_tma<32>(x, wb, b, ya, relu, dilation, STREAM(s));
-    }
+    if (engine != 2) return conv_tcgen05(x, wb, b, ya, Act{}, relu, dilation, STREAM(s));
     if (y->c % 64 == 0) {
         dim3 grid((unsigned)((P + BM - 1) / BM), y->c / 64);
         k_conv3x3<64><<<grid, 128, 0, STREAM(s)>>>(xa, wb, b, ya, relu, dilation);
@@ -1503,6 +1556,20 @@ extern "C" int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const f
         k_conv3x3<32><<<grid, 128, 0, STREAM(s)>>>(xa, wb, b, ya, relu, dilation);
     }
     return cuda_fail(cudaGetLastError(), "conv3x3 launch");
+}
+
+extern "C" int unet_conv3x3_dgrad_relu(const unet_act *dy, const void *wt, const unet_act *gate, const unet_act *dx,
+                                       int dilation, stencil_stream_t s) {
+    CHECK_VIEW(dy);
+    CHECK_VIEW(gate);
+    CHECK_VIEW(dx);
+    if (!wt) return fail(STENCIL_EINVAL, "null weights");
+    if (dilation < 1) return fail(STENCIL_EINVAL, "dilation must be >= 1");
+    if (dy->c % 32 || dx->c % 32) return fail(STENCIL_EINVAL, "channels must be multiples of 32");
+    if (dy->n != dx->n || dy->h != dx->h || dy->w != dx->w || gate->n != dx->n || gate->h != dx->h ||
+        gate->w != dx->w || gate->c != dx->c)
+        return fail(STENCIL_EINVAL, "shape mismatch");
+    return conv_tcgen05(dy, static_cast<const bf16 *>(wt), nullptr, to_act(*dx), to_act(*gate), 0, dilation, STREAM(s));
 }
 
 extern "C" int unet_conv3x3_fwd_dil(const unet_act *x, const void *w, const float *b,
@@ -1673,7 +1740,22 @@ extern "C" int unet_maxpool2_bwd(const unet_act *x, const unet_act *y, const une
     CHECK_VIEW(dy);
     CHECK_VIEW(dx);
     k_pool_bwd<<<grid_for((long long)y->n * y->h * y->w * (y->c / 8)), 256, 0, STREAM(s)>>>(
-        to_act(*x), to_act(*y), to_act(*dy), to_act(*dx));
+        to_act(*x), to_act(*y), to_act(*dy), Act{}, to_act(*dx));
+    return cuda_fail(cudaGetLastError(), "pool bwd launch");
+}
+
+extern "C" int unet_maxpool2_bwd_skip_relu(const unet_act *x, const unet_act *y, const unet_act *dy,
+                                           const unet_act *skip, const unet_act *dx, stencil_stream_t s) {
+    const unet_act *v[5] = {x, y, dy, skip, dx};
+    for (const unet_act *a : v) {
+        int rc = check_act(a, "pool bwd");
+        if (rc) return rc;
+        const int f = a == y || a == dy ? 2 : 1;
+        if (a->n != x->n || a->h * f != x->h || a->w * f != x->w || a->c != x->c)
+            return fail(STENCIL_EINVAL, "pool shapes");
+    }
+    k_pool_bwd<<<grid_for((long long)y->n * y->h * y->w * (y->c / 8)), 256, 0, STREAM(s)>>>(
+        to_act(*x), to_act(*y), to_act(*dy), to_act(*skip), to_act(*dx));
     return cuda_fail(cudaGetLastError(), "pool bwd launch");
 }
 
@@ -1688,7 +1770,19 @@ extern "C" int unet_upsample2_fwd(const unet_act *x, const unet_act *y, stencil_
 extern "C" int unet_upsample2_bwd(const unet_act *dy, const unet_act *dx, stencil_stream_t s) {
     CHECK_VIEW(dy);
     CHECK_VIEW(dx);
-    k_up_bwd<<<grid_for((long long)dx->n * dx->h * dx->w * (dx->c / 8)), 256, 0, STREAM(s)>>>(to_act(*dy), to_act(*dx));
+    k_up_bwd<<<grid_for((long long)dx->n * dx->h * dx->w * (dx->c / 8)), 256, 0, STREAM(s)>>>(to_act(*dy), Act{}, to_act(*dx));
+    return cuda_fail(cudaGetLastError(), "upsample bwd launch");
+}
+
+extern "C" int unet_upsample2_bwd_relu(const unet_act *dy, const unet_act *gate, const unet_act *dx, stencil_stream_t s) {
+    CHECK_VIEW(dy);
+    CHECK_VIEW(gate);
+    CHECK_VIEW(dx);
+    if (dy->n != dx->n || dy->h != 2 * dx->h || dy->w != 2 * dx->w || dy->c != dx->c || gate->n != dx->n ||
+        gate->h != dx->h || gate->w != dx->w || gate->c != dx->c)
+        return fail(STENCIL_EINVAL, "upsample shapes");
+    k_up_bwd<<<grid_for((long long)dx->n * dx->h * dx->w * (dx->c / 8)), 256, 0, STREAM(s)>>>(
+        to_act(*dy), to_act(*gate), to_act(*dx));
     return cuda_fail(cudaGetLastError(), "upsample bwd launch");
 }
 
@@ -1707,13 +1801,26 @@ extern "C" int unet_head_fwd(const unet_act *x, const float *w, const float *b, 
     return cuda_fail(cudaGetLastError(), "head launch");
 }
 
-extern "C" int unet_head_bwd(const unet_act *x, const float *w, const float *dy, const unet_act *dx,
-                             float *dw, float *db, stencil_stream_t s) {
+static int head_bwd(const unet_act *x, const float *w, const float *dy, const unet_act *dx, float *dw, float *db,
+                    bool gate, cudaStream_t s) {
     CHECK_VIEW(x);
     CHECK_VIEW(dx);
     if (!w || !dy || !dw || !db || x->c > 256) return fail(STENCIL_EINVAL, "bad head arguments");
-    k_head_bwd<<<grid_for((long long)x->n * x->h * x->w), 256, 0, STREAM(s)>>>(to_act(*x), w, dy, to_act(*dx), dw, db);
+    const long long px = (long long)x->n * x->h * x->w, per = 256 / (x->c / 8);
+    const int blocks = (int)std::min(8LL * num_sms(), (px + per - 1) / per);
+    if (gate) k_head_bwd<true><<<blocks, 256, 0, s>>>(to_act(*x), w, dy, to_act(*dx), dw, db);
+    else k_head_bwd<false><<<blocks, 256, 0, s>>>(to_act(*x), w, dy, to_act(*dx), dw, db);
     return cuda_fail(cudaGetLastError(), "head bwd launch");
+}
+
+extern "C" int unet_head_bwd(const unet_act *x, const float *w, const float *dy, const unet_act *dx,
+                             float *dw, float *db, stencil_stream_t s) {
+    return head_bwd(x, w, dy, dx, dw, db, false, STREAM(s));
+}
+
+extern "C" int unet_head_bwd_relu(const unet_act *x, const float *w, const float *dy, const unet_act *dx,
+                                  float *dw, float *db, stencil_stream_t s) {
+    return head_bwd(x, w, dy, dx, dw, db, true, STREAM(s));
 }
 
 extern "C" int unet_features(const float *fields, int n, int h, int w, const unet_act *x, float *coons,

@@ -65,14 +65,18 @@ def _L():
             "unet_wgrad_workspace_bytes": [A, A, ctypes.POINTER(ctypes.c_size_t)],
             "unet_flip_weights": [vp, vp, i, i, vp],
             "unet_conv3x3_wgrad": [A, A, vp, vp, vp],
+            "unet_conv3x3_dgrad_relu": [A, vp, A, A, i, vp],
             "unet_relu_bwd": [A, A, vp],
             "unet_maxpool2_fwd": [A, A, vp],
             "unet_maxpool2_bwd": [A, A, A, A, vp],
+            "unet_maxpool2_bwd_skip_relu": [A, A, A, A, A, vp],
             "unet_upsample2_fwd": [A, A, vp],
             "unet_upsample2_bwd": [A, A, vp],
+            "unet_upsample2_bwd_relu": [A, A, A, vp],
             "unet_add": [A, A, vp],
             "unet_head_fwd": [A, vp, vp, vp, vp],
             "unet_head_bwd": [A, vp, vp, A, vp, vp, vp],
+            "unet_head_bwd_relu": [A, vp, vp, A, vp, vp, vp],
             "unet_features": [vp, i, i, i, A, vp, vp],
             "unet_mse": [vp, vp, vp, i, i, i, f, vp, vp, vp],
             "unet_adam": [vp, vp, vp, vp, vp, ll, f, f, f, f, i, vp],
@@ -255,19 +259,22 @@ class UNet:
         return B["out"], B["coons"], B
 
     # -- backward ----------------------------------------------------------
-    def _conv_bwd(self, name, x, y, gy, gx, s):
-        """gy holds dL/dy (post-ReLU output y); accumulates dW/db, writes dL/dx into gx."""
+    def _conv_bwd(self, name, x, gy, gx, s, relu=False):
+        """gy holds the gradient before the layer's ReLU; accumulates dW/db,
+        writes dL/dx into gx (with relu: through the ReLU whose output x is)."""
         L = _L()
         P = self.params[name]
-        _chk(L.unet_relu_bwd(ctypes.byref(gy), ctypes.byref(y), s), "relu_bwd " + name)
         d = DILATION.get(name, 1)
         _chk(L.unet_conv3x3_wgrad_engine(ctypes.byref(x), ctypes.byref(gy), _p(P["dw"]), _p(P["db"]), d, 0, None, 0, s),
              "wgrad " + name)
         if gx is not None:
             cin, cout = P["w"].shape[2], P["w"].shape[0]
             _chk(L.unet_flip_weights(_p(P["wb"]), _p(P["wt"]), cout, cin, s), "flip " + name)
-            _chk(L.unet_conv3x3_fwd_dil(ctypes.byref(gy), _p(P["wt"]), None, ctypes.byref(gx), 0, d, s),
-                 "dgrad " + name)
+            if relu:
+                rc = L.unet_conv3x3_dgrad_relu(ctypes.byref(gy), _p(P["wt"]), ctypes.byref(x), ctypes.byref(gx), d, s)
+            else:
+                rc = L.unet_conv3x3_fwd_dil(ctypes.byref(gy), _p(P["wt"]), None, ctypes.byref(gx), 0, d, s)
+            _chk(rc, "dgrad " + name)
 
     def zero_grad(self):
         for name, _, _ in LAYERS:
@@ -281,36 +288,30 @@ class UNet:
         s = _stream(stream)
         L = _L()
         V = view
-        _chk(L.unet_head_bwd(ctypes.byref(V(B["d0b"])), _p(self.head["w"]), _p(B["dout"]),
-                             ctypes.byref(V(B["g_d0b"])), _p(self.head["dw"]), _p(self.head["db"]), s),
+        _chk(L.unet_head_bwd_relu(ctypes.byref(V(B["d0b"])), _p(self.head["w"]), _p(B["dout"]),
+                                  ctypes.byref(V(B["g_d0b"])), _p(self.head["dw"]), _p(self.head["db"]), s),
              "head_bwd")
-        self._conv_bwd("d0b", V(B["d0a"]), V(B["d0b"]), V(B["g_d0b"]), V(B["g_d0a"]), s)
-        self._conv_bwd("d0a", V(B["cat0"]), V(B["d0a"]), V(B["g_d0a"]), V(B["g_cat0"]), s)
-        _chk(L.unet_upsample2_bwd(ctypes.byref(V(B["g_cat0"], 0, 64)), ctypes.byref(V(B["g_d1b"])), s), "up0 bwd")
-        self._conv_bwd("d1b", V(B["d1a"]), V(B["d1b"]), V(B["g_d1b"]), V(B["g_d1a"]), s)
-        self._conv_bwd("d1a", V(B["cat1"]), V(B["d1a"]), V(B["g_d1a"]), V(B["g_cat1"]), s)
-        _chk(L.unet_upsample2_bwd(ctypes.byref(V(B["g_cat1"], 0, 128)), ctypes.byref(V(B["g_d2b"])), s), "up1 bwd")
-        self._conv_bwd("d2b", V(B["d2a"]), V(B["d2b"]), V(B["g_d2b"]), V(B["g_d2a"]), s)
-        self._conv_bwd("d2a", V(B["cat2"]), V(B["d2a"]), V(B["g_d2a"]), V(B["g_cat2"]), s)
-        _chk(L.unet_upsample2_bwd(ctypes.byref(V(B["g_cat2"], 0, 256)), ctypes.byref(V(B["g_bb"])), s), "up2 bwd")
-        self._conv_bwd("bb", V(B["ba"]), V(B["bb"]), V(B["g_bb"]), V(B["g_ba"]), s)
-        self._conv_bwd("ba", V(B["p2"]), V(B["ba"]), V(B["g_ba"]), V(B["g_p2"]), s)
-        # level 2: pool gradient + skip gradient
-        _chk(L.unet_maxpool2_bwd(ctypes.byref(V(B["cat2"], 256, 128)), ctypes.byref(V(B["p2"])),
-                                 ctypes.byref(V(B["g_p2"])), ctypes.byref(V(B["g_e2b"])), s), "pool2 bwd")
-        _chk(L.unet_add(ctypes.byref(V(B["g_e2b"])), ctypes.byref(V(B["g_cat2"], 256, 128)), s), "add2")
-        self._conv_bwd("e2b", V(B["e2a"]), V(B["cat2"], 256, 128), V(B["g_e2b"]), V(B["g_e2a"]), s)
-        self._conv_bwd("e2a", V(B["p1"]), V(B["e2a"]), V(B["g_e2a"]), V(B["g_p1"]), s)
-        _chk(L.unet_maxpool2_bwd(ctypes.byref(V(B["cat1"], 128, 64)), ctypes.byref(V(B["p1"])),
-                                 ctypes.byref(V(B["g_p1"])), ctypes.byref(V(B["g_e1b"])), s), "pool1 bwd")
-        _chk(L.unet_add(ctypes.byref(V(B["g_e1b"])), ctypes.byref(V(B["g_cat1"], 128, 64)), s), "add1")
-        self._conv_bwd("e1b", V(B["e1a"]), V(B["cat1"], 128, 64), V(B["g_e1b"]), V(B["g_e1a"]), s)
-        self._conv_bwd("e1a", V(B["p0"]), V(B["e1a"]), V(B["g_e1a"]), V(B["g_p0"]), s)
-        _chk(L.unet_maxpool2_bwd(ctypes.byref(V(B["cat0"], 64, 32)), ctypes.byref(V(B["p0"])),
-                                 ctypes.byref(V(B["g_p0"])), ctypes.byref(V(B["g_e0b"])), s), "pool0 bwd")
-        _chk(L.unet_add(ctypes.byref(V(B["g_e0b"])), ctypes.byref(V(B["g_cat0"], 64, 32)), s), "add0")
-        self._conv_bwd("e0b", V(B["e0a"]), V(B["cat0"], 64, 32), V(B["g_e0b"]), V(B["g_e0a"]), s)
-        self._conv_bwd("e0a", V(B["x0"]), V(B["e0a"]), V(B["g_e0a"]), None, s)
+        R = ctypes.byref
+        # every gradient buffer holds the gradient before its layer's ReLU
+        self._conv_bwd("d0b", V(B["d0a"]), V(B["g_d0b"]), V(B["g_d0a"]), s, relu=True)
+        self._conv_bwd("d0a", V(B["cat0"]), V(B["g_d0a"]), V(B["g_cat0"]), s)
+        _chk(L.unet_upsample2_bwd_relu(R(V(B["g_cat0"], 0, 64)), R(V(B["d1b"])), R(V(B["g_d1b"])), s), "up0 bwd")
+        self._conv_bwd("d1b", V(B["d1a"]), V(B["g_d1b"]), V(B["g_d1a"]), s, relu=True)
+        self._conv_bwd("d1a", V(B["cat1"]), V(B["g_d1a"]), V(B["g_cat1"]), s)
+        _chk(L.unet_upsample2_bwd_relu(R(V(B["g_cat1"], 0, 128)), R(V(B["d2b"])), R(V(B["g_d2b"])), s), "up1 bwd")
+        self._conv_bwd("d2b", V(B["d2a"]), V(B["g_d2b"]), V(B["g_d2a"]), s, relu=True)
+        self._conv_bwd("d2a", V(B["cat2"]), V(B["g_d2a"]), V(B["g_cat2"]), s)
+        _chk(L.unet_upsample2_bwd_relu(R(V(B["g_cat2"], 0, 256)), R(V(B["bb"])), R(V(B["g_bb"])), s), "up2 bwd")
+        self._conv_bwd("bb", V(B["ba"]), V(B["g_bb"]), V(B["g_ba"]), s, relu=True)
+        self._conv_bwd("ba", V(B["p2"]), V(B["g_ba"]), V(B["g_p2"]), s)
+        # pool gradient + skip gradient, through the encoder's ReLU
+        for k, up, c in (("2", 256, 128), ("1", 128, 64), ("0", 64, 32)):
+            skip, e = V(B["cat" + k], up, c), "e" + k
+            _chk(L.unet_maxpool2_bwd_skip_relu(R(skip), R(V(B["p" + k])), R(V(B["g_p" + k])),
+                                               R(V(B["g_cat" + k], up, c)), R(V(B["g_" + e + "b"])), s), "pool%s bwd" % k)
+            self._conv_bwd(e + "b", V(B[e + "a"]), V(B["g_" + e + "b"]), V(B["g_" + e + "a"]), s, relu=True)
+            below = {"2": "p1", "1": "p0", "0": None}[k]
+            self._conv_bwd(e + "a", V(B[below or "x0"]), V(B["g_" + e + "a"]), below and V(B["g_" + below]), s)
 
     def loss_and_grad(self, fields, targets, stream=None):
         """Masked MSE of (coons + out) against targets over interior cells;
