@@ -55,6 +55,13 @@ UNET_API int unet_conv3x3_fwd_engine(const unet_act *x, const void *w, const flo
  * convolution, so that dx = unet_conv3x3_fwd(dy, wt, NULL, dx, 0). */
 UNET_API int unet_flip_weights(const void *w, void *wt, int cout, int cin,
                                stencil_stream_t stream);
+/* The same for several layers in one launch. */
+typedef struct unet_flip {
+    const void *w;
+    void *wt;
+    int cout, cin;
+} unet_flip;
+UNET_API int unet_flip_weights_many(const unet_flip *layers, int count, stencil_stream_t stream);
 /* The data gradient through a ReLU: dx = conv3x3(dy, wt) (flipped weights, taps
  * `dilation` apart) where gate > 0, else 0; gate has dx's shape (the layer's
  * input, itself a ReLU's output).  Equals the convolution without bias and

@@ -77,3 +77,30 @@ def test_head_gradient(cuda, shape):
     assert torch.equal(outs[0], (dy[..., None] * hw).to(torch.bfloat16))
     U._chk(L.unet_relu_bwd(R(V(outs[0])), R(V(x)), None), "relu")
     assert torch.equal(outs[1], outs[0])
+
+
+def test_optimizer_step_on_flat_and_rebound_tensors(cuda):
+    """The one-pass update equals the per-tensor one, also for a network whose
+    parameter the caller has replaced by a tensor of its own."""
+    import torch
+    from thesis_gb300 import unet as U
+    nets = [U.UNet(seed=3), U.UNet(seed=3)]
+    nets[1].params["e1a"]["w"] = nets[1].params["e1a"]["w"].clone()
+    for step in range(2):
+        for net in nets:
+            net.zero_grad()
+            g = torch.Generator(device="cuda").manual_seed(step)
+            for P in [net.params[n] for n, _, _ in U.LAYERS] + [net.head]:
+                for k in ("dw", "db"):
+                    assert not P[k].any()
+                    P[k].copy_(torch.randn(P[k].shape, device="cuda", generator=g))
+            net.adam_step(lr=1e-2)
+    for n, cin, cout in U.LAYERS:
+        for k in ("w", "b", "mw", "vw", "mb", "vb", "wb"):
+            assert torch.equal(nets[0].params[n][k], nets[1].params[n][k]), (n, k)
+        P = nets[0].params[n]
+        assert torch.equal(P["wb"], P["w"].to(torch.bfloat16))
+        U._chk(U._L().unet_flip_weights(U._p(P["wb"]), U._p(P["wt"]), cout, cin, None), "flip")
+        assert torch.equal(P["wt"], P["wb"].flip(1).permute(2, 1, 0)), n
+    for k in ("w", "b", "mw", "vw"):
+        assert torch.equal(nets[0].head[k], nets[1].head[k]), k

@@ -979,16 +979,30 @@ __global__ void k_bias_grad(Act dy, float *db) {
     }
 }
 
-__global__ void k_flip(const bf16 *__restrict__ w, bf16 *__restrict__ wt, int cout, int cin) {
-    const long long n = (long long)cout * 9 * cin;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int ci = (int)(i % cin);
-        const int tap = (int)((i / cin) % 9);
-        const int co = (int)(i / ((long long)cin * 9));
-        // wt[ci][tap'][co] with tap' = 8 - tap (ky -> 2-ky, kx -> 2-kx)
-        wt[((long long)ci * 9 + (8 - tap)) * cout + co] = w[i];
-    }
+// Weights [co][tap][ci] -> [ci][8 - tap][co] (ky -> 2-ky, kx -> 2-kx) of up to
+// kFlipMax layers in one launch: block (32-channel tiles of the layers in
+// turn, tap), through shared memory so that both sides are coalesced.
+constexpr int kFlipMax = 32;
+struct FlipTable {
+    const bf16 *w[kFlipMax];
+    bf16 *wt[kFlipMax];
+    int cout[kFlipMax], cin[kFlipMax];
+    int first[kFlipMax + 1];  // tiles of the layers before
+    int n;
+};
+__global__ void __launch_bounds__(256) k_flip(FlipTable t) {
+    __shared__ bf16 v[32][33];
+    int l = 0;
+    while (l + 1 < t.n && (int)blockIdx.x >= t.first[l + 1]) ++l;
+    const int cout = t.cout[l], cin = t.cin[l], tile = (int)blockIdx.x - t.first[l], nci = (cin + 31) / 32;
+    const int co0 = tile / nci * 32, ci0 = tile % nci * 32, tap = blockIdx.y;
+    const int a = (int)threadIdx.x & 31;
+    for (int b = (int)threadIdx.x >> 5; b < 32; b += 8)
+        if (co0 + b < cout && ci0 + a < cin) v[b][a] = t.w[l][((long long)(co0 + b) * 9 + tap) * cin + ci0 + a];
+    __syncthreads();
+    for (int b = (int)threadIdx.x >> 5; b < 32; b += 8)
+        if (ci0 + b < cin && co0 + a < cout)
+            t.wt[l][((long long)(ci0 + b) * 9 + (8 - tap)) * cout + co0 + a] = v[a][b];
 }
 
 // Element-wise kernels over 8-channel vectors of a view.
@@ -1582,11 +1596,33 @@ extern "C" int unet_conv3x3_fwd(const unet_act *x, const void *w, const float *b
     return unet_conv3x3_fwd_dil(x, w, b, y, relu, 1, s);
 }
 
+extern "C" int unet_flip_weights_many(const unet_flip *layers, int count, stencil_stream_t s) {
+    if (count < 0 || (count && !layers)) return fail(STENCIL_EINVAL, "bad arguments");
+    for (int k = 0; k < count; ++k)
+        if (!layers[k].w || !layers[k].wt || layers[k].cout < 1 || layers[k].cin < 1)
+            return fail(STENCIL_EINVAL, "bad arguments (layer %d)", k);
+    for (int k0 = 0; k0 < count; k0 += kFlipMax) {
+        FlipTable t;
+        t.n = std::min(kFlipMax, count - k0);
+        t.first[0] = 0;
+        for (int k = 0; k < t.n; ++k) {
+            const unet_flip &f = layers[k0 + k];
+            t.w[k] = static_cast<const bf16 *>(f.w);
+            t.wt[k] = static_cast<bf16 *>(f.wt);
+            t.cout[k] = f.cout;
+            t.cin[k] = f.cin;
+            t.first[k + 1] = t.first[k] + (f.cout + 31) / 32 * ((f.cin + 31) / 32);
+        }
+        k_flip<<<dim3(t.first[t.n], 9), 256, 0, STREAM(s)>>>(t);
+        int rc = cuda_fail(cudaGetLastError(), "flip launch");
+        if (rc) return rc;
+    }
+    return STENCIL_OK;
+}
+
 extern "C" int unet_flip_weights(const void *w, void *wt, int cout, int cin, stencil_stream_t s) {
-    if (!w || !wt || cout < 1 || cin < 1) return fail(STENCIL_EINVAL, "bad arguments");
-    k_flip<<<grid_for((long long)cout * 9 * cin), 256, 0, STREAM(s)>>>(
-        static_cast<const bf16 *>(w), static_cast<bf16 *>(wt), cout, cin);
-    return cuda_fail(cudaGetLastError(), "flip launch");
+    const unet_flip f = {w, wt, cout, cin};
+    return unet_flip_weights_many(&f, 1, s);
 }
 
 namespace {

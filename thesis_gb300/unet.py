@@ -47,6 +47,10 @@ class Act(ctypes.Structure):
                 ("c", ctypes.c_int), ("reserved", ctypes.c_int)]
 
 
+class Flip(ctypes.Structure):
+    _fields_ = [("w", ctypes.c_void_p), ("wt", ctypes.c_void_p), ("cout", ctypes.c_int), ("cin", ctypes.c_int)]
+
+
 _sig_done = False
 
 
@@ -64,6 +68,7 @@ def _L():
             "unet_conv3x3_wgrad_engine": [A, A, vp, vp, i, i, vp, ctypes.c_size_t, vp],
             "unet_wgrad_workspace_bytes": [A, A, ctypes.POINTER(ctypes.c_size_t)],
             "unet_flip_weights": [vp, vp, i, i, vp],
+            "unet_flip_weights_many": [ctypes.POINTER(Flip), i, vp],
             "unet_conv3x3_wgrad": [A, A, vp, vp, vp],
             "unet_conv3x3_dgrad_relu": [A, vp, A, A, i, vp],
             "unet_relu_bwd": [A, A, vp],
@@ -133,25 +138,43 @@ class UNet:
 
     # -- parameters --------------------------------------------------------
     def _alloc_state(self):
+        """Parameters, gradients and moments as views of one tensor each (in
+        one layout, 512-byte aligned), so that a step clears and updates them
+        in one pass."""
         import torch
-        for name, cin, cout in LAYERS:
-            P = self.params[name]
-            P["wb"] = torch.empty(P["w"].shape, dtype=torch.bfloat16, device=self.device)
-            P["wt"] = torch.empty((cin, 9, cout), dtype=torch.bfloat16, device=self.device)
-            for k in ("w", "b"):
-                P["d" + k] = torch.zeros_like(P[k])
-                P["m" + k] = torch.zeros_like(P[k])
-                P["v" + k] = torch.zeros_like(P[k])
+        tensors = [(self.params[name], k) for name, _, _ in LAYERS for k in ("w", "b")]
         self.head = {"w": self.head_w, "b": self.head_b}
-        for k in ("w", "b"):
-            self.head["d" + k] = torch.zeros_like(self.head[k])
-            self.head["m" + k] = torch.zeros_like(self.head[k])
-            self.head["v" + k] = torch.zeros_like(self.head[k])
+        tensors += [(self.head, k) for k in ("w", "b")]
+        offsets, n = [], 0
+        for P, k in tensors:
+            offsets.append(n)
+            n += -(-P[k].numel() // 128) * 128
+        self._flat = {k: torch.zeros(n, device=self.device) for k in ("w", "d", "m", "v")}
+        self._flat["wb"] = torch.zeros(n, dtype=torch.bfloat16, device=self.device)
+        self._views = []  # (dict, key, tensor) of every view of a flat tensor
+        for (P, k), o in zip(tensors, offsets):
+            shape, size = P[k].shape, P[k].numel()
+            self._flat["w"][o:o + size].copy_(P[k].reshape(-1))
+            for flat, key in (("w", k), ("d", "d" + k), ("m", "m" + k), ("v", "v" + k), ("wb", "wb")):
+                if flat != "wb" or (k == "w" and P is not self.head):
+                    P[key] = self._flat[flat][o:o + size].view(shape)
+                    self._views.append((P, key, P[key]))
+        self.head_w, self.head_b = self.head["w"], self.head["b"]
+        for name, cin, cout in LAYERS:
+            self.params[name]["wt"] = torch.empty((cin, 9, cout), dtype=torch.bfloat16, device=self.device)
         self.sync_bf16()
+
+    def _whole(self):
+        """Whether every tensor is still the view made above (a caller may
+        have put its own in the dicts)."""
+        return all(P[key] is t for P, key, t in self._views)
 
     def sync_bf16(self, stream=None):
         s = _stream(stream)
         L = _L()
+        if self._whole():
+            _chk(L.unet_to_bf16(_p(self._flat["w"]), _p(self._flat["wb"]), self._flat["w"].numel(), s), "unet_to_bf16")
+            return
         for name, cin, cout in LAYERS:
             P = self.params[name]
             _chk(L.unet_to_bf16(_p(P["w"]), _p(P["wb"]), P["w"].numel(), s), "unet_to_bf16")
@@ -261,15 +284,14 @@ class UNet:
     # -- backward ----------------------------------------------------------
     def _conv_bwd(self, name, x, gy, gx, s, relu=False):
         """gy holds the gradient before the layer's ReLU; accumulates dW/db,
-        writes dL/dx into gx (with relu: through the ReLU whose output x is)."""
+        writes dL/dx into gx (with relu: through the ReLU whose output x is;
+        the layer's flipped weights are in "wt")."""
         L = _L()
         P = self.params[name]
         d = DILATION.get(name, 1)
         _chk(L.unet_conv3x3_wgrad_engine(ctypes.byref(x), ctypes.byref(gy), _p(P["dw"]), _p(P["db"]), d, 0, None, 0, s),
              "wgrad " + name)
         if gx is not None:
-            cin, cout = P["w"].shape[2], P["w"].shape[0]
-            _chk(L.unet_flip_weights(_p(P["wb"]), _p(P["wt"]), cout, cin, s), "flip " + name)
             if relu:
                 rc = L.unet_conv3x3_dgrad_relu(ctypes.byref(gy), _p(P["wt"]), ctypes.byref(x), ctypes.byref(gx), d, s)
             else:
@@ -277,6 +299,9 @@ class UNet:
             _chk(rc, "dgrad " + name)
 
     def zero_grad(self):
+        if self._whole():
+            self._flat["d"].zero_()
+            return
         for name, _, _ in LAYERS:
             self.params[name]["dw"].zero_()
             self.params[name]["db"].zero_()
@@ -288,6 +313,11 @@ class UNet:
         s = _stream(stream)
         L = _L()
         V = view
+        flips = (Flip * len(LAYERS))()
+        for f, (name, cin, cout) in zip(flips, LAYERS):
+            P = self.params[name]
+            f.w, f.wt, f.cout, f.cin = P["wb"].data_ptr(), P["wt"].data_ptr(), cout, cin
+        _chk(L.unet_flip_weights_many(flips, len(LAYERS), s), "flip")
         _chk(L.unet_head_bwd_relu(ctypes.byref(V(B["d0b"])), _p(self.head["w"]), _p(B["dout"]),
                                   ctypes.byref(V(B["g_d0b"])), _p(self.head["dw"]), _p(self.head["db"]), s),
              "head_bwd")
@@ -329,6 +359,11 @@ class UNet:
         s = _stream(stream)
         L = _L()
         self.step += 1
+        if self._whole():
+            F = self._flat
+            _chk(L.unet_adam(_p(F["w"]), _p(F["d"]), _p(F["m"]), _p(F["v"]), _p(F["wb"]), F["w"].numel(), lr, beta1,
+                             beta2, eps, self.step, s), "adam")
+            return
         for name, _, _ in LAYERS:
             P = self.params[name]
             _chk(L.unet_adam(_p(P["w"]), _p(P["dw"]), _p(P["mw"]), _p(P["vw"]), _p(P["wb"]),
