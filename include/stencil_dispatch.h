@@ -73,7 +73,7 @@ enum {
                                           `temporal` sweeps per halo exchange, tile
                                           block_x * coarsen_x by block_y cells (0: chosen);
                                           larger 2-D grids: a grid barrier per sweep
-                                          (nx % 4 == 0, R <= 4); 3-D grids that fit
+                                          (R <= 4); 3-D grids that fit
                                           one cluster's shared memory go to CLUSTER */
     STENCIL_VARIANT_CLUSTER = 6        /* all sweeps on one thread-block cluster: the grid
                                           resident in its shared memory when it fits, else
@@ -378,8 +378,9 @@ STENCIL_API const char *stencil_strerror(int status);
 /* Text of the last failure on the calling thread (empty if none). */
 STENCIL_API const char *stencil_last_error(void);
 /* What this thread's last stencil_dispatch_ex (or stencil_run_host*) ran:
- * the engine ("stream3d", "stream3d-persistent", "rows3d", "tb3d", "cluster",
- * "base", "tile"; the first one when a dispatch uses two) and how many kernel
+ * the engine ("stream3d", "stream3d-persistent", "ragged3d-persistent",
+ * "rows3d", "rows2d-persistent", "tb2d-persistent", "tb3d", "cluster", "base",
+ * "tile"; the first one when a dispatch uses two) and how many kernel
  * launches it made (iterations for one launch per sweep, 1 for the
  * persistent engines).  For diagnostics and launch accounting. */
 STENCIL_API int stencil_last_dispatch(const char **engine, long long *kernel_launches);

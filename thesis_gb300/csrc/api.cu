@@ -240,7 +240,8 @@ static int choose_variant(const stencil_params &p) {
     const Geom g = make_geom(p);
     // 2-D: small grids every SM, temporally blocked (2-5x the one-cluster
     // engine); larger ones every sweep in one persistent launch
-    if (p.dims == 2 && p.iterations >= 8 && (tb2d_supported(g, 2) || rows2d_supported(g, 2)))
+    if (p.dims == 2 && p.iterations >= 8 &&
+        (tb2d_supported(g, 2) || rows2d_supported(g, 2) || rows2d_any_supported(g, 2)))
         return STENCIL_VARIANT_COOP;
     if (p.iterations >= 8 && cluster_resident(g, p.dims)) return STENCIL_VARIANT_CLUSTER;
     if (p.dims == 3 && stream3d_supported(g)) return STENCIL_VARIANT_SMEM_REGISTER;
@@ -328,13 +329,24 @@ int stencil_dispatch_ex(const stencil_params *p, float *d_u1, float *d_u2,
         float *res = nullptr;
         rc = run_tb2d(g, cur, nxt, p->iterations, p->temporal,
                       p->block_x * std::max(p->coarsen_x, 1), p->block_y, s, &res);
-        if (rc) return rc;
-        if (d_result) *d_result = res;
-        return STENCIL_OK;
+        // its exchange buffer cannot be made inside a graph capture: rows that
+        // are not 16-byte aligned go to the rows kernel then, which needs none
+        if (rc != STENCIL_EUNSUPPORTED || !rows2d_any_supported(g, 2)) {
+            if (rc) return rc;
+            if (d_result) *d_result = res;
+            return STENCIL_OK;
+        }
     }
     if (variant == STENCIL_VARIANT_COOP && p->dims == 2 && rows2d_supported(g, 2)) {
         float *res = nullptr;
         rc = run_rows2d(g, cur, nxt, p->iterations, s, &res);
+        if (rc) return rc;
+        if (d_result) *d_result = res;
+        return STENCIL_OK;
+    }
+    if (variant == STENCIL_VARIANT_COOP && rows2d_any_supported(g, p->dims)) {
+        float *res = nullptr;
+        rc = run_rows2d_any(g, cur, nxt, p->iterations, s, &res);
         if (rc) return rc;
         if (d_result) *d_result = res;
         return STENCIL_OK;
@@ -390,6 +402,18 @@ int stencil_dispatch_ex(const stencil_params *p, float *d_u1, float *d_u2,
         float *res = nullptr;
         rc = run_stream3d(g, cur, nxt, p->iterations, p->block_x ? 4 * p->block_x : 0,
                           p->block_y, s, &res, p->block_z, persistent);
+        if (rc) return rc;
+        if (d_result) *d_result = res;
+        return STENCIL_OK;
+    }
+    if (auto_pick && ragged3d_supported(g, p->dims) &&
+        (p->iterations >= 4 || cell_count(*p) >= (1LL << 22))) {
+        // 3-D rows that are not 16-byte aligned, left to the library; a few
+        // sweeps of a small grid are launched one by one (the persistent
+        // launch costs about 6 us more: 101 x 99 x 97 R = 2, one sweep 25 us
+        // against 19, 20 sweeps 8.5 us each against 16).
+        float *res = nullptr;
+        rc = run_ragged3d(g, cur, nxt, p->iterations, s, &res);
         if (rc) return rc;
         if (d_result) *d_result = res;
         return STENCIL_OK;

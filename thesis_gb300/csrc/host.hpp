@@ -85,11 +85,21 @@ void tb2d_release();
 // device that the kernel for g's radius can hold at once.
 bool rows2d_supported(const Geom &g, int dims);
 int rows2d_capacity(const Geom &g);
+// The same on rows that are not 16-byte aligned (nx % 4 != 0).
+bool rows2d_any_supported(const Geom &g, int dims);
+int run_rows2d_any(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res);
 // Row blocks of a rows sweep of g on `threads` threads: *hb rows per block,
 // *nblk blocks.
 void rows2d_plan(const Geom &g, long long threads, int *hb, int *nblk);
 int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res,
                int max_ctas = 0);
+// 3-D grids whose rows are not 16-byte aligned (nx % 4 != 0, R <= 4): all
+// sweeps in one cooperative launch (k_ragged.cu).
+bool ragged3d_supported(const Geom &g, int dims);
+int run_ragged3d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res);
+// Resident CTAs of a kernel on the whole device; sets its shared-memory limit
+// (k_stream.cu).
+int grid_resident_ctas(const void *fn, int threads, int smem, int *ctas);
 // All sweeps of one grid on one thread-block cluster (k_cluster.cu).
 int run_cluster(const Geom &g, int dims, float *a, float *b, int iters, cudaStream_t s,
                 float **res);

@@ -32,14 +32,17 @@ namespace {
 
 constexpr int kRowsThreads = 512;
 
-template <int R, bool L1>
-__global__ void __launch_bounds__(kRowsThreads, R <= 2 ? 2 : 1)
+// ANY: rows that are not 16-byte aligned, one column per thread
+// (rows2d_sweep_any).
+template <int R, bool L1, bool ANY = false>
+__global__ void __launch_bounds__(kRowsThreads, R <= 2 || ANY ? 2 : 1)
     k_rows2d(float *a, float *b, Geom g, int hb, int nblk, int iters, unsigned *bar) {
     __shared__ int s_ok;
     for (int sw = 0; sw < iters; ++sw) {
         const float *src = (sw & 1) ? b : a;
         float *dst = (sw & 1) ? a : b;
-        rows2d_sweep<R, kRowsThreads, L1>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
+        if constexpr (ANY) rows2d_sweep_any<R, kRowsThreads>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
+        else rows2d_sweep<R, kRowsThreads, L1>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
         if (sw + 1 < iters) {
             // every CTA's writes of this sweep before any CTA's next reads
             __syncthreads();
@@ -76,27 +79,33 @@ RowsFn rows_fn(int r, bool l1 = false) {
     }
 }
 
+RowsFn rows_any_fn(int r) {
+    return r == 1 ? k_rows2d<1, true, true> : r == 2 ? k_rows2d<2, true, true>
+         : r == 3 ? k_rows2d<3, true, true> : k_rows2d<4, true, true>;
+}
+
 bool rows_l1() {
     const char *e = std::getenv("STENCIL_ROWS_L1");
     return !(e && e[0] == '0');
 }
 
-// Resident CTAs of the radius-r kernel (once per radius and device).
-int rows_ctas(int r) {
+// Resident CTAs of the radius-r kernel (once per kernel and device).
+int rows_ctas(int r, bool any = false) {
     static std::mutex mu;
-    static std::vector<std::pair<int, int>> cache;  // (device * 8 + r, ctas)
+    static std::vector<std::pair<int, int>> cache;  // (device * 16 + 8 * any + r, ctas)
     const int dev = current_device();
     std::lock_guard<std::mutex> lock(mu);
+    const int key = dev * 16 + 8 * any + r;
     for (auto &c : cache)
-        if (c.first == dev * 8 + r) return c.second;
+        if (c.first == key) return c.second;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void *>(rows_fn(r)),
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void *>(any ? rows_any_fn(r) : rows_fn(r)),
                                                       kRowsThreads, 0) != cudaSuccess) {
         cudaGetLastError();
         n = 0;
     }
     const int ctas = n * num_sms();
-    cache.push_back({dev * 8 + r, ctas});
+    cache.push_back({key, ctas});
     return ctas;
 }
 
@@ -105,6 +114,13 @@ int rows_ctas(int r) {
 bool rows2d_supported(const Geom &g, int dims) {
     return dims == 2 && g.sy % 4 == 0 && g.radius >= 1 && g.radius <= 4 &&
            (long long)(g.sy / 4) * (g.ny - 2 * g.radius) < (1LL << 31) && rows_ctas(g.radius) > 0;
+}
+
+// Rows that are not 16-byte aligned: fewer than 2^31 (column, row) pairs, and
+// row offsets that the kernel's 64-bit products hold.
+bool rows2d_any_supported(const Geom &g, int dims) {
+    return dims == 2 && g.sy % 4 != 0 && g.radius >= 1 && g.radius <= 4 &&
+           (long long)g.nx * g.ny < (1LL << 31) && rows_ctas(g.radius, true) > 0;
 }
 
 int rows2d_capacity(const Geom &g) { return rows_ctas(g.radius); }
@@ -120,6 +136,30 @@ void rows2d_plan(const Geom &g, long long threads, int *hb, int *nblk) {
     h = std::max(1, std::min(h, rows));
     *hb = h;
     *nblk = (rows + h - 1) / h;
+}
+
+// The persistent rows kernel on rows that are not 16-byte aligned.  Row blocks
+// as rows2d_plan's, for one column per thread: about four items per thread, 4
+// to 64 rows.
+int run_rows2d_any(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res) {
+    if (res) *res = (iters & 1) ? b : a;
+    if (iters <= 0) return STENCIL_OK;
+    const int ctas = rows_ctas(g.radius, true);
+    const int cols = g.nx - 2 * g.radius, rows = g.ny - 2 * g.radius;
+    int hb = (int)std::min<long long>(64, std::max<long long>(4, (long long)cols * rows / (4LL * ctas * kRowsThreads)));
+    hb = std::min(hb, rows);
+    int nblk = (rows + hb - 1) / hb;
+    const int grid = (int)std::min<long long>(ctas, ((long long)cols * nblk + kRowsThreads - 1) / kRowsThreads);
+    unsigned *bar = nullptr;
+    int rc = grid_bar_slot(s, &bar);
+    if (rc) return rc;
+    Geom gg = g;
+    int n = iters;
+    void *args[] = {&a, &b, &gg, &hb, &nblk, &n, &bar};
+    ST_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(rows_any_fn(g.radius)), dim3(grid),
+                                        dim3(kRowsThreads), args, 0, s));
+    note_launches("rows2d-persistent", 1);
+    return STENCIL_OK;
 }
 
 int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res,

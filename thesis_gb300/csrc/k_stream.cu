@@ -156,6 +156,14 @@ int kernel_residency(const void *fn, int threads, int smem, int *per_sm) {
 
 }  // namespace
 
+// Resident CTAs of a kernel on the whole device (kernel_residency).
+int grid_resident_ctas(const void *fn, int threads, int smem, int *ctas) {
+    int per_sm = 0;
+    const int rc = kernel_residency(fn, threads, smem, &per_sm);
+    *ctas = per_sm * num_sms();
+    return rc;
+}
+
 bool stream3d_supported(const Geom &g) {
     return g.sy % 4 == 0 && (g.radius >= 1 && g.radius <= 4);
 }

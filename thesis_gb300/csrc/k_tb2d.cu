@@ -109,10 +109,13 @@ template <int R, bool LEGACY, int NI>
 __global__ void __launch_bounds__(kTb2Threads, 1)
     k_tb2d(float *g0, float *g1, Geom g, Tb2Plan p, int iters, unsigned long long *xch) {
     extern __shared__ __align__(16) float tb2_smem[];
-    // nx: the grid's width (update region x < nx - R); px: its row pitch (a
-    // multiple of 4; cells nx .. px-1 of a row are padding that no update
-    // reads and no sweep writes)
-    const int nx = g.nx, ny = g.ny, px = (int)g.sy, pw = p.pw;
+    // nx: the grid's width (update region x < nx - R); px: the row in whole
+    // chunks (cells nx .. px-1 are padding that no update reads and no sweep
+    // writes); pitch: the row pitch in the caller's buffers, px unless rows are
+    // not 16-byte aligned (cells are then loaded and stored one by one, at the
+    // launch's start and end only: 256 x 255 0.40 us a sweep, as 256^2)
+    const int nx = g.nx, ny = g.ny, pitch = (int)g.sy, px = (pitch + 3) & ~3, pw = p.pw;
+    const bool aligned = pitch == px;
     float *const S0 = tb2_smem, *const S1 = tb2_smem + pw * p.ph;
     const int tile = blockIdx.x, ntiles = p.tiles_x * p.tiles_y;
     const int x0 = (tile % p.tiles_x) * p.tx, y0 = (tile / p.tiles_x) * p.ty;
@@ -194,8 +197,17 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
         const int n = cw * (eyb - eya);
         for (int u = threadIdx.x; u < n; u += kTb2Threads) {
             const int y = eya + u / cw, x = exa + 4 * (u % cw);
-            const long long gi = (long long)y * px + x;
+            const long long gi = (long long)y * pitch + x;
             const int si = (y - oy) * pw + (x - ox);
+            if (!aligned) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (x + e < nx) {
+                        S0[si + e] = __ldcg(g0 + gi + e);
+                        if (y < R || y >= ny - R || x + e < R || x + e >= nx - R) S1[si + e] = __ldcg(g1 + gi + e);
+                    }
+                continue;
+            }
             *reinterpret_cast<float4 *>(S0 + si) = __ldcg(reinterpret_cast<const float4 *>(g0 + gi));
             if (y < R || y >= ny - R) {
                 *reinterpret_cast<float4 *>(S1 + si) = __ldcg(reinterpret_cast<const float4 *>(g1 + gi));
@@ -304,9 +316,9 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
         for (int u = threadIdx.x; u < n; u += kTb2Threads) {
             const int y = ya + u / cw, x = x0 + 4 * (u % cw);
             const int si = (y - oy) * pw + (x - ox);
-            const long long gi = (long long)y * px + x;
+            const long long gi = (long long)y * pitch + x;
             const float4 vn = tb2_ld4(Sn + si), vp = tb2_ld4(Sp + si);
-            if (x >= R && x + 3 < nx - R) {
+            if (aligned && x >= R && x + 3 < nx - R) {
                 __stcg(reinterpret_cast<float4 *>(Gn + gi), vn);
                 if (iters >= 2) __stcg(reinterpret_cast<float4 *>(Gp + gi), vp);
             } else {
@@ -361,7 +373,7 @@ bool make_plan(const Geom &g, int t, int tx, int ty, int max_ctas, Tb2Plan *p) {
     q.hy = t * R;
     q.pw = tx + 2 * q.hx;
     q.ph = ty + 2 * q.hy;
-    q.tiles_x = ((int)g.sy + tx - 1) / tx;  // tiles cover the row pitch
+    q.tiles_x = (roundup4((int)g.sy) + tx - 1) / tx;  // tiles cover the row in whole chunks
     q.tiles_y = (g.ny + ty - 1) / ty;
     if ((long long)q.tiles_x * q.tiles_y > max_ctas) return false;
     // the halo reaches the adjacent tiles only
@@ -525,7 +537,7 @@ void tb2d_release() {
 }
 
 bool tb2d_supported(const Geom &g, int dims) {
-    if (dims != 2 || g.sy % 4 || g.radius < 1 || g.radius > 4) return false;
+    if (dims != 2 || g.radius < 1 || g.radius > 4) return false;
     const int ctas = tb2_max_ctas(g.radius);
     Tb2Plan p;
     return ctas > 0 && choose_plan(g, 1, 1, 0, 0, ctas, &p);
@@ -533,8 +545,7 @@ bool tb2d_supported(const Geom &g, int dims) {
 
 int run_tb2d(const Geom &g, float *a, float *b, int iters, int temporal, int tile_x, int tile_y,
              cudaStream_t s, float **res) {
-    if (g.sy % 4 || g.radius < 1 || g.radius > 4)
-        return fail(STENCIL_EUNSUPPORTED, "2-D temporal blocking needs a row pitch %% 4 == 0 and R <= 4");
+    if (g.radius < 1 || g.radius > 4) return fail(STENCIL_EUNSUPPORTED, "2-D temporal blocking needs R <= 4");
     const int ctas = tb2_max_ctas(g.radius);
     Tb2Plan p;
     // a caller tile (then a caller depth) that does not fit falls back to the
