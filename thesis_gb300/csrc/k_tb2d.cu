@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "host.hpp"
@@ -268,38 +269,40 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
         kk = min(T, iters - done);
         plan_block(kk);
         // Read the halo ring from the neighbours' tiles, waiting for block
-        // blk: every pair of a thread is requested before any is checked, so
-        // the common case costs one L2 round trip.
+        // blk: every pair of a thread is requested before any is checked, and
+        // again those that have not arrived, so the wait is that of the
+        // slowest (about two L2 round trips).
         bool ok = true;
         {
             unsigned long long a[NP], b[NP];
+            unsigned want = 0;
+            uint64_t t0 = 0;
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                a[i] = b[i] = 0;
-                if (ring_w[i] >= 0)
-                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
-                                 : "=l"(a[i]), "=l"(b[i])
-                                 : "l"(slot + ring_w[i])
-                                 : "memory");
-            }
+            for (int i = 0; i < NP; ++i)
+                if (ring_w[i] >= 0) want |= 1u << i;
+            while (want && ok) {
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                if (ring_w[i] < 0) continue;
-                uint64_t t0 = 0;
-                while (ok && ((unsigned)(a[i] >> 32) != blk || (unsigned)(b[i] >> 32) != blk)) {
+                for (int i = 0; i < NP; ++i)
+                    if ((want >> i) & 1u)
+                        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
+                                     : "=l"(a[i]), "=l"(b[i])
+                                     : "l"(slot + ring_w[i])
+                                     : "memory");
+#pragma unroll
+                for (int i = 0; i < NP; ++i)
+                    if (((want >> i) & 1u) && (unsigned)(a[i] >> 32) == blk && (unsigned)(b[i] >> 32) == blk) {
+                        want &= ~(1u << i);
+                        *reinterpret_cast<float2 *>(Sw + ring_s[i]) =
+                            make_float2(__uint_as_float((unsigned)a[i]), __uint_as_float((unsigned)b[i]));
+                    }
+                if (want) {
                     const uint64_t t = globaltimer_ns();
                     if (!t0) t0 = t;
                     else if (t - t0 > kWaitLimitNs) {
                         report_status(kStatusTimeout);
                         ok = false;
                     }
-                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
-                                 : "=l"(a[i]), "=l"(b[i])
-                                 : "l"(slot + ring_w[i])
-                                 : "memory");
                 }
-                *reinterpret_cast<float2 *>(Sw + ring_s[i]) =
-                    make_float2(__uint_as_float((unsigned)a[i]), __uint_as_float((unsigned)b[i]));
             }
         }
         if (!__syncthreads_and(ok)) return;
@@ -334,6 +337,255 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same engine with the extended tile in registers, for tiles of at most
+// 128 cells a row and 512 threads of up to four rows (R = 1) or three (R = 2).  A row lies across LW lanes (4 cells each) and
+// a thread holds its chunk column of RW rows, in both ping-pong buffers.  In a
+// sweep the y-neighbours are the thread's own registers except R rows above
+// and below its block, which pass through shared memory (double-buffered by
+// sweep parity: one CTA barrier), and the x-neighbours come from the adjacent
+// lanes by shuffles.  Every sweep updates the whole tile: what lies beyond the
+// shrinking valid region is garbage that never reaches a valid cell, so there
+// is no region to test; cells outside the update region keep the value that
+// their buffer holds (the border bands of the two buffers may differ).  The
+// exchange is the one above, straight from and to the registers that own the
+// cells.
+// What bounds it: latency (a sweep is a barrier, two dependent shared-memory
+// accesses and some 30 dependent instructions a row, issued by seven warps)
+// and the exchange, two to three L2 round trips.  GB300, us a sweep, against
+// the form in shared memory: 256^2 R = 1 0.308 / 0.398, R = 2 0.497 / 0.590; 512^2
+// 0.57 / 0.74; 128^2 0.29 / 0.32.  Polling every chunk before checking any (the
+// form above checks one after the other) took an exchange from 1.8 to 1.0 us;
+// packed f32x2 sums 0.320 -> 0.308; five or six rows a thread spill.
+// ---------------------------------------------------------------------------
+template <int R, int LW, int RW>
+__global__ void __launch_bounds__(kTb2Threads, 1)
+    k_tb2d_reg(float *g0, float *g1, Geom g, Tb2Plan p, int iters, unsigned long long *xch) {
+    static_assert(RW >= R, "a block's neighbours are the adjacent blocks");
+    constexpr int C = 4 * R;
+    constexpr bool POW2 = (C & (C - 1)) == 0;
+    extern __shared__ __align__(16) float tb2_smem[];
+    const int nx = g.nx, ny = g.ny, pitch = (int)g.sy, px = (pitch + 3) & ~3;
+    const bool aligned = pitch == px;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    // halo rows [parity][first / last][R][nt + 2 LW], LW spare entries before
+    // and behind the threads'
+    const int hrow = nt + 2 * LW;
+    float4 *halo = reinterpret_cast<float4 *>(tb2_smem) + LW;
+    const int tile = blockIdx.x, ntiles = p.tiles_x * p.tiles_y;
+    const int x0 = (tile % p.tiles_x) * p.tx, y0 = (tile / p.tiles_x) * p.ty;
+    const int x1 = min(x0 + p.tx, px), y1 = min(y0 + p.ty, ny);
+    const size_t tile_words = (size_t)p.tx * p.ty;
+    const int T = iters >= 2 ? min(p.t, iters - 1) : 1;
+    const int x = x0 - p.hx + 4 * (tid % LW), yb = y0 - p.hy + (tid / LW) * RW;  // this thread's chunk and first row
+    const bool col = tid % LW < p.pw / 4 && x >= 0 && x < px;
+    unsigned mask = 0;  // cells of the chunk inside the update region
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (col && x + e >= R && x + e < nx - R) mask |= 1u << e;
+    float4 A[RW], B[RW];
+    int pub[RW], ring[RW];  // word offsets in the exchange slot; -1: none
+    unsigned live = 0;      // rows inside the update region
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const int y = yb + r;
+        A[r] = B[r] = zero;
+        pub[r] = ring[r] = -1;
+        if (y >= R && y < ny - R) live |= 1u << r;
+        if (!col || y < 0 || y >= ny || y >= y0 - p.hy + p.ph) continue;
+        const long long gi = (long long)y * pitch + x;
+        const bool edge = y < R || y >= ny - R || mask != 15u;  // the second buffer is read in its border band only
+        if (aligned) {
+            A[r] = __ldcg(reinterpret_cast<const float4 *>(g0 + gi));
+            if (edge) B[r] = __ldcg(reinterpret_cast<const float4 *>(g1 + gi));
+        } else {
+            float va[4] = {0.f, 0.f, 0.f, 0.f}, vb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (x + e < nx) {
+                    va[e] = __ldcg(g0 + gi + e);
+                    if (edge) vb[e] = __ldcg(g1 + gi + e);
+                }
+            A[r] = make_float4(va[0], va[1], va[2], va[3]);
+            B[r] = make_float4(vb[0], vb[1], vb[2], vb[3]);
+        }
+        const int ocx = x / p.tx, ocy = y / p.ty;
+        const int word = (int)((ocy * p.tiles_x + ocx) * tile_words) + (y - ocy * p.ty) * p.tx + (x - ocx * p.tx);
+        if (x >= x0 && x < x1 && y >= y0 && y < y1) pub[r] = word;
+        else ring[r] = word;
+    }
+    for (int i = tid; i < 2 * 2 * R * hrow; i += nt) reinterpret_cast<float4 *>(tb2_smem)[i] = zero;
+    __syncthreads();
+
+    int par = 0;
+    // out where the cell is in the update region, else what its buffer holds
+    unsigned sel[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sel[e] = (mask >> e) & 1u ? 0xffffffffu : 0u;
+    auto keep = [](float out, float old, unsigned m) {
+        return __uint_as_float((__float_as_uint(out) & m) | (__float_as_uint(old) & ~m));
+    };
+    const bool all_live = __all_sync(0xffffffffu, live == (1u << RW) - 1u);
+    auto sweep_rows = [&](const float4 (&S)[RW], float4 (&D)[RW], auto whole) {
+        float4 *first = halo + par * 2 * R * hrow, *last = first + R * hrow;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            first[i * hrow + tid] = S[i];
+            last[i * hrow + tid] = S[RW - R + i];
+        }
+        __syncthreads();
+        float4 up[R], dn[R];  // rows -R .. -1 and RW .. RW+R-1
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            up[i] = last[i * hrow + tid - LW];
+            dn[i] = first[i * hrow + tid + LW];
+        }
+        par ^= 1;
+        auto row = [&](int r) -> const float4 & { return r < 0 ? up[R + r] : r < RW ? S[r] : dn[r - RW]; };
+#pragma unroll
+        for (int q = 0; q < RW; ++q) {
+            // rows that need no halo row first
+            const int mid = RW > 2 * R ? RW - 2 * R : 0;
+            const int r = q < mid ? R + q : (q - mid < R ? q - mid : RW - 1 - (q - mid - R));
+            const float4 c = S[r];
+            float w[4 + 2 * R];
+#pragma unroll
+            for (int o = 0; o < R; ++o) {
+                w[o] = __shfl_up_sync(0xffffffffu, f4get(c, 4 - R + o), 1, LW);
+                w[R + 4 + o] = __shfl_down_sync(0xffffffffu, f4get(c, o), 1, LW);
+            }
+            w[R] = c.x, w[R + 1] = c.y, w[R + 2] = c.z, w[R + 3] = c.w;
+            // x sums of single cells, y sums and the division of pairs (the same
+            // roundings)
+            float2 a0, a1;
+            {
+                float acc[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] = POW2 ? w[e] : 0.0f + w[e];
+#pragma unroll
+                for (int o = 1; o <= 2 * R; ++o) {
+                    if (o == R) continue;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[e] += w[e + o];
+                }
+                a0 = make_float2(acc[0], acc[1]);
+                a1 = make_float2(acc[2], acc[3]);
+            }
+#pragma unroll
+            for (int o = -R; o <= R; ++o) {
+                if (!o) continue;
+                const float4 v = row(r + o);
+                a0 = fadd2(a0, make_float2(v.x, v.y));
+                a1 = fadd2(a1, make_float2(v.z, v.w));
+            }
+            if (POW2) {
+                const float2 rc = make_float2(1.0f / C, 1.0f / C), z2 = make_float2(0.f, 0.f);
+                a0 = ffma2(a0, rc, z2);
+                a1 = ffma2(a1, rc, z2);
+            } else {
+                a0 = make_float2(div_coeff<C>(a0.x), div_coeff<C>(a0.y));
+                a1 = make_float2(div_coeff<C>(a1.x), div_coeff<C>(a1.y));
+            }
+            float out[4] = {a0.x, a0.y, a1.x, a1.y};
+            if (g.legacy)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) out[e] -= w[R + e];
+            if (!whole.value && !((live >> r) & 1u)) continue;
+            D[r].x = keep(out[0], D[r].x, sel[0]);
+            D[r].y = keep(out[1], D[r].y, sel[1]);
+            D[r].z = keep(out[2], D[r].z, sel[2]);
+            D[r].w = keep(out[3], D[r].w, sel[3]);
+        }
+    };
+    auto sweep = [&](const float4 (&S)[RW], float4 (&D)[RW]) {
+        if (all_live) sweep_rows(S, D, std::true_type());
+        else sweep_rows(S, D, std::false_type());
+    };
+    // Publishes the owned cells of S and reads the others of the tile from
+    // their owners, waiting for block blk (see above).
+    auto exchange = [&](float4 (&S)[RW], unsigned blk) -> bool {
+        unsigned long long *slot = xch + (size_t)(blk & 1) * ntiles * tile_words;
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+            if (pub[r] >= 0) {
+                asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot + pub[r]), "l"(tb2_word(S[r].x, blk)),
+                             "l"(tb2_word(S[r].y, blk)) : "memory");
+                asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot + pub[r] + 2),
+                             "l"(tb2_word(S[r].z, blk)), "l"(tb2_word(S[r].w, blk)) : "memory");
+            }
+        // every chunk is requested before any is checked, and again those
+        // that have not arrived: the wait is that of the slowest
+        unsigned long long v[RW][4];
+        unsigned want = 0;
+        uint64_t t0 = 0;
+        bool ok = true;
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+            if (ring[r] >= 0) want |= 1u << r;
+        while (want && ok) {
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+                if ((want >> r) & 1u) {
+                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[r][0]), "=l"(v[r][1]) : "l"(slot + ring[r]) : "memory");
+                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[r][2]), "=l"(v[r][3]) : "l"(slot + ring[r] + 2) : "memory");
+                }
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+                if (((want >> r) & 1u) && (unsigned)(v[r][0] >> 32) == blk && (unsigned)(v[r][1] >> 32) == blk &&
+                    (unsigned)(v[r][2] >> 32) == blk && (unsigned)(v[r][3] >> 32) == blk) {
+                    want &= ~(1u << r);
+                    S[r] = make_float4(__uint_as_float((unsigned)v[r][0]), __uint_as_float((unsigned)v[r][1]),
+                                       __uint_as_float((unsigned)v[r][2]), __uint_as_float((unsigned)v[r][3]));
+                }
+            if (want) {
+                const uint64_t t = globaltimer_ns();
+                if (!t0) t0 = t;
+                else if (t - t0 > kWaitLimitNs) {
+                    report_status(kStatusTimeout);
+                    ok = false;
+                }
+            }
+        }
+        return __syncthreads_and(ok) != 0;
+    };
+
+    int cur = 0;  // 0: A holds the newest state
+    unsigned blk = 0;
+    for (int done = 0; done < iters;) {
+        const int kk = min(T, iters - done);
+#pragma unroll 1
+        for (int k = 0; k < kk; ++k, cur ^= 1) {
+            if (cur == 0) sweep(A, B);
+            else sweep(B, A);
+        }
+        done += kk;
+        ++blk;
+        if (done >= iters) break;
+        if (!(cur == 0 ? exchange(A, blk) : exchange(B, blk))) return;
+    }
+    // Owned cells of the update region back to the caller's buffers: the last
+    // sweep to the result buffer, the one before to the other.
+    float *Gn = (iters & 1) ? g1 : g0, *Gp = (iters & 1) ? g0 : g1;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        if (pub[r] < 0 || !((live >> r) & 1u)) continue;
+        const float4 vn = cur ? B[r] : A[r], vp = cur ? A[r] : B[r];
+        const long long gi = (long long)(yb + r) * pitch + x;
+        if (aligned && mask == 15u) {
+            __stcg(reinterpret_cast<float4 *>(Gn + gi), vn);
+            if (iters >= 2) __stcg(reinterpret_cast<float4 *>(Gp + gi), vp);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if ((mask >> e) & 1u) {
+                    Gn[gi + e] = f4get(vn, e);
+                    if (iters >= 2) Gp[gi + e] = f4get(vp, e);
+                }
+        }
+    }
+}
+
 using Tb2Fn = void (*)(float *, float *, Geom, Tb2Plan, int, unsigned long long *);
 
 template <int R, bool LEGACY>
@@ -359,6 +611,43 @@ int plan_items(const Tb2Plan &p) {
 }
 
 int roundup4(int v) { return (v + 3) & ~3; }
+
+// The register form's kernel for lw lanes a row and rw rows a thread, null if
+// there is none (radii above 2: their halo rows and neighbour values leave too
+// few registers; 256^2 R = 4 measured 1.13 us a sweep against 0.87).
+template <int LW>
+Tb2Fn tb2_reg_fn_lw(int r, int rw) {
+    if (r == 1) return rw == 1 ? k_tb2d_reg<1, LW, 1> : rw == 2 ? k_tb2d_reg<1, LW, 2>
+                     : rw == 3 ? k_tb2d_reg<1, LW, 3> : rw == 4 ? k_tb2d_reg<1, LW, 4> : nullptr;
+    if (r == 2) return rw == 2 ? k_tb2d_reg<2, LW, 2> : rw == 3 ? k_tb2d_reg<2, LW, 3> : nullptr;
+    return nullptr;
+}
+Tb2Fn tb2_reg_fn(int r, int lw, int rw) { return lw == 16 ? tb2_reg_fn_lw<16>(r, rw) : tb2_reg_fn_lw<32>(r, rw); }
+
+// The register form of a plan -- lanes a row (lw, 0: the extended tile does not
+// fit), rows a thread, threads, dynamic shared memory -- and its modelled SM
+// cycles per sweep: a + b * warps + x / T for each (R, rows a thread), fitted
+// to 2700 timed plans of 64^2 to 512^2 (6 to 9 % rms; the model's choice is
+// within 8 % of the best plan on each).
+struct Tb2Reg {
+    int lw, rw, threads, smem;
+    double cost;
+};
+Tb2Reg reg_plan(int r, const Tb2Plan &p) {
+    static const struct { int r, rw; double a, b, x; } model[] = {
+        {1, 1, 68, 27, 1930}, {1, 2, 174, 28, 2030}, {1, 3, 204, 33, 2280}, {1, 4, 342, 27, 2840},
+        {2, 2, 236, 54, 2210}, {2, 3, 248, 58, 2370}};
+    Tb2Reg best = {0, 0, 0, 0, 1e30};
+    if (p.pw > 128) return best;
+    const int lw = p.pw <= 64 ? 16 : 32;
+    for (const auto &m : model) {
+        if (m.r != r) continue;
+        const int nt = (lw * ((p.ph + m.rw - 1) / m.rw) + 31) / 32 * 32;
+        const double c = m.a + m.b * (nt / 32) + m.x / p.t;
+        if (nt <= kTb2Threads && c < best.cost) best = {lw, m.rw, nt, 4 * r * (nt + 2 * lw) * 16, c};
+    }
+    return best;
+}
 
 // Fills the geometry of a (tile, T) choice; false if it does not fit the
 // engine's limits (one CTA per SM, items per thread, shared memory).
@@ -438,7 +727,7 @@ bool choose_plan(const Geom &g, int iters, int temporal, int tile_x, int tile_y,
                 if (tile_y > 0 && ty != tile_y) continue;
                 Tb2Plan q;
                 if (!make_plan(g, t, tx, ty, max_ctas, &q)) continue;
-                const double c = plan_cost(g, q);
+                const double c = std::min(plan_cost(g, q), reg_plan(g.radius, q).cost);
                 if (c < best - 1e-9) {
                     best = c;
                     bestp = q;
@@ -518,6 +807,18 @@ int tb2_max_ctas(int r) {
             }
             n = std::min(n, m);
         }
+    for (int lw : {16, 32})
+        for (int rw = 1; rw <= 4; ++rw) {
+            const void *fn = reinterpret_cast<const void *>(tb2_reg_fn(r, lw, rw));
+            int m = 0;
+            if (!fn) continue;
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTb2SmemMax) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, fn, kTb2Threads, kTb2SmemMax) != cudaSuccess) {
+                cudaGetLastError();
+                m = 0;
+            }
+            n = std::min(n, m);
+        }
     const int ctas = n >= 1 ? std::min(num_sms(), kTb2MaxTiles) : 0;
     cache.push_back({dev * 8 + r, ctas});
     return ctas;
@@ -556,16 +857,20 @@ int run_tb2d(const Geom &g, float *a, float *b, int iters, int temporal, int til
         return fail(STENCIL_EUNSUPPORTED, "grid too large for one tile per SM");
     if (res) *res = (iters & 1) ? b : a;
     if (iters <= 0) return STENCIL_OK;
-    const void *fn = reinterpret_cast<const void *>(tb2_fn(g.radius, g.legacy != 0, plan_items(p)));
-    const int grid = p.tiles_x * p.tiles_y;
-    const size_t smem = 2ull * p.pw * p.ph * sizeof(float);
+    // in registers where the models say so
+    Tb2Reg reg = reg_plan(g.radius, p);
+    if (reg.cost >= plan_cost(g, p)) reg.lw = 0;
+    const void *fn = reg.lw ? reinterpret_cast<const void *>(tb2_reg_fn(g.radius, reg.lw, reg.rw))
+                            : reinterpret_cast<const void *>(tb2_fn(g.radius, g.legacy != 0, plan_items(p)));
+    const int grid = p.tiles_x * p.tiles_y, threads = reg.lw ? reg.threads : kTb2Threads;
+    const size_t smem = reg.lw ? (size_t)reg.smem : 2ull * p.pw * p.ph * sizeof(float);
     unsigned long long *xch = nullptr;
     int rc = xch_slot(s, 2ull * grid * p.tx * p.ty * sizeof(unsigned long long), &xch);
     if (rc) return rc;
     Geom gg = g;
     int n = iters;
     void *args[] = {&a, &b, &gg, &p, &n, &xch};
-    ST_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kTb2Threads), args, smem, s));
+    ST_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, s));
     note_launches("tb2d-persistent", 1);
     return STENCIL_OK;
 }
