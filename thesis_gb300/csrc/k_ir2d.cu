@@ -356,34 +356,37 @@ __global__ void __launch_bounds__(kIr2Threads, 1) k_ir2d(Geom g, Ir2Plan p, Ir2A
         }
         kk = min(T, a.m - done);
         plan_block(kk);
+        // every quad is requested before any is checked, and again those that
+        // have not arrived: the wait is that of the slowest
         {
             unsigned long long lo[NP], hi[NP];
+            unsigned want = 0;
+            uint64_t t0 = 0;
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                lo[i] = hi[i] = 0;
-                if (ring_w[i] >= 0)
-                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
-                                 : "=l"(lo[i]), "=l"(hi[i])
-                                 : "l"(slot + 2 * (size_t)ring_w[i])
-                                 : "memory");
-            }
+            for (int i = 0; i < NP; ++i)
+                if (ring_w[i] >= 0) want |= 1u << i;
+            while (want && ok) {
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                if (ring_w[i] < 0) continue;
-                uint64_t t0 = 0;
-                while (ok && ((unsigned)(lo[i] >> 32) != tag || (unsigned)(hi[i] >> 32) != tag)) {
+                for (int i = 0; i < NP; ++i)
+                    if ((want >> i) & 1u)
+                        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
+                                     : "=l"(lo[i]), "=l"(hi[i])
+                                     : "l"(slot + 2 * (size_t)ring_w[i])
+                                     : "memory");
+#pragma unroll
+                for (int i = 0; i < NP; ++i)
+                    if (((want >> i) & 1u) && (unsigned)(lo[i] >> 32) == tag && (unsigned)(hi[i] >> 32) == tag) {
+                        want &= ~(1u << i);
+                        *reinterpret_cast<uint2 *>(Sw + ring_s[i]) = make_uint2((unsigned)lo[i], (unsigned)hi[i]);
+                    }
+                if (want) {
                     const uint64_t t = globaltimer_ns();
                     if (!t0) t0 = t;
                     else if (t - t0 > kWaitLimitNs) {
                         report_status(kStatusTimeout);
                         ok = false;
                     }
-                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
-                                 : "=l"(lo[i]), "=l"(hi[i])
-                                 : "l"(slot + 2 * (size_t)ring_w[i])
-                                 : "memory");
                 }
-                *reinterpret_cast<uint2 *>(Sw + ring_s[i]) = make_uint2((unsigned)lo[i], (unsigned)hi[i]);
             }
         }
         if (!__syncthreads_and(ok)) return;
@@ -414,6 +417,225 @@ __global__ void __launch_bounds__(kIr2Threads, 1) k_ir2d(Geom g, Ir2Plan p, Ir2A
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same step with the correction in registers (R = 1, grown tiles of at
+// most 128 cells by five rows a thread): a row lies across LW lanes of 4 cells
+// and a thread holds its chunk column of RW rows, each value widened from its
+// 16-bit storage, and the scaled residual beside it.  A sweep takes the
+// y-neighbours from the thread's registers, except the rows above and below
+// its block, which pass through shared memory (double-buffered by parity: one
+// CTA barrier), and the x-neighbours from the adjacent lanes by shuffles; it
+// updates the whole grown tile (what lies beyond the shrinking valid region
+// never reaches a valid cell, and e is zero outside the update region).  The
+// division by 4 is exact on sums of 16-bit values, so one FMA adds the
+// residual with the one rounding of the other form.  Bound by latency.  GB300,
+// FP16, us a sweep, against the form in shared memory: 512^2 0.465 / 0.73, 256^2
+// 0.38 / 0.49, 573 x 952 0.57 / 0.96.
+// ---------------------------------------------------------------------------
+template <typename E, int LW, int RW>
+__global__ void __launch_bounds__(kIr2Threads, 1) k_ir2d_reg(Geom g, Ir2Plan p, Ir2Args a) {
+    extern __shared__ __align__(16) uint16_t ir2_smem[];
+    static_assert(RW >= 2, "a block's first and last row differ");
+    const int nx = g.nx, ny = g.ny, pw = p.pw, ph = p.ph, nt = blockDim.x, tid = threadIdx.x;
+    float *const W = reinterpret_cast<float *>(ir2_smem);  // prologue only: u on the grown tile
+    const int hrow = nt + 2 * LW;  // halo rows [parity][first / last], LW spare entries on either side
+    float4 *const halo = reinterpret_cast<float4 *>(ir2_smem) + LW;
+    const int tile = blockIdx.x, ntiles = p.tiles_x * p.tiles_y;
+    const int x0 = (tile % p.tiles_x) * p.tx, y0 = (tile / p.tiles_x) * p.ty;
+    const int ox = x0 - p.hx, oy = y0 - p.hy;
+    const int x1 = min(x0 + p.tx, nx), y1 = min(y0 + p.ty, ny);
+    const size_t quads_per_tile = (size_t)(p.tx / 4) * p.ty;
+    const int T = p.t;
+    const int lx = 4 * (tid % LW), x = ox + lx, ly = (tid / LW) * RW, yb = oy + ly;  // chunk and first row
+    const bool col = lx < pw && x >= 0 && x < nx;
+    unsigned sel[4], live = 0;  // cells and rows inside the update region
+    int pub[RW], ring[RW];      // quad indices in the exchange slot; -1: none
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sel[e] = col && in_range(x + e, nx, 1) ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const int y = yb + r;
+        pub[r] = ring[r] = -1;
+        if (in_range(y, ny, 1)) live |= 1u << r;
+        if (!col || y < 0 || y >= ny || ly + r >= ph) continue;
+        const int ocx = x / p.tx, ocy = y / p.ty;
+        const int quad = (int)((ocy * p.tiles_x + ocx) * quads_per_tile) + (y - ocy * p.ty) * (p.tx / 4) + (x - ocx * p.tx) / 4;
+        if (x >= x0 && x < x1 && y >= y0 && y < y1) pub[r] = quad;
+        else ring[r] = quad;
+    }
+    __shared__ float s_red[kIr2Threads / 32];
+    __shared__ float s_scale;
+
+    // ---- 1. prologue: u on the grown tile, r, the scale, rhs = e_1 -------
+    {
+        const int exa = max(ox, 0), exb = min(ox + pw, nx), eya = max(oy, 0), eyb = min(oy + ph, ny);
+        const int cw = (exb - exa) >> 2, n = cw * (eyb - eya);
+        for (int q = tid; q < n; q += nt) {
+            const int yy = eya + q / cw, xx = exa + 4 * (q % cw);
+            *reinterpret_cast<float4 *>(W + (yy - oy) * pw + (xx - ox)) =
+                __ldcg(reinterpret_cast<const float4 *>(a.u + (long long)yy * nx + xx));
+        }
+    }
+    __syncthreads();
+    // r on the owned tile grown by T - 1 cells, inside the update region
+    const int rxa = max(x0 - (T - 1), 1), rxb = min(x1 + T - 1, nx - 1);
+    const int rya = max(y0 - (T - 1), 1), ryb = min(y1 + T - 1, ny - 1);
+    float rr[RW][4], local = 0.0f;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const int y = yb + r;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            rr[r][e] = 0.0f;
+            if (!col || ly + r >= ph || y < rya || y >= ryb || x + e < rxa || x + e >= rxb) continue;
+            // k_ir_resid's arithmetic: a sum from +0 over axis i then axis j,
+            // the correctly rounded division, minus the centre
+            const float *c = W + (ly + r) * pw + lx + e;
+            float acc = 0.0f;
+            acc += c[-1];
+            acc += c[1];
+            acc += c[-pw];
+            acc += c[pw];
+            rr[r][e] = div_coeff<4>(acc) - c[0];
+            if (pub[r] >= 0) local = fmaxf(local, fabsf(rr[r][e]));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
+    if ((tid & 31) == 0) s_red[tid >> 5] = local;
+    __syncthreads();  // also: every read of W is done
+    bool ok = true;
+    if (tid == 0) {
+        float m = 0.0f;
+        for (int w = 0; w < nt / 32; ++w) m = fmaxf(m, s_red[w]);
+        // non-negative floats order as their bit patterns
+        atomicMax(a.max_bits + (a.step & 1), __float_as_uint(m));
+        grid_arrive(a.bar);
+        ok = grid_wait_bounded(a.bar, a.bar_target);
+        unsigned mb;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(mb) : "l"(a.max_bits + (a.step & 1)) : "memory");
+        const float mx = __uint_as_float(mb);
+        int ex = 0;
+        if (mx > 0.0f) frexpf(mx, &ex);  // mx = f * 2^ex, f in [0.5, 1)
+        s_scale = ldexpf(1.0f, ex);
+        if (blockIdx.x == 0) {
+            *a.scale = s_scale;
+            a.max_bits[(a.step + 1) & 1] = 0u;  // the next step's word (unused by this one)
+        }
+    }
+    for (int i = tid; i < 4 * hrow; i += nt) reinterpret_cast<float4 *>(ir2_smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!__syncthreads_and(ok)) return;
+    const float s = s_scale, inv = 1.0f / s;
+    float4 v[RW], rhs[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const float2 lo = Ir2Cvt<E>::two(Ir2Cvt<E>::pack(rr[r][0] * inv, rr[r][1] * inv));
+        const float2 hi = Ir2Cvt<E>::two(Ir2Cvt<E>::pack(rr[r][2] * inv, rr[r][3] * inv));
+        v[r] = rhs[r] = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+
+    // ---- 2./3. correction sweeps in blocks of T, exchanges between -----
+    const bool all_live = __all_sync(0xffffffffu, live == (1u << RW) - 1u);
+    int par = 0;
+    auto row = [&](const float4 &c, const float4 &up, const float4 &dn, const float4 &rh, bool on) -> float4 {
+        const float l = __shfl_up_sync(0xffffffffu, c.w, 1, LW), q = __shfl_down_sync(0xffffffffu, c.x, 1, LW);
+        float2 s0 = make_float2(l + c.y, c.x + c.z), s1 = make_float2(c.y + c.w, c.z + q);
+        s0 = fadd2(fadd2(s0, make_float2(up.x, up.y)), make_float2(dn.x, dn.y));
+        s1 = fadd2(fadd2(s1, make_float2(up.z, up.w)), make_float2(dn.z, dn.w));
+        const float2 k = make_float2(0.25f, 0.25f);
+        s0 = ffma2(s0, k, make_float2(rh.x, rh.y));
+        s1 = ffma2(s1, k, make_float2(rh.z, rh.w));
+        const float2 lo = Ir2Cvt<E>::two(Ir2Cvt<E>::pack(s0.x, s0.y)), hi = Ir2Cvt<E>::two(Ir2Cvt<E>::pack(s1.x, s1.y));
+        if (!on) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return make_float4(__uint_as_float(__float_as_uint(lo.x) & sel[0]), __uint_as_float(__float_as_uint(lo.y) & sel[1]),
+                           __uint_as_float(__float_as_uint(hi.x) & sel[2]), __uint_as_float(__float_as_uint(hi.y) & sel[3]));
+    };
+    int kk = min(T, a.m), k0 = 2;  // the first block's first sweep was e_1 = rhs
+    unsigned tag = a.tag0;
+    for (int done = 0; done < a.m;) {
+#pragma unroll 1
+        for (int k = k0; k <= kk; ++k, par ^= 1) {
+            float4 *first = halo + par * 2 * hrow, *last = first + hrow;
+            first[tid] = v[0];
+            last[tid] = v[RW - 1];
+            __syncthreads();
+            const float4 up = last[tid - LW], dn = first[tid + LW];
+            // inner rows first: the rows from shared memory arrive meanwhile
+            const float4 old1 = v[1], old2 = v[RW - 2];
+            float4 prev = v[0];
+#pragma unroll
+            for (int r = 1; r < RW - 1; ++r) {
+                const float4 c = v[r];
+                v[r] = row(c, prev, v[r + 1], rhs[r], all_live || ((live >> r) & 1u));
+                prev = c;
+            }
+            const float4 top = row(v[0], up, RW > 2 ? old1 : v[1], rhs[0], all_live || (live & 1u));
+            v[RW - 1] = row(v[RW - 1], RW > 2 ? old2 : v[0], dn, rhs[RW - 1], all_live || ((live >> (RW - 1)) & 1u));
+            v[0] = top;
+        }
+        done += kk;
+        k0 = 1;
+        if (done >= a.m) break;
+        ++tag;
+        unsigned long long *slot = a.xch + (size_t)(tag & 1) * ntiles * quads_per_tile * 2;
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+            if (pub[r] >= 0)
+                asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot + 2 * (size_t)pub[r]),
+                             "l"(ir2_word(Ir2Cvt<E>::pack(v[r].x, v[r].y), tag)),
+                             "l"(ir2_word(Ir2Cvt<E>::pack(v[r].z, v[r].w), tag))
+                             : "memory");
+        kk = min(T, a.m - done);
+        unsigned long long lo[RW], hi[RW];
+        unsigned want = 0;
+        uint64_t t0 = 0;
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+            if (ring[r] >= 0) want |= 1u << r;
+        while (want && ok) {
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+                if ((want >> r) & 1u)
+                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
+                                 : "=l"(lo[r]), "=l"(hi[r])
+                                 : "l"(slot + 2 * (size_t)ring[r])
+                                 : "memory");
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+                if (((want >> r) & 1u) && (unsigned)(lo[r] >> 32) == tag && (unsigned)(hi[r] >> 32) == tag) {
+                    want &= ~(1u << r);
+                    const float2 e01 = Ir2Cvt<E>::two((unsigned)lo[r]), e23 = Ir2Cvt<E>::two((unsigned)hi[r]);
+                    v[r] = make_float4(e01.x, e01.y, e23.x, e23.y);
+                }
+            if (want) {
+                const uint64_t t = globaltimer_ns();
+                if (!t0) t0 = t;
+                else if (t - t0 > kWaitLimitNs) {
+                    report_status(kStatusTimeout);
+                    ok = false;
+                }
+            }
+        }
+        if (!__syncthreads_and(ok)) return;
+    }
+
+    // ---- 4. epilogue: u += s * e_m on the owned tile ---------------------
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        if (pub[r] < 0 || !((live >> r) & 1u)) continue;
+        float *up = a.u + (long long)(yb + r) * nx + x;
+        const float4 w = __ldcg(reinterpret_cast<const float4 *>(up));
+        const float o4[4] = {fmaf(s, v[r].x, w.x), fmaf(s, v[r].y, w.y), fmaf(s, v[r].z, w.z), fmaf(s, v[r].w, w.w)};
+        if (sel[0] & sel[1] & sel[2] & sel[3]) {
+            __stcg(reinterpret_cast<float4 *>(up), make_float4(o4[0], o4[1], o4[2], o4[3]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (sel[e]) up[e] = o4[e];
+        }
+    }
+}
+
 using Ir2Fn = void (*)(Geom, Ir2Plan, Ir2Args);
 
 template <typename E, int R>
@@ -429,6 +651,37 @@ Ir2Fn ir2_fn(int r, int ni) {
         case 4: return ir2_fn_ni<E, 4>(ni);
         default: return nullptr;
     }
+}
+
+// The register form's kernel for lw lanes a row and rw rows a thread.
+template <typename E>
+Ir2Fn ir2_reg_fn(int lw, int rw) {
+    if (lw == 16) return rw == 2 ? k_ir2d_reg<E, 16, 2> : rw == 3 ? k_ir2d_reg<E, 16, 3> : rw == 4 ? k_ir2d_reg<E, 16, 4> : k_ir2d_reg<E, 16, 5>;
+    return rw == 2 ? k_ir2d_reg<E, 32, 2> : rw == 3 ? k_ir2d_reg<E, 32, 3> : rw == 4 ? k_ir2d_reg<E, 32, 4> : k_ir2d_reg<E, 32, 5>;
+}
+
+// The register form of a plan -- lanes a row (lw, 0: the grown tile does not
+// fit), rows a thread, threads, dynamic shared memory -- and its modelled SM
+// cycles per sweep: a + b * warps + (x + y * warps) / T for each number of rows
+// a thread, fitted to 4200 timed plans of 128 x 136 to 573 x 952 (3 to 5 % rms;
+// the model's choice is within 5 % of the best plan on each).
+struct Ir2Reg {
+    int lw, rw, threads, smem;
+    double cost;
+};
+Ir2Reg ir2_reg_plan(int r, const Ir2Plan &p) {
+    static const struct { int rw; double a, b, x, y; } model[] = {
+        {2, 392, 20, 1534, 27}, {3, 359, 31, 1628, 30}, {4, 400, 35, 1597, 45}, {5, 359, 43, 1853, 33}};
+    Ir2Reg best = {0, 0, 0, 0, 1e30};
+    if (r != 1 || p.pw > 128) return best;
+    const int lw = p.pw <= 64 ? 16 : 32;
+    for (const auto &m : model) {
+        const int nt = (lw * ((p.ph + m.rw - 1) / m.rw) + 31) / 32 * 32, warps = nt / 32;
+        const int smem = std::max(4 * (nt + 2 * lw) * 16, 4 * p.pw * p.ph);
+        const double c = m.a + m.b * warps + (m.x + m.y * warps) / p.t;
+        if (nt <= kIr2Threads && c < best.cost) best = {lw, m.rw, nt, smem, c};
+    }
+    return best;
 }
 
 int ir2_items(const Ir2Plan &p) {
@@ -484,13 +737,13 @@ bool ir2_choose(const Geom &g, int m, int temporal, int tile_x, int tile_y, int 
     double best = 1e30;
     for (int t = 1; t <= tmax; ++t) {
         if (temporal > 0 && t != std::min(temporal, tmax)) continue;
-        for (int tx : {16, 24, 32, 40, 48, 64, 96, 128, 256}) {
+        for (int tx : {16, 24, 32, 40, 48, 64, 80, 96, 128, 256}) {
             if (tile_x > 0 && tx != tile_x) continue;
-            for (int ty : {4, 8, 12, 16, 20, 24, 32, 48, 64, 128}) {
+            for (int ty : {4, 8, 12, 16, 20, 24, 32, 40, 48, 56, 64, 128}) {
                 if (tile_y > 0 && ty != tile_y) continue;
                 Ir2Plan q;
                 if (!ir2_make_plan(g, t, tx, ty, max_ctas, &q)) continue;
-                const double c = ir2_cost(g, q);
+                const double c = std::min(ir2_cost(g, q), ir2_reg_plan(g.radius, q).cost);
                 if (c < best - 1e-9) {
                     best = c;
                     *out = q;
@@ -526,6 +779,17 @@ int ir2_max_ctas(int r) {
         }
         n = std::min(n, k);
     }
+    for (int lw : {16, 32})
+        for (int rw = 2; r == 1 && rw <= 5; ++rw) {
+            const void *fn = reinterpret_cast<const void *>(ir2_reg_fn<E>(lw, rw));
+            int k = 0;
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kIr2SmemMax) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, kIr2Threads, kIr2SmemMax) != cudaSuccess) {
+                cudaGetLastError();
+                k = 0;
+            }
+            n = std::min(n, k);
+        }
     const int ctas = n >= 1 ? std::min(num_sms(), kIr2MaxTiles) : 0;
     cache.push_back({dev * 8 + r, ctas});
     return ctas;
@@ -568,9 +832,13 @@ int ir2_launch(const Geom &g, const Ir2Plan &p, float *u, unsigned long long *xc
     Geom gg = g;
     Ir2Plan pp = p;
     void *args[] = {&gg, &pp, &a};
-    const size_t smem = 6ull * p.pw * p.ph;
+    // in registers where the models say so
+    Ir2Reg reg = ir2_reg_plan(g.radius, p);
+    if (reg.cost >= ir2_cost(g, p)) reg.lw = 0;
+    if (reg.lw) fn = ir2_reg_fn<E>(reg.lw, reg.rw);
+    const size_t smem = reg.lw ? (size_t)reg.smem : 6ull * p.pw * p.ph;
     ST_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fn), dim3(grid),
-                                        dim3(kIr2Threads), args, smem, s));
+                                        dim3(reg.lw ? reg.threads : kIr2Threads), args, smem, s));
     return STENCIL_OK;
 }
 
