@@ -87,6 +87,14 @@ static_assert(B1S<1>::NS <= kB1MaxSlots && B1S<2>::NS <= kB1MaxSlots && B1S<1, t
 #define STENCIL_B1_ROWS_L1 1
 #endif
 
+// Rows in flight ahead of the one being computed in 2-D grids (one CTA of 16
+// warps an SM).  GB300, a batch of grids that fit the L2 together / of grids
+// that do not, GCell/s: R = 1 3 rows 760 / 568, 4 rows 780 / 598, 6 rows 738 /
+// 594; R = 2 2 rows 650 / 533, 4 rows 724 / 606; R = 4 1 row 610 / 497, 2 rows
+// 582 / 533.  (With the x-neighbours' chunks loaded too: 740 / 445, 675 / 428
+// and 590 / 412.)
+template <int R> constexpr int kB1RowsAhead = R <= 2 ? 4 : 1;
+
 constexpr int kB1MaxTiers = 12;
 constexpr int kB1MaxCtas = 1024;
 constexpr unsigned kB1Stop = 0xffffffffu;
@@ -301,14 +309,16 @@ __device__ __forceinline__ void job3d(const B1Args &A, const B1Job *__restrict__
     if (threadIdx.x == 0) c.scnt += (unsigned)(J->iters - 1) * P;
 }
 
-// All sweeps of a 2-D grid on the team.
+// All sweeps of a 2-D grid on the team.  A function of its own: what the
+// kernel keeps in registers is saved once a grid instead of spilled inside
+// the row loop.
 template <int R>
-__device__ __forceinline__ bool job2d(const B1Args &A, const B1Job *__restrict__ J, B1Ctl &c) {
+__device__ __noinline__ bool job2d(const B1Args &A, const B1Job *__restrict__ J, B1Ctl &c) {
     const int iters = J->iters;
     for (int sw = 0; sw < iters; ++sw) {
         const float *src = (sw & 1) ? J->b : J->a;
         float *dst = (sw & 1) ? J->a : J->b;
-        rows2d_sweep_d<R, kB1Threads, (R == 1 ? 4 : R == 2 ? 2 : 1), STENCIL_B1_ROWS_L1 != 0>(
+        rows2d_sweep<R, kB1Threads, kB1RowsAhead<R>, STENCIL_B1_ROWS_L1 != 0>(
             src, dst, J->g, J->hb, J->nblk, c.rel, c.size);
         if (sw + 1 < iters && !team_barrier(A, c)) return false;
     }

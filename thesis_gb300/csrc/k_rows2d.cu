@@ -6,11 +6,20 @@
 // A thread owns one float4 chunk column of a block of HB rows: it keeps the
 // column's rows j-R .. j+R in a register queue (one new 16-byte load per
 // row, the smem_register idea of src/stencils.cu:71-83 on registers) and
-// loads the chunks left and right of its own for the x-neighbours, so a
-// 4-cell update costs three 16-byte loads at any R <= 4 (the base kernel:
-// 3 + 2R).  Items (chunk column, row block) are spread over the resident CTAs
-// with a grid stride; consecutive threads take consecutive chunk columns, so
-// a warp's loads and stores are contiguous 512-byte segments.
+// takes the x-neighbours from the lanes beside it, so a 4-cell update costs
+// one 16-byte load at any R <= 4 (the base kernel: 3 + 2R) and one short load
+// in a warp's first and last lane.  Items (chunk column, row block) are spread
+// over the resident CTAs with a grid stride; consecutive threads take
+// consecutive chunk columns, so a warp's loads and stores are contiguous
+// 512-byte segments.
+//
+// Bounds: device memory above the L2's size (91 % of a plain copy's rate at
+// R = 1), L2 reads and the barrier below it.  What was in the way was bytes
+// in flight: with the left and right chunks loaded too, registers allowed one
+// row ahead (16 KB an SM), and hb blocks that left a nearly empty last wave.
+// GB300, microseconds a sweep before -> now: R = 1 1024^2 3.07 -> 3.00, 2048^2
+// 6.23 -> 5.4, 4096^2 26.1 -> 22.3, 8192^2 111.8 -> 86.6, 16384^2 401 -> 336;
+// 8192^2 R = 2 114.7 -> 88.8, R = 3 216 -> 146, R = 4 186 -> 109.
 //
 // Loads are plain (L1-cached): a buffer is rewritten every other sweep
 // inside the launch, and every read of another CTA's writes follows the grid
@@ -32,6 +41,12 @@ namespace {
 
 constexpr int kRowsThreads = 512;
 
+// Rows in flight ahead of the row being computed: as many as leave two CTAs
+// (R <= 2) or one CTA of 16 warps on an SM without spills in the loop.  GB300,
+// GCell/s for 1 / 2 / 3 / 4 rows, R = 1 8192^2: - / 739 / 775 / 731; R = 2:
+// 707 / 755; R = 3: 388 / 445 / 460; R = 4: 514 / 574 / 615.
+template <int R> constexpr int kRowsAhead = R == 2 ? 2 : 3;
+
 // ANY: rows that are not 16-byte aligned, one column per thread
 // (rows2d_sweep_any).
 template <int R, bool L1, bool ANY = false>
@@ -42,7 +57,7 @@ __global__ void __launch_bounds__(kRowsThreads, R <= 2 || ANY ? 2 : 1)
         const float *src = (sw & 1) ? b : a;
         float *dst = (sw & 1) ? a : b;
         if constexpr (ANY) rows2d_sweep_any<R, kRowsThreads>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
-        else rows2d_sweep<R, kRowsThreads, L1>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
+        else rows2d_sweep<R, kRowsThreads, kRowsAhead<R>, L1>(src, dst, g, hb, nblk, blockIdx.x, gridDim.x);
         if (sw + 1 < iters) {
             // every CTA's writes of this sweep before any CTA's next reads
             __syncthreads();
@@ -58,13 +73,10 @@ __global__ void __launch_bounds__(kRowsThreads, R <= 2 || ANY ? 2 : 1)
 
 using RowsFn = void (*)(float *, float *, Geom, int, int, int, unsigned *);
 
-// Loads: plain, L1-cached (the x-neighbour chunks are other threads' centre
-// chunks of the same row), legal because every read of another CTA's writes
-// follows the grid barrier's acquire and a CTA barrier; STENCIL_ROWS_L1=0
-// (read at each launch) selects ld.global.cg.  GB300, R = 1, bit-identical:
-// 1024^2 309.5 -> 327.0, 1500^2 438.7 -> 493.0, 2048^2 575.1 -> 640.4,
-// 4096^2 626.1 -> 634.4, 8192^2 592.8 -> 596.1 GCell/s; R = 4 2048^2
-// 426.0 -> 445.0.
+// Loads: plain, L1-cached (a warp's edge cells are its neighbour warp's
+// chunks), legal because every read of another CTA's writes follows the grid
+// barrier's acquire and a CTA barrier; STENCIL_ROWS_L1=0 (read at each
+// launch) selects ld.global.cg.
 RowsFn rows_fn(int r, bool l1 = false) {
     switch (r * 2 + (l1 ? 1 : 0)) {
         case 2: return k_rows2d<1, false>;
@@ -125,17 +137,23 @@ bool rows2d_any_supported(const Geom &g, int dims) {
 
 int rows2d_capacity(const Geom &g) { return rows_ctas(g.radius); }
 
-// Row blocks of a rows sweep of g on `threads` threads: as tall as keeps
-// about four items per thread (a taller block re-reads fewer halo rows), at
-// most 64 rows and at least 4 (R = 1) or 8 rows (measured on 1024^2 to
-// 32768^2 grids).
+// Row blocks of a rows sweep of g on `threads` threads: the height, at most
+// 64 rows and at least 4 (R = 1) or 8, that costs the busiest thread the
+// fewest rows, each of its items counted with its 2R halo rows and about
+// three rows' time for the first load.  (About four items per thread, as
+// before, left one more, nearly empty wave: 4.14 items per thread on 8192^2.
+// Limits of 128 rows and 1 or 6 rows for the first load measured within 1 %.)
 void rows2d_plan(const Geom &g, long long threads, int *hb, int *nblk) {
     const int nch = (int)(g.sy / 4), rows = g.ny - 2 * g.radius;
-    const long long hb_min = g.radius == 1 ? 4 : 8;
-    int h = (int)std::min<long long>(64, std::max<long long>(hb_min, (long long)nch * rows / (4 * std::max(1LL, threads))));
-    h = std::max(1, std::min(h, rows));
-    *hb = h;
-    *nblk = (rows + h - 1) / h;
+    const int lo = std::min(rows, g.radius == 1 ? 4 : 8), hi = std::min(rows, 64);
+    threads = std::max(1LL, threads);
+    double best = 1e300;
+    for (int h = hi; h >= lo; --h) {
+        const int n = (rows + h - 1) / h;
+        const long long waves = ((long long)nch * n + threads - 1) / threads;
+        const double cost = (double)waves * (h + 3 + 2 * g.radius);
+        if (cost < best) { best = cost; *hb = h; *nblk = n; }
+    }
 }
 
 // The persistent rows kernel on rows that are not 16-byte aligned.  Row blocks
