@@ -234,10 +234,11 @@ STENCIL_API int stencil_batch_launch(const void *d_workspace, stencil_stream_t s
  * sweeps (3-D grids with the stream kernel's TMA-ring code, 2-D grids with
  * the rows kernel's register-queue code, a bounded barrier over the team
  * between sweeps) and then takes the next grid from a device queue; grids
- * are placed in tiers by the team size their cells keep busy (about
- * STENCIL_BATCH1_CELLS_PER_CTA_2D = 50000 / _3D = 50000 update cells per
- * CTA, at most STENCIL_BATCH1_MAX_TEAM = a quarter of the CTAs; environment
- * variables of these names override them at prepare time), every team
+ * are placed in tiers by team sizes chosen at prepare time to end the batch
+ * earliest under a model of the sweep times (where the environment sets
+ * STENCIL_BATCH1_CELLS_PER_CTA_2D or _3D, update cells per CTA, or
+ * STENCIL_BATCH1_MAX_TEAM: by the cells alone, the others being 50000, 50000
+ * and a quarter of the CTAs), every team
  * starts in the largest tier and splits into the next tier's teams when its
  * queue is empty; ragged grids are copied in and out by their team inside the
  * launch.  It uses the jobs' team fields, not temporal / tile_x / tile_y.  AUTO:

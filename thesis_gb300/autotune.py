@@ -331,7 +331,7 @@ def tune_batch(make_jobs, classes=None, repeats=2, log=print):
 # ---- batches, one-launch engine: CTAs per grid ----------------------------
 #
 # The one-launch engine gives each grid a team of CTAs (the device's CTA
-# count halved repeatedly); its default is the grid's update cells / 50000.
+# count halved repeatedly), by default from a model of the whole batch.
 # The tuner picks, per class of grid, the cells per CTA that set each grid's
 # team field (cells of the whole grid, border included).
 BATCH1_SPACE = {cls: {"cells_per_cta": [12500, 25000, 50000, 100000, 200000]}
@@ -365,7 +365,7 @@ def tune_batch_teams(make_jobs, classes=None, repeats=1, time_batch=None, log=pr
     e.g. its grids with a tenth of their sweeps: the classes share the GPU
     in one launch, so each is tuned beside the others).  The cells per CTA
     of each class present (BATCH1_SPACE) are chosen by coordinate descent
-    from the library's default, each candidate setting every grid's team
+    from 50000, each candidate setting every grid's team
     field and scored by the CUDA-event time of one launch (min over
     repeats) and kept only when it gains 1 %; a candidate whose results
     differ in any bit from the default's is rejected.  time_batch(jobs_with_hints) -> (seconds,

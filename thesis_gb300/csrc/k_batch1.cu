@@ -13,10 +13,10 @@
 // the reference's summation order and division, so results are bit-identical
 // to the ping-pong loop.
 //
-// Teams and tiers.  The host puts each grid in a tier by the team size its
-// cells keep busy (about STENCIL_BATCH1_CELLS_PER_CTA_{2D,3D} update cells
-// per CTA per sweep, so the per-sweep barrier stays a small share), or by the
-// job's own team field (an autotuner's choice); tier t has
+// Teams and tiers.  The host puts each grid in a tier by its team size: the
+// one that ends the whole batch earliest under a model of the sweep times
+// (plan_tiers below), or the job's own team field (an autotuner's choice);
+// tier t has
 // a nominal team size and a queue of its grids, largest work first.  All
 // CTAs start in the first tier as teams of its size; a team whose tier queue
 // is empty splits into the next tier's teams (its own CTAs: never waiting on
@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <mutex>
 #include <vector>
 
@@ -445,8 +446,9 @@ long long env_ll(const char *name, long long dflt) {
 
 }  // namespace
 
-// Update cells per CTA per sweep that a team keeps, and the largest team
-// (environment variables of the same names override them at prepare time).
+// The rule by cells, used when an environment variable of one of these names
+// is set at prepare time and as the plan that plan_tiers has to beat: the
+// update cells per CTA per sweep that a team keeps, and the largest team.
 // GB300, the 512-grid benchmark batch, seconds per batch for 2-D / 3-D
 // cells per CTA: 25k/50k 2.79, 50k/50k 2.76, 50k/100k 2.90, 100k/100k 3.06,
 // 100k/200k 3.36 (before the L1-cached 2-D loads; with them 50k/50k 2.63).
@@ -456,6 +458,175 @@ long long env_ll(const char *name, long long dflt) {
 #ifndef STENCIL_BATCH1_CELLS_PER_CTA_3D
 #define STENCIL_BATCH1_CELLS_PER_CTA_3D 50000
 #endif
+
+namespace {
+
+// The tile and plane counts a 3-D job's stream code is planned with.
+void b1_tile(const Geom &g, bool narrow, int *tx, int *ty) {
+    switch (g.radius * 2 + narrow) {
+        case 2: *tx = B1S<1>::TX; *ty = B1S<1>::TY; break;
+        case 3: *tx = B1S<1, true>::TX; *ty = B1S<1, true>::TY; break;
+        case 4: *tx = B1S<2>::TX; *ty = B1S<2>::TY; break;
+        case 5: *tx = B1S<2, true>::TX; *ty = B1S<2, true>::TY; break;
+        case 6: *tx = B1S<3>::TX; *ty = B1S<3>::TY; break;
+        default: *tx = B1S<4>::TX; *ty = B1S<4>::TY; break;
+    }
+}
+
+// One sweep of a grid on a team of k CTAs, in microseconds: the rows or
+// planes of the busiest thread or CTA at one row's or plane's time, and the
+// barrier with the first loads.  (GB300, one grid at a time, 21 3-D and 24 2-D
+// shapes on every team size: 3-D within 11 %, 2-D within 27 %, a standard
+// deviation of 2 to 5 % and 3 to 10 %.)
+double b1_sweep_us(const Geom &g, int dims, bool narrow, int k) {
+    const int R = g.radius;
+    if (dims == 2) {
+        static const double row[5] = {0, 0.281, 0.304, 0.559, 0.378}, first[5] = {0, 2.28, 2.62, 3.31, 2.51};
+        // rows2d_plan's choice without its search: one block per thread
+        // where blocks of at most 64 rows do, else an even share
+        const double chunks = (double)(g.sy / 4), blocks = std::floor((double)k * kB1Threads / chunks);
+        const double rows = g.ny - 2 * R;
+        const double busy = 64 * blocks >= rows ? std::max(R == 1 ? 4.0 : 8.0, std::ceil(rows / blocks))
+                                                : 1.03 * rows * chunks / (k * kB1Threads);
+        return busy * row[R] + first[R];
+    }
+    static const double plane[5] = {0, 0.359, 0.621, 0.419, 0.459}, plane_narrow[3] = {0, 0.373, 0.413};
+    int tx, ty, tiles_x, tiles_y, zchunk, items;
+    b1_tile(g, narrow, &tx, &ty);
+    stream3d_plan(g, tx, ty, k, &tiles_x, &tiles_y, &zchunk, &items);
+    return (double)((items + k - 1) / k) * (zchunk * (narrow ? plane_narrow : plane)[R] + 0.5) + 3.0;
+}
+
+struct B1Cost {
+    std::vector<double> us;  // on each team size of the ladder
+    double mb;               // both buffers
+    bool rows;               // 2-D
+};
+
+// When the last grid ends, by the kernel's own schedule: each team takes its
+// tier's next grid (`order`: largest work first) when it is free, and splits
+// for the next tier once that queue is empty.  While the grids being swept do
+// not fit the L2 together, the 2-D ones take up to 1.65 times as long (1.5 to
+// 1.7 measured; the 3-D ones 1.03 to 1.1, left out): many large grids on small
+// teams lose to few on large ones.  *last is the grid that ends last.
+double b1_schedule(const std::vector<int> &ladder, const std::vector<B1Cost> &cost, const std::vector<int> &order,
+                   const std::vector<int> &tier_of, int *last) {
+    constexpr double kOutside = 1.65, kFits = 70, kSpills = 125;  // MB of the L2's 129
+    struct Run {
+        double until;  // 3-D: the end; 2-D: the end on a clock that stands back by the factor
+        int tier, ctas, job;
+        bool operator<(const Run &o) const { return until > o.until; }
+    };
+    const int L = (int)ladder.size();
+    std::vector<std::vector<int>> queue(L);
+    for (int i : order) queue[tier_of[i]].push_back(i);
+    std::vector<int> tiers;  // those with grids
+    for (int t = 0; t < L; ++t)
+        if (!queue[t].empty()) tiers.push_back(t);
+    if (tiers.empty()) return 0;
+    std::vector<size_t> head(L, 0);
+    std::vector<Run> busy[2];  // [2-D]: heaps
+    double now[2] = {0, 0}, mb = 0;
+    std::vector<std::pair<int, int>> free{{-1, ladder[0]}};  // (tier's place, CTAs)
+    for (;;) {
+        while (!free.empty()) {
+            const std::pair<int, int> m = free.back();
+            free.pop_back();
+            const int t = m.first < 0 ? -1 : tiers[m.first];
+            if (t >= 0 && head[t] < queue[t].size()) {
+                const int i = queue[t][head[t]++], k = cost[i].rows;
+                busy[k].push_back({now[k] + cost[i].us[t], m.first, m.second, i});
+                std::push_heap(busy[k].begin(), busy[k].end());
+                mb += cost[i].mb;
+            } else if (m.first + 1 < (int)tiers.size()) {
+                const int team = ladder[tiers[m.first + 1]], parts = std::max(1, m.second / team);
+                for (int q = 0; q < parts; ++q)
+                    free.push_back({m.first + 1, q + 1 < parts ? team : m.second - q * team});
+            }
+        }
+        if (busy[0].empty() && busy[1].empty()) return now[0];
+        const double slow = 1 + (kOutside - 1) * std::min(1.0, std::max(0.0, (mb - kFits) / (kSpills - kFits)));
+        const double d0 = busy[0].empty() ? 1e300 : busy[0][0].until - now[0];
+        const double d1 = busy[1].empty() ? 1e300 : (busy[1][0].until - now[1]) * slow;
+        const int k = d1 < d0;
+        now[0] += k ? d1 : d0;
+        now[1] += (k ? d1 : d0) / slow;
+        std::pop_heap(busy[k].begin(), busy[k].end());
+        const Run r = busy[k].back();
+        busy[k].pop_back();
+        mb -= cost[r.job].mb;
+        *last = r.job;
+        free.push_back({r.tier, r.ctas});
+    }
+}
+
+// Team sizes that end the batch earliest.  tier_of holds the rule's choice on
+// entry; grids with fixed[i] keep theirs.  For a range of end times the
+// smallest teams that keep every grid within that time (small teams lose
+// least to barriers) are put through the schedule; from the best of them, the
+// grid that ends last is moved a tier up or down while that helps.  The rule
+// alone ends a batch of few grids on one slow team, since it knows neither
+// the sweeps of a grid nor how many grids share the GPU.  GB300, milliseconds
+// a launch by the rule -> by this, the model's figures in brackets: 36 2-D
+// (64 to 2048 a side, R = 1) and 12 3-D grids (32 to 256, R = 2), 100 to 500
+// sweeps 19.7 -> 14.8 (20.4 -> 13.9); 23 and 7 grids 7.95 -> 2.58; 14 and 4
+// 4.55 -> 2.52; 26 and 2 3.45 -> 1.38; 40 and 11 9.10 -> 9.22; 11 and 15 13.2
+// -> 12.1; 384 and 128 with 20 sweeps 11.46 -> 10.95; the 512-grid benchmark
+// batch keeps the rule's plan (2592 ms, 2603 by the model).  The search takes
+// 0.15 ms of host time at 48 grids, 0.8 ms at 512; from 4096 grids on, which
+// leave little to gain at the end, there is none.
+void plan_tiers(const std::vector<int> &ladder, const std::vector<B1Cost> &cost, const std::vector<int> &order,
+                const std::vector<char> &fixed, std::vector<int> *tier_of) {
+    const int L = (int)ladder.size(), n = (int)order.size();
+    int targets = std::min(96, (1 << 13) / std::max(1, n)), moves = targets, last = -1;
+    if (targets < 2) return;
+    const double step = 1.02 + 0.04 * std::min(1.0, n / 512.0);
+    std::vector<int> best = *tier_of, cand(n);
+    const double rule = b1_schedule(ladder, cost, order, best, &last);
+    double end = rule, longest = 0, area = 0;
+    for (int i = 0; i < n; ++i) {
+        double lo = 1e300, a = 1e300;
+        for (int t = 0; t < L; ++t) {
+            lo = std::min(lo, cost[i].us[t]);
+            a = std::min(a, cost[i].us[t] * ladder[t]);
+        }
+        longest = std::max(longest, lo);
+        area += a / ladder[0];
+    }
+    for (double target = std::max(longest, area); target < 1.3 * end && targets-- > 0; target *= step) {
+        for (int i = 0; i < n; ++i) {
+            const double *u = cost[i].us.data();
+            const double within = std::max(target, 1.03 * *std::min_element(u, u + L));
+            int t = L - 1;
+            while (t > 0 && u[t] > within) --t;
+            cand[i] = fixed[i] ? (*tier_of)[i] : t;
+        }
+        const double e = b1_schedule(ladder, cost, order, cand, &last);
+        if (e < end) { end = e; best = cand; }
+    }
+    b1_schedule(ladder, cost, order, best, &last);
+    for (bool moved = true; moved && last >= 0 && !fixed[last];) {
+        moved = false;
+        const int at = last;
+        for (int d : {-1, 1, -2}) {
+            if (best[at] + d < 0 || best[at] + d >= L || --moves < 0) continue;
+            cand = best;
+            cand[at] += d;
+            int who = at;
+            const double e = b1_schedule(ladder, cost, order, cand, &who);
+            if (e < 0.999 * end) {
+                end = e;
+                best = cand;
+                last = who;
+                moved = true;
+                break;
+            }
+        }
+    }
+    if (end < 0.97 * rule) *tier_of = best;  // less is within the model's error
+}
+
+}  // namespace
 
 size_t batch1_bytes_for(const stencil_batch_job *jobs, int njobs) {
     int n3 = 0;
@@ -490,17 +661,22 @@ int batch1_prepare(const stencil_batch_job *jobs, int njobs, void *d_workspace,
     const size_t ctr_off = maps_off + round256((size_t)n3 * 2 * sizeof(CUtensorMap));
     size_t copy_off = ctr_off + round256(b1_ctr_bytes(kB1MaxCtas));
 
-    // Team sizes: G, G/2, G/4, ... 1; a grid's tier is the largest of them
-    // at most its cells / cells-per-CTA (and at most the largest team).
+    // Team sizes: G, G/2, G/4, ... 1.
     std::vector<int> ladder;
     for (int k = grid; k >= 1; k /= 2) ladder.push_back(k);
-    const long long cpc2 = env_ll("STENCIL_BATCH1_CELLS_PER_CTA_2D", STENCIL_BATCH1_CELLS_PER_CTA_2D);
-    const long long cpc3 = env_ll("STENCIL_BATCH1_CELLS_PER_CTA_3D", STENCIL_BATCH1_CELLS_PER_CTA_3D);
-    const long long kmax = env_ll("STENCIL_BATCH1_MAX_TEAM", std::max(1, grid / 4));
+    const long long cpc2 = env_ll("STENCIL_BATCH1_CELLS_PER_CTA_2D", 0);
+    const long long cpc3 = env_ll("STENCIL_BATCH1_CELLS_PER_CTA_3D", 0);
+    const long long cap = env_ll("STENCIL_BATCH1_MAX_TEAM", 0);
+    const bool by_rule = cpc2 || cpc3 || cap;
+    const long long rule2 = cpc2 ? cpc2 : STENCIL_BATCH1_CELLS_PER_CTA_2D;
+    const long long rule3 = cpc3 ? cpc3 : STENCIL_BATCH1_CELLS_PER_CTA_3D;
+    const long long kmax = cap ? cap : std::max(1, grid / 4);
 
     std::vector<B1Job> table(njobs);
     std::vector<int> tier_of(njobs);
     std::vector<double> work(njobs);
+    std::vector<B1Cost> cost(by_rule ? 0 : njobs);
+    std::vector<char> fixed(njobs);
     std::vector<CUtensorMap> maps;
     maps.reserve(2 * n3);
     for (int i = 0; i < njobs; ++i) {
@@ -531,27 +707,19 @@ int batch1_prepare(const stencil_batch_job *jobs, int njobs, void *d_workspace,
         J.g = g;
         const long long cells = (long long)(p.nx - 2 * p.radius) * (p.ny - 2 * p.radius) *
                                 (p.dims == 3 ? p.nz - 2 * p.radius : 1);
-        // the job's own team size (a tuner's choice), else from its cells
-        const long long want =
-            b.team > 0 ? std::min<long long>(b.team, grid)
-                       : std::max(1LL, std::min(kmax, cells / (p.dims == 3 ? cpc3 : cpc2)));
+        // the job's own team size (a tuner's choice), else from its cells:
+        // the largest of the ladder at most that
+        fixed[i] = b.team > 0;
+        const long long want = fixed[i] ? std::min<long long>(b.team, grid)
+                                        : std::max(1LL, std::min(kmax, cells / (p.dims == 3 ? rule3 : rule2)));
         int t = 0;
         while (ladder[t] > want) ++t;
         tier_of[i] = t;
         work[i] = (double)cells * b.iterations;
-        const int team = ladder[t];
+        J.narrow = p.dims == 3 && p.radius <= 2 && p.nx <= 64;
         if (p.dims == 3) {
             int tx = 0, ty = 0;
-            J.narrow = p.radius <= 2 && p.nx <= 64;
-            switch (p.radius * 2 + J.narrow) {
-                case 2: tx = B1S<1>::TX; ty = B1S<1>::TY; break;
-                case 3: tx = B1S<1, true>::TX; ty = B1S<1, true>::TY; break;
-                case 4: tx = B1S<2>::TX; ty = B1S<2>::TY; break;
-                case 5: tx = B1S<2, true>::TX; ty = B1S<2, true>::TY; break;
-                case 6: tx = B1S<3>::TX; ty = B1S<3>::TY; break;
-                default: tx = B1S<4>::TX; ty = B1S<4>::TY; break;
-            }
-            stream3d_plan(g, tx, ty, team, &J.tiles_x, &J.tiles_y, &J.zchunk, &J.items);
+            b1_tile(g, J.narrow, &tx, &ty);
             CUtensorMap m[2];
             const long long dims[3] = {g.nx, g.ny, g.nz};
             const int box[3] = {tx + 2 * ((p.radius + 3) & ~3), ty + 2 * p.radius, 1};
@@ -561,18 +729,32 @@ int batch1_prepare(const stencil_batch_job *jobs, int njobs, void *d_workspace,
             J.map_pair = (int)(maps.size() / 2);
             maps.push_back(m[0]);
             maps.push_back(m[1]);
-        } else {
-            if ((long long)(g.sy / 4) * (g.ny - 2 * g.radius) >= (1LL << 31))
-                return fail(STENCIL_EUNSUPPORTED, "job %d: 2-D grid of 2^31 or more chunk-rows", i);
-            rows2d_plan(g, (long long)team * kB1Threads, &J.hb, &J.nblk);
+        } else if ((long long)(g.sy / 4) * (g.ny - 2 * g.radius) >= (1LL << 31)) {
+            return fail(STENCIL_EUNSUPPORTED, "job %d: 2-D grid of 2^31 or more chunk-rows", i);
+        }
+        if (!by_rule) {
+            cost[i].mb = 8e-6 * (double)J.rows * g.sy;
+            cost[i].rows = p.dims == 2;
+            for (int k : ladder) cost[i].us.push_back(b.iterations * b1_sweep_us(g, p.dims, J.narrow, k));
         }
     }
-    // job table: by tier, then largest work first
+    // largest work first, then by tier: the job table's order
     std::vector<int> order(njobs);
     for (int i = 0; i < njobs; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        return tier_of[x] != tier_of[y] ? tier_of[x] < tier_of[y] : work[x] > work[y];
-    });
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work[x] > work[y]; });
+    if (!by_rule) plan_tiers(ladder, cost, order, fixed, &tier_of);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tier_of[x] < tier_of[y]; });
+    for (int i = 0; i < njobs; ++i) {
+        B1Job &J = table[i];
+        const int team = ladder[tier_of[i]];
+        if (J.dims == 3) {
+            int tx = 0, ty = 0;
+            b1_tile(J.g, J.narrow, &tx, &ty);
+            stream3d_plan(J.g, tx, ty, team, &J.tiles_x, &J.tiles_y, &J.zchunk, &J.items);
+        } else {
+            rows2d_plan(J.g, (long long)team * kB1Threads, &J.hb, &J.nblk);
+        }
+    }
     std::vector<B1Job> sorted(njobs);
     B1Plan plan;
     B1Args &A = plan.args;

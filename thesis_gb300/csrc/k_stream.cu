@@ -215,8 +215,9 @@ void stream3d_plan(const Geom &g, int tx, int ty, int resident, int *tiles_x, in
     resident = std::max(1, resident);
     int nchunks = 1;
     double best = 1e30;
-    for (int n = 1; n <= std::max(1, zin / 2); ++n) {
-        const int zc = (zin + n - 1) / n;
+    // one n for each chunk height: the smallest
+    for (int n = 1, zc; n <= std::max(1, zin / 2); n = zc > 1 ? (zin + zc - 2) / (zc - 1) : zin + 1) {
+        zc = (zin + n - 1) / n;
         const long long it = (long long)tiles * ((zin + zc - 1) / zc);
         const double waves = std::ceil((double)it / resident);
         const double fill = (double)it / (waves * resident);  // <= 1
