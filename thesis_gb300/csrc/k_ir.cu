@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "host.hpp"
+#include "stream_read.cuh"
 
 namespace st {
 
@@ -164,36 +165,76 @@ __device__ __forceinline__ float4 ir_ld4(const float *p) { return *reinterpret_c
 // r = (M u + c) - u over the update region (FP32, the sweep's summation
 // order).  pass 0: max |r| into *max_bits.  pass 1: stores r * 2^-ceil(log2
 // max) in E and the scale in *scale.
-template <typename E, int D, int R>
-__global__ void __launch_bounds__(256)
-    k_ir_resid(const float *__restrict__ u, E *__restrict__ r, Geom g, unsigned *max_bits,
-               float *scale, int pass) {
-    constexpr int C = 2 * D * R;
-    constexpr int RA = (R + 3) & ~3;
-    float inv = 1.0f;
-    if (pass == 1) {
-        const float m = __uint_as_float(*max_bits);
+template <typename E, int R>
+struct IrResidual {
+    struct Args {
+        E *r;
+        unsigned *max_bits;
+        float *scale;
+        int pass;
+    };
+    static constexpr bool kDiff = false;
+    Args a;
+    const Geom &g;
+    float inv, local;
+
+    __device__ IrResidual(const Args &a_, const Geom &g_) : a(a_), g(g_), inv(1.0f), local(0.0f) {
+        if (a.pass != 1) return;
+        const float m = __uint_as_float(*a.max_bits);
         int ex = 0;
         if (m > 0.0f) frexpf(m, &ex);  // m = f * 2^ex, f in [0.5, 1)
         const float s = ldexpf(1.0f, ex);
         inv = 1.0f / s;
-        if (blockIdx.x == 0 && threadIdx.x == 0) *scale = s;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.scale = s;
     }
-    const IrRows rows(g, D, R);
-    const int wpb = blockDim.x >> 5, lane = threadIdx.x & 31;
-    float local = 0.0f;
-    for (int q = blockIdx.x * wpb + (threadIdx.x >> 5); q < rows.nrows; q += gridDim.x * wpb) {
-        const long long base = rows.base(g, q);
-        const float *row = u + base;
-        for (int c = lane; c < rows.nch; c += 32) {
+    // new values of cells x .. x + 3 and the old ones
+    __device__ __forceinline__ void row(int x, int y, int z, const float2 (&v)[2], float4 c) {
+        const float res[4] = {v[0].x - c.x, v[0].y - c.y, v[1].x - c.z, v[1].y - c.w};
+        const bool full = x >= R && x + 3 < g.nx - R;
+        E *at = a.r + (long long)z * g.sz + (long long)y * g.sy + x;
+        if (a.pass == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (full || in_range(x + e, g.nx, R)) local = fmaxf(local, fabsf(res[e]));
+        } else if (full) {
+            uint2 q2;
+            q2.x = LowP<E>::from2(res[0] * inv, res[1] * inv);
+            q2.y = LowP<E>::from2(res[2] * inv, res[3] * inv);
+            *reinterpret_cast<uint2 *>(at) = q2;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (in_range(x + e, g.nx, R)) at[e] = LowP<E>::from(res[e] * inv);
+        }
+    }
+    __device__ void finish() {
+        if (a.pass != 0) return;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(a.max_bits, __float_as_uint(local));
+    }
+};
+
+// 2-D.  3-D grids take one pass of the streaming sweep's code instead
+// (stream_read.cuh): the same loads with a warp per row read a cell from the
+// L2 2R + 1 times over (GB300, 768^3 R = 4: 1440 us a pass; now 780, the sums
+// as in the sweep).
+template <typename E, int R>
+__global__ void __launch_bounds__(256)
+    k_ir_resid_2d(const float *__restrict__ u, typename IrResidual<E, R>::Args args, Geom g) {
+    IrResidual<E, R> out(args, g);
+    const int wpb = blockDim.x >> 5, lane = threadIdx.x & 31, nch = g.nx >> 2;
+    for (int y = R + blockIdx.x * wpb + (threadIdx.x >> 5); y < g.ny - R; y += gridDim.x * wpb) {
+        const float *row = u + (long long)y * g.sy;
+        for (int c = lane; c < nch; c += 32) {
             const int x0 = 4 * c;
             if (x0 + 3 < R || x0 >= g.nx - R) continue;
-            float w[4 + 2 * RA];
+            float w[12];
 #pragma unroll
-            for (int h = 0; h < (4 + 2 * RA) / 4; ++h) {
-                const int cc = c - RA / 4 + h;
+            for (int h = 0; h < 3; ++h) {
+                const int cc = c - 1 + h;
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (cc >= 0 && cc < rows.nch) v = ir_ld4(row + 4 * cc);
+                if (cc >= 0 && cc < nch) v = ir_ld4(row + 4 * cc);
                 w[4 * h] = v.x; w[4 * h + 1] = v.y; w[4 * h + 2] = v.z; w[4 * h + 3] = v.w;
             }
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -201,7 +242,7 @@ __global__ void __launch_bounds__(256)
             for (int o = -R; o <= R; ++o) {
                 if (!o) continue;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[e] += w[RA + e + o];
+                for (int e = 0; e < 4; ++e) acc[e] += w[4 + e + o];
             }
 #pragma unroll
             for (int o = -R; o <= R; ++o) {
@@ -209,65 +250,56 @@ __global__ void __launch_bounds__(256)
                 const float4 v = ir_ld4(row + x0 + o * g.sy);
                 acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
             }
-            if (D == 3) {
-#pragma unroll
-                for (int o = -R; o <= R; ++o) {
-                    if (!o) continue;
-                    const float4 v = ir_ld4(row + x0 + o * g.sz);
-                    acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-                }
-            }
-            float res[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) res[e] = div_coeff<C>(acc[e]) - w[RA + e];
-            const bool full = x0 >= R && x0 + 3 < g.nx - R;
-            if (pass == 0) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (full || in_range(x0 + e, g.nx, R)) local = fmaxf(local, fabsf(res[e]));
-            } else if (full) {
-                uint2 q2;
-                q2.x = LowP<E>::from2(res[0] * inv, res[1] * inv);
-                q2.y = LowP<E>::from2(res[2] * inv, res[3] * inv);
-                *reinterpret_cast<uint2 *>(r + base + x0) = q2;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (in_range(x0 + e, g.nx, R)) r[base + x0 + e] = LowP<E>::from(res[e] * inv);
-            }
+            const float2 v[2] = {make_float2(div_coeff<4 * R>(acc[0]), div_coeff<4 * R>(acc[1])),
+                                 make_float2(div_coeff<4 * R>(acc[2]), div_coeff<4 * R>(acc[3]))};
+            out.row(x0, y, 0, v, make_float4(w[4], w[5], w[6], w[7]));
         }
     }
-    if (pass == 0) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
-        if ((threadIdx.x & 31) == 0) atomicMax(max_bits, __float_as_uint(local));
-    }
+    out.finish();
 }
 
-// u += s * e over the update region.
+// u += s * e over the update region.  A lane owns 8 cells; the loads of
+// three of them (96 bytes) are issued before the first is stored, since a
+// store to u holds back the loads after it (GB300, 768^3: 1480 -> 724 us for
+// 4.5 GB).
 template <typename E, int D, int R>
 __global__ void __launch_bounds__(256)
     k_ir_update(float *__restrict__ u, const E *__restrict__ e, Geom g, const float *scale) {
+    constexpr int N = 3;
     const float s = *scale;
     const IrRows rows(g, D, R);
-    const int wpb = blockDim.x >> 5, lane = threadIdx.x & 31;
+    const int wpb = blockDim.x >> 5, lane = threadIdx.x & 31, nv = g.nx >> 3;
     for (int q = blockIdx.x * wpb + (threadIdx.x >> 5); q < rows.nrows; q += gridDim.x * wpb) {
         const long long base = rows.base(g, q);
-        for (int c = lane; c < rows.nch; c += 32) {
-            const int x0 = 4 * c;
-            if (x0 + 3 < R || x0 >= g.nx - R) continue;
-            float *up = u + base + x0;
-            const float4 v = ir_ld4(up);
-            const uint2 ew = *reinterpret_cast<const uint2 *>(e + base + x0);
-            const float2 e01 = LowP<E>::to2(ew.x), e23 = LowP<E>::to2(ew.y);
-            const float out[4] = {fmaf(s, e01.x, v.x), fmaf(s, e01.y, v.y), fmaf(s, e23.x, v.z),
-                                  fmaf(s, e23.y, v.w)};
-            if (x0 >= R && x0 + 3 < g.nx - R) {
-                *reinterpret_cast<float4 *>(up) = make_float4(out[0], out[1], out[2], out[3]);
-            } else {
+        for (int v0 = lane; v0 < nv; v0 += 32 * N) {
+            float4 a[N][2];
+            uint4 ew[N];
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (in_range(x0 + k, g.nx, R)) up[k] = out[k];
+            for (int n = 0; n < N; ++n) {
+                if (v0 + 32 * n >= nv) continue;
+                const long long at = base + 8 * (v0 + 32 * n);
+                a[n][0] = ir_ld4(u + at);
+                a[n][1] = ir_ld4(u + at + 4);
+                ew[n] = *reinterpret_cast<const uint4 *>(e + at);
+            }
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const int x0 = 8 * (v0 + 32 * n);
+                if (x0 >= g.nx) continue;
+                float f[8];
+                unpack8<E>(ew[n], f);
+                const float4 p = a[n][0], r = a[n][1];
+                const float out[8] = {fmaf(s, f[0], p.x), fmaf(s, f[1], p.y), fmaf(s, f[2], p.z), fmaf(s, f[3], p.w),
+                                      fmaf(s, f[4], r.x), fmaf(s, f[5], r.y), fmaf(s, f[6], r.z), fmaf(s, f[7], r.w)};
+                float *up = u + base + x0;
+                if (x0 >= R && x0 + 7 < g.nx - R) {
+                    *reinterpret_cast<float4 *>(up) = make_float4(out[0], out[1], out[2], out[3]);
+                    *reinterpret_cast<float4 *>(up + 4) = make_float4(out[4], out[5], out[6], out[7]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (in_range(x0 + k, g.nx, R)) up[k] = out[k];
+                }
             }
         }
     }
@@ -310,7 +342,6 @@ template <typename E, int D, int R>
 int ir_loop(const stencil_params &p, const stencil_ir_params &ir, float *u, char *ws,
             cudaStream_t s, stencil_ir_result *out) {
     const Geom g = make_geom(p);
-    const size_t n = (size_t)cell_count(p);
     const IrLayout L = ir_layout(p, ir.storage);
     E *r = reinterpret_cast<E *>(ws);
     E *ea = reinterpret_cast<E *>(ws + L.lp);
@@ -361,11 +392,15 @@ int ir_loop(const stencil_params &p, const stencil_ir_params &ir, float *u, char
             ++launches;
         } else {
             ST_CUDA(cudaMemsetAsync(max_bits, 0, sizeof(unsigned), s));
-            k_ir_resid<E, D, R><<<blocks, 256, 0, s>>>(u, r, g, max_bits, scale, 0);
-            k_ir_resid<E, D, R><<<blocks, 256, 0, s>>>(u, r, g, max_bits, scale, 1);
+            for (int pass = 0; pass < 2; ++pass) {
+                const typename IrResidual<E, R>::Args args = {r, max_bits, scale, pass};
+                int rc = STENCIL_OK, ctas = 0;
+                if constexpr (D == 3) rc = launch_stream_read<R, IrResidual<E, R>>(g, u, args, 1 << 30, s, &ctas);
+                else k_ir_resid_2d<E, R><<<blocks, 256, 0, s>>>(u, args, g);
+                if (rc) return rc;
+            }
             ST_CUDA(cudaGetLastError());
-            ST_CUDA(cudaMemcpyAsync(ea, r, n * sizeof(E), cudaMemcpyDeviceToDevice, s));
-            E *cur = ea, *nxt = eb;
+            E *cur = r, *nxt = ea;  // e_1 = r, read in place
             const bool streamed = lp_stream_supported(g, D);
             for (int it = 1; it < m; ++it) {
                 if (streamed) {
@@ -374,7 +409,8 @@ int ir_loop(const stencil_params &p, const stencil_ir_params &ir, float *u, char
                 } else {
                     k_lp_sweep<E, D, R><<<8 * num_sms(), 256, 0, s>>>(cur, nxt, r, g);
                 }
-                std::swap(cur, nxt);
+                cur = nxt;
+                nxt = cur == ea ? eb : ea;
             }
             ST_CUDA(cudaGetLastError());
             k_ir_update<E, D, R><<<blocks, 256, 0, s>>>(u, cur, g, scale);

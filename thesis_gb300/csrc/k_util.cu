@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "host.hpp"
+#include "stream_read.cuh"
 
 namespace st {
 
@@ -62,6 +63,12 @@ __global__ void k_copy_border(const float *__restrict__ src, float *__restrict__
 // result does not depend on scheduling) and divides by (2DR)^2.  One warp per
 // row of the update region (rows handed out round-robin), lanes along x.
 constexpr int kResidBlocks = 1024;
+// 3-D grids from this many cells on go through the streaming sweep's code,
+// with one more launch: GB300, stencil_residual, per-row kernel / stream, us:
+// 64^3 R = 1 46 / 52, 128^3 R = 2 55 / 63, 132 x 900 x 96 R = 3 133 / 116,
+// 256^3 R = 4 220 / 146, 512^3 R = 1 568 / 285, R = 4 1764 / 507, 768^3 R = 4
+// 5916 / 1500.
+constexpr long long kResidStreamCells = 1LL << 23;
 constexpr int kResidThreads = 256;
 
 __device__ __forceinline__ void block_sum2(double &a, double &b, double *sh) {
@@ -225,6 +232,103 @@ __global__ void __launch_bounds__(kResidThreads)
     if (threadIdx.x == 0) { part[2 * blockIdx.x] = rr; part[2 * blockIdx.x + 1] = bb; }
 }
 
+// 3-D, nx % 4 == 0 and R <= 4, large grids: the sums of d^2 from one pass of
+// the streaming sweep's code, and the border's part from the cells next to it.
+// (The per-row kernel above reads a cell from the L2 2R + 1 times over, with
+// the latency of each row's loads exposed: 768^3 R = 4 5830 us; this 1090, bound
+// by the sums as the sweep is, and the border's 350.)
+template <int R>
+struct NormOut {
+    struct Args { double *part; };
+    static constexpr bool kDiff = true;
+    double *part;
+    const Geom &g;
+    float s, cs;
+
+    __device__ NormOut(Args a, const Geom &g_) : part(a.part), g(g_), s(0.0f), cs(0.0f) {}
+    __device__ __forceinline__ void row(int x, int, int, const float2 (&d)[2], float4) {
+        const float v[4] = {d[0].x, d[0].y, d[1].x, d[1].y};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (in_range(x + e, g.nx, R)) acc_square(v[e], s, cs);
+    }
+    __device__ void finish() {
+        __shared__ double sh[2 * 32];
+        double rr = (double)s + (double)cs, none = 0.0;
+        block_sum2(rr, none, sh);
+        if (threadIdx.x == 0) part[2 * blockIdx.x] = rr;
+    }
+};
+
+// part[2 b + 1]: sums of bsum^2; part[2 b] of the blocks from `filled` on: 0.
+template <int R>
+__global__ void __launch_bounds__(kResidThreads)
+    k_residual_border_3d(const float *__restrict__ u, Geom g, int filled, double *__restrict__ part) {
+    __shared__ double sh[2 * (kResidThreads / 32)];
+    double none = 0.0, bb = 0.0;
+    // every load issued before the first is used (all lie in the grid)
+    auto cell = [&](int i, int j, int k, bool yz) {
+        const float *c = u + (long long)k * g.sz + (long long)j * g.sy + i;
+        float bs = 0.0f, x[2 * R + 1], v[4 * R];
+#pragma unroll
+        for (int o = -R; o <= R; ++o) x[R + o] = c[o];
+        if (yz)
+#pragma unroll
+            for (int o = 1; o <= R; ++o) {
+                v[2 * o - 2] = c[-o * g.sy];
+                v[2 * o - 1] = c[o * g.sy];
+                v[2 * R + 2 * o - 2] = c[-o * g.sz];
+                v[2 * R + 2 * o - 1] = c[o * g.sz];
+            }
+#pragma unroll
+        for (int o = -R; o <= R; ++o)
+            if (o && !in_range(i + o, g.nx, R)) bs += x[R + o];
+        if (yz) {
+#pragma unroll
+            for (int o = 1; o <= R; ++o) {
+                if (!in_range(j - o, g.ny, R)) bs += v[2 * o - 2];
+                if (!in_range(j + o, g.ny, R)) bs += v[2 * o - 1];
+            }
+#pragma unroll
+            for (int o = 1; o <= R; ++o) {
+                if (!in_range(k - o, g.nz, R)) bs += v[2 * R + 2 * o - 2];
+                if (!in_range(k + o, g.nz, R)) bs += v[2 * R + 2 * o - 1];
+            }
+        }
+        if (bs != 0.0f) bb = fma((double)bs, (double)bs, bb);
+    };
+    const int ry = g.ny - 2 * R, nrows = ry * (g.nz - 2 * R), lane = threadIdx.x & 31;
+    const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), warps = gridDim.x * (blockDim.x >> 5);
+    // rows near a y or z face, and every row of a grid too narrow for two ends
+    const bool narrow = g.nx < 4 * R;
+    // four rows per warp: 8 lanes for the 2R cells at a far row's ends
+    for (int q = 4 * warp; q < nrows; q += 4 * warps) {
+        const int qr = q + (lane >> 3), l = lane & 7;
+        const int j = R + qr % ry, k = R + qr / ry;
+        const bool near = narrow || j < 2 * R || j >= g.ny - 2 * R || k < 2 * R || k >= g.nz - 2 * R;
+        const bool in = qr < nrows;
+        if (in && !near && l < 2 * R) cell(l < R ? R + l : g.nx - 3 * R + l, j, k, false);
+        for (unsigned todo = __ballot_sync(~0u, in && near && l == 0); todo; todo &= todo - 1) {
+            const int n = q + ((__ffs(todo) - 1) >> 3);
+            for (int i = R + lane; i < g.nx - R; i += 32) cell(i, R + n % ry, R + n / ry, true);
+        }
+    }
+    block_sum2(none, bb, sh);
+    if (threadIdx.x == 0) {
+        if ((int)blockIdx.x >= filled) part[2 * blockIdx.x] = 0.0;
+        part[2 * blockIdx.x + 1] = bb;
+    }
+}
+
+template <int R>
+int launch_residual_stream(const Geom &g, const float *u, double *part, int blocks, cudaStream_t s) {
+    int ctas = 0;
+    const int rc = launch_stream_read<R, NormOut<R>>(g, u, {part}, blocks, s, &ctas);
+    if (rc) return rc;
+    k_residual_border_3d<R><<<blocks, kResidThreads, 0, s>>>(u, g, ctas, part);
+    return cuda_fail(cudaGetLastError(), "residual launch");
+}
+
 // inv_c2 = 1 / (2DR)^2 turns the sums of d^2 and bsum^2 into sums of r^2 and b^2.
 __global__ void __launch_bounds__(kResidThreads)
     k_residual_final(const double *__restrict__ part, int nparts, double *__restrict__ out,
@@ -263,6 +367,13 @@ size_t residual_scratch_bytes() { return (2 * kResidBlocks + 2) * sizeof(double)
 int launch_residual_partial(const Geom &g, int dims, const float *u, double *part, int blocks,
                             cudaStream_t s) {
     const bool vec = g.nx % 4 == 0 && g.radius <= 4;
+    if (vec && dims == 3 && (long long)g.nx * g.ny * g.nz >= kResidStreamCells)
+        switch (g.radius) {
+            case 1: return launch_residual_stream<1>(g, u, part, blocks, s);
+            case 2: return launch_residual_stream<2>(g, u, part, blocks, s);
+            case 3: return launch_residual_stream<3>(g, u, part, blocks, s);
+            default: return launch_residual_stream<4>(g, u, part, blocks, s);
+        }
     if (!vec) {
         k_residual_partial_any<<<blocks, kResidThreads, 0, s>>>(u, g, dims, part);
     } else {

@@ -15,9 +15,14 @@
 // share the grid (this CTA is number `cta` of them).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace st {
+
+template <class Out> struct OutDiff { static constexpr bool value = Out::kDiff; };
+template <> struct OutDiff<void> { static constexpr bool value = false; };
 
 template <int R, int TX, int TY, int RY, int NS>
 struct StreamShape {
@@ -78,18 +83,28 @@ __device__ __forceinline__ void fence_proxy_async_global() {
 // centre chunks by warp shuffles (only the lanes at the tile's x edges read
 // the halo chunk from shared memory) instead of two 16-byte shared loads per
 // row.  Returns early after a bounded wait gave up (the device status word
-// says so).
-template <int R, int TX, int TY, int RY, int NS, bool MULTI, bool XS>
+// says so).  Out: void for a sweep; else nothing is stored and every row of
+// four cells with one in the update region is given to out->row(x, y, z, sum,
+// centre) -- the new values or, with Out::kDiff, the sums of (neighbour -
+// centre) in place of the sums of neighbours, undivided.
+template <int R, int TX, int TY, int RY, int NS, bool MULTI, bool XS, class Out = void>
 __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uint64_t *empty,
                                                 uint64_t *swept, const CUtensorMap *map0,
                                                 const CUtensorMap *map1, float *dst0, float *dst1,
                                                 const Geom g, int tiles_x, int tiles_y, int zchunk,
                                                 int items, int sweeps, unsigned *grid_bar,
                                                 unsigned bar_base, unsigned cta, unsigned nctas,
-                                                bool entry_fence) {
+                                                bool entry_fence, Out *out = nullptr) {
     using S = StreamShape<R, TX, TY, RY, NS>;
     constexpr int C = 6 * R;  // 2*D*R with D = 3
     constexpr bool PK = R >= 3;
+    constexpr bool SWEEP = std::is_void<Out>::value;
+    constexpr bool DIFF = OutDiff<Out>::value;
+    // a pair of a sum's terms: the neighbours, or less their centres
+    auto term = [](float2 v, float2 c) {
+        if constexpr (DIFF) return add_pair<PK>(v, make_float2(-c.x, -c.y));
+        else return v;
+    };
     // How a consumer warp leaves after a bounded wait gave up: R = 1 returns
     // at once; R >= 2 clears `ok` and leaves its loops, and the warps agree at
     // a named barrier.  Same behaviour, but the code generated for each form
@@ -228,18 +243,21 @@ __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uin
                     // axis i: an even offset reads aligned pairs of the
                     // loaded vectors (pair adds), an odd one straddles them
                     // (scalar adds)
-                    acc[r][0] = make_float2(w[S::RA - R], w[S::RA - R + 1]);
-                    acc[r][1] = make_float2(w[S::RA - R + 2], w[S::RA - R + 3]);
+                    const float2 c01 = make_float2(c.x, c.y), c23 = make_float2(c.z, c.w);
+                    acc[r][0] = term(make_float2(w[S::RA - R], w[S::RA - R + 1]), c01);
+                    acc[r][1] = term(make_float2(w[S::RA - R + 2], w[S::RA - R + 3]), c23);
 #pragma unroll
                     for (int o = -R + 1; o <= R; ++o) {
                         if (o == 0) continue;
                         const int off = S::RA + o;
                         if ((off & 1) == 0) {
-                            acc[r][0] = add_pair<PK>(acc[r][0], make_float2(w[off], w[off + 1]));
-                            acc[r][1] = add_pair<PK>(acc[r][1], make_float2(w[off + 2], w[off + 3]));
+                            acc[r][0] = add_pair<PK>(acc[r][0], term(make_float2(w[off], w[off + 1]), c01));
+                            acc[r][1] = add_pair<PK>(acc[r][1], term(make_float2(w[off + 2], w[off + 3]), c23));
                         } else {
-                            acc[r][0].x += w[off]; acc[r][0].y += w[off + 1];
-                            acc[r][1].x += w[off + 2]; acc[r][1].y += w[off + 3];
+                            const float2 a = term(make_float2(w[off], w[off + 1]), c01);
+                            const float2 b = term(make_float2(w[off + 2], w[off + 3]), c23);
+                            acc[r][0].x += a.x; acc[r][0].y += a.y;
+                            acc[r][1].x += b.x; acc[r][1].y += b.y;
                         }
                     }
                     // axis j
@@ -247,15 +265,15 @@ __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uin
                     for (int o = -R; o <= R; ++o) {
                         if (o == 0) continue;
                         const float4 v = col[r + R + o];
-                        acc[r][0] = add_pair<PK>(acc[r][0], make_float2(v.x, v.y));
-                        acc[r][1] = add_pair<PK>(acc[r][1], make_float2(v.z, v.w));
+                        acc[r][0] = add_pair<PK>(acc[r][0], term(make_float2(v.x, v.y), c01));
+                        acc[r][1] = add_pair<PK>(acc[r][1], term(make_float2(v.z, v.w), c23));
                     }
                     // axis k, previous planes z-R .. z-1 (queue indices (ph + R + o) % QN)
 #pragma unroll
                     for (int o = -R; o <= -1; ++o) {
                         const float4 v = qz[r][(ph + R + o + QN) % QN];
-                        acc[r][0] = add_pair<PK>(acc[r][0], make_float2(v.x, v.y));
-                        acc[r][1] = add_pair<PK>(acc[r][1], make_float2(v.z, v.w));
+                        acc[r][0] = add_pair<PK>(acc[r][0], term(make_float2(v.x, v.y), c01));
+                        acc[r][1] = add_pair<PK>(acc[r][1], term(make_float2(v.z, v.w), c23));
                     }
                 }
                 // The centre slot is no longer read by this warp.
@@ -279,10 +297,11 @@ __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uin
                 for (int r = 0; r < RY; ++r)
 #pragma unroll
                     for (int o = 1; o <= R; ++o) {
-                        const float4 v = qz[r][(ph + R + o) % QN];
-                        acc[r][0] = add_pair<PK>(acc[r][0], make_float2(v.x, v.y));
-                        acc[r][1] = add_pair<PK>(acc[r][1], make_float2(v.z, v.w));
+                        const float4 v = qz[r][(ph + R + o) % QN], c = col[r + R];
+                        acc[r][0] = add_pair<PK>(acc[r][0], term(make_float2(v.x, v.y), make_float2(c.x, c.y)));
+                        acc[r][1] = add_pair<PK>(acc[r][1], term(make_float2(v.z, v.w), make_float2(c.z, c.w)));
                     }
+                if constexpr (!DIFF) {
                 // Epilogue: correctly rounded division by 6R.  The fast path
                 // applies when every stored sum lies in [2^-100, 2^120] (NaN
                 // sums pass through it as NaN); otherwise the warp divides.
@@ -309,6 +328,12 @@ __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uin
                             acc[r][h].y = div_slow_from_first<C>(acc[r][h].y);
                         }
                 }
+                }
+                if constexpr (!SWEEP) {
+#pragma unroll
+                    for (int r = 0; r < RY; ++r)
+                        if (live & (1u << r)) out->row(x, ybase + r, z, acc[r], col[r + R]);
+                } else {
                 if (g.legacy) {
 #pragma unroll
                     for (int r = 0; r < RY; ++r) {
@@ -334,6 +359,7 @@ __device__ __forceinline__ void stream3d_sweeps(float *ring, uint64_t *full, uin
                             for (int e = 0; e < 4; ++e)
                                 if (in_range(x + e, g.nx, R)) drow[r * g.sy + e] = v[e];
                         }
+                }
                 }
                 drow += g.sz;
             }
