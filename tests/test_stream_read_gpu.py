@@ -54,3 +54,39 @@ def test_refinement_step_of_one_sweep_is_exact(cuda, storage, shape, radius):
     d = torch.from_numpy(u).cuda()
     S.ir_solve_ex(d, radius, 1, storage, inner_sweeps=1)
     assert np.array_equal(d.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("storage,ulp", [("bf16", 2.0 ** -8), ("fp16", 2.0 ** -11)])
+@pytest.mark.parametrize("shape", [(9, 9, 8), (10, 41, 24), (22, 40, 136), (35, 9, 264), (300, 33, 128), (64, 300, 152)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_tensor_core_correction_sweeps(cuda, storage, ulp, shape):
+    """R = 4, three sweeps: z ranges shorter and longer than the plane ring, one
+    and several chunks, partial tiles.  Sums in FP64 here, so a cell's rounding
+    to 16 bits may fall the other way: one unit of the largest e (at most 1.5,
+    M being a mean) per sweep, and e is read as 16 bits once more at the end."""
+    import torch
+    from thesis_gb300 import stencil as S
+    R = 4
+    u = O.uniform(shape, seed=6) - np.float32(0.5)
+    swept = O.run(u.copy(), u.copy(), R, O.JACOBI, 1)
+    inner = (slice(R, -R),) * 3
+    r = swept[inner] - u[inner]
+    s = np.float32(np.ldexp(1.0, int(np.frexp(np.abs(r).max())[1])))
+    rhs = np.zeros(shape, np.float64)
+    rhs[inner] = IRO.ROUND[storage](r * (np.float32(1) / s))
+    e = rhs.copy()
+    for _ in range(2):
+        m = np.zeros(shape, np.float64)
+        for ax in range(3):
+            for o in (-4, -3, -2, -1, 1, 2, 3, 4):
+                m += np.roll(e, -o, ax)
+        nxt = np.zeros(shape, np.float64)
+        nxt[inner] = IRO.ROUND[storage]((m[inner] / 24 + rhs[inner]).astype(np.float32))
+        e = nxt
+    d = torch.from_numpy(u).cuda()
+    S.ir_solve_ex(d, R, 3, storage, inner_sweeps=3)
+    got = d.cpu().numpy()
+    assert np.abs(got - (u + s * e)).max() <= s * np.abs(e).max() * 3 * ulp
+    border = np.ones(shape, bool)
+    border[inner] = False
+    assert np.array_equal(got[border], u[border])

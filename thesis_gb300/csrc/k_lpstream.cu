@@ -331,8 +331,7 @@ __global__ void __launch_bounds__(LpShape<R>::THREADS, LpShape<R>::MIN_BLOCKS)
 // that also holds the centre, which the -1 of Bx cancels; W is the
 // accumulator the products are added to.  A warp owns one 16 x 16 block of
 // the CTA's 128 x 32 tile (16 consumer warps, two 16-row blocks sharing one
-// halo), so a cell costs about 0.3 warp instructions against about 1.4 for
-// the per-term mixed-precision adds.  The result differs from the in-order
+// halo).  The result differs from the in-order
 // FP32 sum by FP32 roundings only (the correction equation is not bound to
 // the reference's order).
 //
@@ -340,8 +339,13 @@ __global__ void __launch_bounds__(LpShape<R>::THREADS, LpShape<R>::MIN_BLOCKS)
 // structure with 128 x 16 tiles and per-thread rhs loads / stores 248 us (9
 // warps per SM: latency-bound); 128 x 32 tiles 195 us (the L1/TEX pipe 90 %
 // busy: per-thread global accesses in the mma fragment layout touch 8
-// half-used sectors per warp instruction); rhs and output by TMA as below:
-// 768^3 refinement 1.24x the FP32 loop.  The producer issues
+// half-used sectors per warp instruction); rhs and output by TMA 156 us, 207
+// warp instructions and 1420 cycles a block and plane, in one chain of waits,
+// shared loads, products and the store.  As below -- fragments by one
+// ldmatrix / stmatrix, the next plane's operands loaded a step ahead, ring
+// positions counted instead of divided, TMA issued by predicate in uniform
+// code -- it is bound by device memory: 768^3 518 -> 430 us (6.1 TB/s), 512^3
+// 159 -> 134, 128^3 10.4 -> 7.6, the same bits.  The producer issues
 // fence.proxy.async after acquiring a slot and before its TMA write into it,
 // ordering the consumers' generic-proxy reads (released to it through the
 // empty mbarrier) before the async-proxy write; repeated runs are
@@ -385,6 +389,11 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
+}
+__device__ __forceinline__ void stsm_x4(uint32_t addr, const uint32_t (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
 }
 __device__ __forceinline__ void ldsm_x2_t(uint32_t (&r)[2], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
@@ -434,23 +443,17 @@ struct Mma<__half> {
     }
 };
 
-// A bounded mbarrier wait that every lane of the warp leaves the same way
-// (the warp-wide ldmatrix / mma after it need all lanes).
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
-}
-
 // Data movement: the e plane tiles (152 x 40) by TMA into a ring of NE slots;
 //   * the producer also streams each step's rhs tile (136 x 32: 68-word rows,
 //     conflict-free fragment reads) into a ring of 4 slots, issued with the
 //     e plane that the same step first needs;
 //   * a consumer warp writes its 16 x 16 output block into one of two staging
-//     buffers and one lane stores it with cp.async.bulk.tensor (the box is
+//     buffers and its elected lane stores it with cp.async.bulk.tensor (the box is
 //     clipped at the grid's end; cells of the border band are written as 0,
 //     the value they hold for the whole refinement).
 template <int NE>
 struct LpTc3Shape {
-    static constexpr int R = 4, RB = 2, TY = 32;
+    static constexpr int R = 4, TY = 32;
     static constexpr int PH = TY + 2 * R;
     static constexpr int E_BYTES = kTcPW * PH * 2;            // 12160
     static constexpr int E_SLOT = (E_BYTES + 127) & ~127;
@@ -468,11 +471,12 @@ struct LpTc3Shape {
     static_assert(NE >= 2 * R + 2, "ring too short for the running z sum");
 };
 
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int x, int y, int z) {
+__device__ __forceinline__ void tma_store_3d_if(uint32_t on, const CUtensorMap *map, uint32_t src, int x, int y, int z) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "@p cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];\n\t}" ::"l"(
             reinterpret_cast<uint64_t>(map)),
-        "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z)
+        "r"(src), "r"(x), "r"(y), "r"(z), "r"(on)
         : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -499,7 +503,7 @@ __global__ void __launch_bounds__(LpTc3Shape<NE>::THREADS, 1)
     uint64_t *empty = full + NE;
     uint64_t *rfull = empty + NE;
     uint64_t *rempty = rfull + NR;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     if (tid == 0) {
         prefetch_tensormap(&e_map);
         prefetch_tensormap(&r_map);
@@ -518,32 +522,27 @@ __global__ void __launch_bounds__(LpTc3Shape<NE>::THREADS, 1)
     const int ntiles = tiles_x * tiles_y;
 
     if (warp == S::CWARPS) {
-        if (lane != 0) return;
-        uint32_t q = 0, qr = 0;
+        const uint32_t on = elect_lane(), es = smem_u32(ering), rs = smem_u32(rring);
+        RingPos e, r;
         for (int item = blockIdx.x; item < items; item += gridDim.x) {
             const int t = item % ntiles, ch = item / ntiles;
             const int x0 = (t % tiles_x) * kTcTX, y0 = (t / tiles_x) * S::TY;
             const int z0 = R + ch * zchunk, z1 = min(z0 + zchunk, g.nz - R);
-            const int np = (z1 - z0) + 2 * R;
-            for (int p = 0; p < np; ++p, ++q) {
-                const int s = (int)(q % NE);
-                const uint32_t use = q / NE;
-                if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1)) return;
+            for (int z = z0 - R; z < z1 + R; ++z) {
+                if (!warp_wait_bounded(&empty[e.slot], e.parity ^ 1)) return;
                 // the consumers' reads of the slot (they arrived after them)
                 // before this TMA write into it
                 fence_proxy_async();
-                mbar_arrive_expect_tx(&full[s], S::E_BYTES);
-                tma_load_3d(ering + s * S::E_SLOT, &e_map, &full[s], x0 - 8, y0 - R, z0 - R + p);
-                if (p >= 2 * R) {
-                    // the rhs of step p - 2R (plane z0 + p - 2R), first needed with e plane p
-                    const int rs = (int)(qr % NR);
-                    const uint32_t ruse = qr / NR;
-                    if (ruse > 0 && !mbar_wait_bounded(&rempty[rs], (ruse - 1) & 1)) return;
-                    fence_proxy_async();
-                    mbar_arrive_expect_tx(&rfull[rs], S::R_BYTES);
-                    tma_load_3d(rring + rs * S::R_SLOT, &r_map, &rfull[rs], x0, y0, z0 + p - 2 * R);
-                    ++qr;
-                }
+                expect_tx_if(on, smem_u32(&full[e.slot]), S::E_BYTES);
+                tma_load_3d_if(on, es + e.slot * S::E_SLOT, &e_map, smem_u32(&full[e.slot]), x0 - 8, y0 - R, z);
+                e.next(NE);
+                if (z < z0 + R) continue;
+                // the rhs of plane z - R, first needed with e plane z
+                if (!warp_wait_bounded(&rempty[r.slot], r.parity ^ 1)) return;
+                fence_proxy_async();
+                expect_tx_if(on, smem_u32(&rfull[r.slot]), S::R_BYTES);
+                tma_load_3d_if(on, rs + r.slot * S::R_SLOT, &r_map, smem_u32(&rfull[r.slot]), x0, y0, z - R);
+                r.next(NR);
             }
         }
         return;
@@ -577,137 +576,113 @@ __global__ void __launch_bounds__(LpTc3Shape<NE>::THREADS, 1)
     const uint32_t off_a = ((R + ry + rr + (mi & 1) * 8) * kTcPW + cw + (mi >> 1) * 8) * 2;
     const uint32_t off_b16 = ((ry + rr + (mi & 1) * 8) * kTcPW + cw + 8 + (mi >> 1) * 8) * 2;
     const uint32_t off_b8 = ((ry + 16 + rr) * kTcPW + cw + 8 + (mi & 1) * 8) * 2;
-    const uint32_t off_w = ((R + ry + gq) * kTcPW + cw + 8 + 2 * tq) * 2;
-    const uint32_t off_r = ((ry + gq) * S::RW + cw + 2 * tq) * 2;  // rhs words; +16: n block 1; +8 rows
-    const uint32_t off_o = (gq * 16 + 2 * tq) * 2;                 // staging words; +16; +8 rows
-    constexpr uint32_t HALF = 8 * kTcPW * 2, RHALF = 8 * S::RW * 2, OHALF = 8 * 16 * 2;
-    const uint32_t ering_s = smem_u32(ering);
-    unsigned char *stage0 = ostage + warp * 2 * S::STAGE;
-    // a slot's reads are done: one arrival per warp
-    auto release = [&](uint64_t *bar) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar);
+    // the block's own cells as the accumulator's fragment (also the rhs and
+    // the output): one ldmatrix / stmatrix of four 8 x 8 blocks
+    const uint32_t off_w = ((R + ry + rr + (mi >> 1) * 8) * kTcPW + cw + 8 + (mi & 1) * 8) * 2;
+    const uint32_t off_r = ((ry + rr + (mi >> 1) * 8) * S::RW + cw + (mi & 1) * 8) * 2;
+    const uint32_t off_o = ((rr + (mi >> 1) * 8) * 16 + (mi & 1) * 8) * 2;
+    const uint32_t on = elect_lane(), es = smem_u32(ering), rs = smem_u32(rring) + off_r;
+    const uint32_t stage0 = smem_u32(ostage) + warp * 2 * S::STAGE;
+    const uint32_t empty_s = smem_u32(empty), rempty_s = smem_u32(rempty);
+    // the 16-bit operands of the products of the plane in slot `at`
+    uint32_t a1[4], a2[4], b16[4], b8[2];
+    auto operands = [&](uint32_t at) {
+        ldsm_x4(a1, at + off_a);
+        ldsm_x4(a2, at + off_a + 32);
+        ldsm_x4_t(b16, at + off_b16);
+        ldsm_x2_t(b8, at + off_b8);
     };
-    auto bail = [&]() {
-        if (lane == 0) bulk_wait_all();
-    };
-    auto words = [&](int s, uint32_t (&wv)[2][2]) {
-        const unsigned char *b = ering + s * S::E_SLOT + off_w;
-        wv[0][0] = *reinterpret_cast<const uint32_t *>(b);
-        wv[0][1] = *reinterpret_cast<const uint32_t *>(b + 16);
-        wv[1][0] = *reinterpret_cast<const uint32_t *>(b + HALF);
-        wv[1][1] = *reinterpret_cast<const uint32_t *>(b + HALF + 16);
-    };
-    uint32_t qb = 0, qr = 0, sb = 0;  // e plane, rhs and staging sequence numbers
+    // positions of the newest, the centre and the oldest plane of a step
+    RingPos pn, pc, po, pr;
+    uint32_t flip = 0;  // this step's staging buffer
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int t = item % ntiles, ch = item / ntiles;
         const int x0 = (t % tiles_x) * kTcTX, y0 = (t / tiles_x) * S::TY;
         const int z0 = R + ch * zchunk, z1 = min(z0 + zchunk, g.nz - R);
-        const int np = (z1 - z0) + 2 * R;
         const int xa = x0 + cw + 2 * tq, ya = y0 + ry + gq;
         const bool r0 = in_range(ya, g.ny, R), r1 = in_range(ya + 8, g.ny, R);
         const bool c0 = xa >= R && xa + 1 < g.nx - R, c1 = xa + 8 >= R && xa + 9 < g.nx - R;
-        const bool ok[2][2] = {{r0 && c0, r0 && c1}, {r1 && c0, r1 && c1}};
-        float2 wsum[2][2];
+        const bool ok[4] = {r0 && c0, r0 && c1, r1 && c0, r1 && c1};
+        float2 wsum[4];  // fragment words: rows 0-7 and 8-15, each columns 0-7, 8-15
+        pc = pn;
 #pragma unroll
         for (int p = 0; p <= 2 * R; ++p) {
-            const uint32_t q = qb + p;
-            if (!warp_wait(&full[q % NE], (q / NE) & 1)) { bail(); return; }
-            uint32_t wv[2][2];
-            words((int)(q % NE), wv);
+            if (!warp_wait_bounded(&full[pn.slot], pn.parity)) { bulk_wait_all(); return; }
+            uint32_t wv[4];
+            ldsm_x4(wv, es + pn.slot * S::E_SLOT + off_w);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int nb = 0; nb < 2; ++nb) {
-                    const float2 v = Cvt<E>::two(wv[h][nb]);
-                    wsum[h][nb] = p == 0 ? v : fadd2(wsum[h][nb], v);
-                }
+            for (int i = 0; i < 4; ++i) {
+                const float2 v = Cvt<E>::two(wv[i]);
+                wsum[i] = p == 0 ? v : fadd2(wsum[i], v);
+            }
+            pn.next(NE);
+            if (p < R) pc.next(NE);
         }
+        operands(es + pc.slot * S::E_SLOT);
         for (int z = z0; z < z1; ++z) {
-            const int step = z - z0;
-            int old_slot = -1;
-            if (step > 0) {
-                const uint32_t qn = qb + step + 2 * R, qo = qb + step - 1;
-                if (!warp_wait(&full[qn % NE], (qn / NE) & 1)) { bail(); return; }
-                uint32_t wn[2][2], wo[2][2];
-                words((int)(qn % NE), wn);
-                words((int)(qo % NE), wo);
+            if (z > z0) {
+                if (!warp_wait_bounded(&full[pn.slot], pn.parity)) { bulk_wait_all(); return; }
+                uint32_t wn[4], wo[4];
+                ldsm_x4(wn, es + pn.slot * S::E_SLOT + off_w);
+                ldsm_x4(wo, es + po.slot * S::E_SLOT + off_w);
+                pn.next(NE);
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int nb = 0; nb < 2; ++nb) {
-                        const float2 d = ffma2(Cvt<E>::two(wo[h][nb]), make_float2(-1.0f, -1.0f),
-                                               Cvt<E>::two(wn[h][nb]));
-                        wsum[h][nb] = fadd2(wsum[h][nb], d);
-                    }
-                old_slot = (int)(qo % NE);
+                for (int i = 0; i < 4; ++i) {
+                    const float2 d = ffma2(Cvt<E>::two(wo[i]), make_float2(-1.0f, -1.0f), Cvt<E>::two(wn[i]));
+                    wsum[i] = fadd2(wsum[i], d);
+                }
             }
-            float wc[2][4];
-#pragma unroll
-            for (int nb = 0; nb < 2; ++nb) {
-                wc[nb][0] = wsum[0][nb].x; wc[nb][1] = wsum[0][nb].y;
-                wc[nb][2] = wsum[1][nb].x; wc[nb][3] = wsum[1][nb].y;
-            }
-            const uint32_t cs = ering_s + ((qb + step + R) % NE) * S::E_SLOT;
-            uint32_t a1[4], a2[4], b16[4], b8[2];
-            ldsm_x4(a1, cs + off_a);
-            ldsm_x4(a2, cs + off_a + 32);
-            ldsm_x4_t(b16, cs + off_b16);
-            ldsm_x2_t(b8, cs + off_b8);
             float acc[2][4];
 #pragma unroll
             for (int nb = 0; nb < 2; ++nb) {
+                const float wc[4] = {wsum[nb].x, wsum[nb].y, wsum[2 + nb].x, wsum[2 + nb].y};
                 float t1[4], t2[4], t3[4];
-                Mma<E>::k16(t1, a1, bx[0][nb][0], bx[0][nb][1], wc[nb]);
+                Mma<E>::k16(t1, a1, bx[0][nb][0], bx[0][nb][1], wc);
                 Mma<E>::k16(t2, a2, bx[1][nb][0], bx[1][nb][1], t1);
                 Mma<E>::k16(t3, ay16, b16[2 * nb], b16[2 * nb + 1], t2);
                 Mma<E>::k8(acc[nb], ay8, b8[nb], t3);
             }
+            // the next step's centre plane arrived R - 1 steps ago (at the last
+            // step this reads a plane that no product uses)
+            pc.next(NE);
+            operands(es + pc.slot * S::E_SLOT);
             // rhs of this step
-            const int rs = (int)(qr % NR);
-            if (!warp_wait(&rfull[rs], (qr / NR) & 1)) { bail(); return; }
-            uint32_t rw[2][2];
-            {
-                const unsigned char *b = rring + rs * S::R_SLOT + off_r;
-                rw[0][0] = *reinterpret_cast<const uint32_t *>(b);
-                rw[0][1] = *reinterpret_cast<const uint32_t *>(b + 16);
-                rw[1][0] = *reinterpret_cast<const uint32_t *>(b + RHALF);
-                rw[1][1] = *reinterpret_cast<const uint32_t *>(b + RHALF + 16);
-            }
+            if (!warp_wait_bounded(&rfull[pr.slot], pr.parity)) { bulk_wait_all(); return; }
+            uint32_t rw[4], ow[4];
+            ldsm_x4(rw, rs + pr.slot * S::R_SLOT);
             // the staging buffer of this step: free once the store issued two
-            // steps ago has read it
-            unsigned char *st = stage0 + (sb & 1) * S::STAGE;
-            if (lane == 0) bulk_wait_read<1>();
+            // steps ago (by the elected lane) has read it
+            const uint32_t st = stage0 + flip;
+            bulk_wait_read<1>();
             __syncwarp();
             constexpr float kInv = 1.0f / (float)C;
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int nb = 0; nb < 2; ++nb) {
-                    const float2 r = Cvt<E>::two(rw[h][nb]);
-                    const float2 o = ffma2(make_float2(acc[nb][2 * h], acc[nb][2 * h + 1]),
-                                           make_float2(kInv, kInv), r);
-                    *reinterpret_cast<uint32_t *>(st + off_o + h * OHALF + nb * 16) =
-                        ok[h][nb] ? Cvt<E>::pack(o.x, o.y) : 0u;
-                }
+            for (int i = 0; i < 4; ++i) {
+                const float2 r = Cvt<E>::two(rw[i]);
+                const int nb = i & 1, h = i >> 1;
+                const float2 o = ffma2(make_float2(acc[nb][2 * h], acc[nb][2 * h + 1]), make_float2(kInv, kInv), r);
+                ow[i] = ok[i] ? Cvt<E>::pack(o.x, o.y) : 0u;
+            }
+            stsm_x4(st + off_o, ow);
             // the staged block becomes visible to the bulk copy, then one lane
             // stores it
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) {
-                tma_store_3d(&o_map, st, x0 + cw, y0 + ry, z);
-                bulk_commit();
+            tma_store_3d_if(on, &o_map, st, x0 + cw, y0 + ry, z);
+            bulk_commit();
+            flip ^= S::STAGE;
+            mbar_arrive_if(on, rempty_s + 8 * pr.slot);
+            pr.next(NR);
+            if (z > z0) {
+                mbar_arrive_if(on, empty_s + 8 * po.slot);
+                po.next(NE);
             }
-            ++sb;
-            release(&rempty[rs]);
-            ++qr;
-            if (old_slot >= 0) release(&empty[old_slot]);
         }
-        const int last = (z1 - z0) - 1;
-        for (int p = last; p < np; ++p) release(&empty[(qb + p) % NE]);
-        qb += np;
+        // the last step's planes z1 - 1 - R .. z1 - 1 + R
+        __syncwarp();
+        for (; po.slot != pn.slot; po.next(NE)) mbar_arrive_if(on, empty_s + 8 * po.slot);
     }
-    if (lane == 0) bulk_wait_all();
+    bulk_wait_all();
 }
 
 template <typename E, int NE>

@@ -201,20 +201,6 @@ __device__ __forceinline__ constexpr uint32_t umma_idesc() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// One issuing thread, uniform code: the whole warp runs the loop, so that the
-// compiler keeps addresses, coordinates and descriptors in uniform registers
-// (where TMA and MMA instructions take them), and only the instructions
-// themselves are predicated on the elected lane.  In a branch of one lane
-// every operand is moved to a uniform register first: about 90 cycles an MMA
-// and 200 a TMA load, on the weight gradient of 128 x 128 x 32 channels.
-__device__ __forceinline__ uint32_t elect_lane() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p;
-}
-
-__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
-
 __device__ __forceinline__ void tc_commit_if(uint32_t on, uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
@@ -228,24 +214,6 @@ __device__ __forceinline__ void mma_f16_if(uint32_t on, uint32_t d, uint64_t a, 
         "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
         "r"(acc), "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void expect_tx_if(uint32_t on, uint32_t bar, uint32_t bytes) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
-        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
-        "r"(bytes), "r"(on)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d_if(uint32_t on, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                               int c1, int c2) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
-        "@p cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(on)
         : "memory");
 }
 
@@ -268,23 +236,6 @@ __device__ __forceinline__ void tma_load_5d_if(uint32_t on, uint32_t dst, const 
         "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(on)
         : "memory");
 }
-
-// mbar_wait_bounded of a whole warp; its lanes agree on the outcome.
-__device__ __forceinline__ bool warp_wait_bounded(uint64_t *bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
-}
-
-// A ring position: slot, and the parity of the slot's current use.
-struct RingPos {
-    int slot = 0;
-    uint32_t parity = 0;
-    __device__ __forceinline__ void next(int n) {
-        if (++slot == n) {
-            slot = 0;
-            parity ^= 1;
-        }
-    }
-};
 
 // ---------------------------------------------------------------------------
 // Tiles fed by TMA.  A tile is 128 pixels, 128 /
