@@ -57,7 +57,7 @@ def test_refinement_step_of_one_sweep_is_exact(cuda, storage, shape, radius):
 
 
 @pytest.mark.parametrize("storage,ulp", [("bf16", 2.0 ** -8), ("fp16", 2.0 ** -11)])
-@pytest.mark.parametrize("shape", [(9, 9, 8), (10, 41, 24), (22, 40, 136), (35, 9, 264), (300, 33, 128), (64, 300, 152)],
+@pytest.mark.parametrize("shape", [(9, 9, 16), (10, 41, 24), (22, 40, 136), (35, 9, 264), (300, 33, 128), (64, 300, 152)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_tensor_core_correction_sweeps(cuda, storage, ulp, shape):
     """R = 4, three sweeps: z ranges shorter and longer than the plane ring, one
