@@ -1417,9 +1417,19 @@ int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act
     return cuda_fail(cudaGetLastError(), "conv3x3 (tcgen05, TMA) launch");
 }
 
+// Tiles of BN output channels, or of half as many as long as all their CTAs
+// still find an SM of their own: a lone CTA's time is its chain of K chunks,
+// each as long as its TMA rows (128 of the input, BN of the weights) take.
+// One image, us: 32^2 384 -> 128 14.9 -> 8.9 with 32 output channels a tile
+// instead of 128, 16^2 256 -> 256 16.3 -> 9.5, 64^2 192 -> 64 9.5 -> 7.8.
 template <int BN>
 int launch_conv_tma(const unet_act *x, const bf16 *wb, const float *b, const Act &ya, const Act &gate, int relu,
                     int dil, cudaStream_t s) {
+    if constexpr (BN > 32) {
+        const int tw = tma_tile_w(x->h, x->w), th = BM / tw;
+        const long long tiles = (long long)((x->w + tw - 1) / tw) * ((x->h + th - 1) / th) * x->n;
+        if (2 * tiles * (ya.c / BN) <= num_sms()) return launch_conv_tma<BN / 2>(x, wb, b, ya, gate, relu, dil, s);
+    }
     return x->c % 64 == 0 ? launch_conv_tma<BN, 64>(x, wb, b, ya, gate, relu, dil, s)
                           : launch_conv_tma<BN, 32>(x, wb, b, ya, gate, relu, dil, s);
 }
