@@ -15,6 +15,10 @@ BATCHES = {
     # equal grids, more and fewer than the CTAs; some with no sweep
     "equal": [((40, 44), 2, 5, "jacobi")] * 200,
     "few": [((150, 131), 3, 7, "legacy"), ((30, 33, 37), 4, 5, "jacobi"), ((64, 64), 1, 0, "jacobi")],
+    # either tile at R <= 2: widths around 64, 128 and 192, heights around 60
+    "narrow_tiles": [((40, 93, 42), 2, 4, "jacobi"), ((21, 61, 63), 2, 3, "legacy"), ((30, 121, 150), 2, 3, "jacobi"),
+                     ((33, 59, 190), 2, 2, "jacobi"), ((9, 64, 200), 2, 5, "jacobi"), ((26, 163, 176), 2, 3, "legacy"),
+                     ((17, 31, 66), 1, 4, "jacobi"), ((12, 91, 129), 1, 3, "jacobi")],
     "no_sweeps": [((16, 16), 1, 0, "jacobi"), ((12, 12, 12), 2, 0, "jacobi")],
 }
 

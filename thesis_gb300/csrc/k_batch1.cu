@@ -51,15 +51,18 @@ namespace {
 // block is 16 warps: four per SM sub-partition leave 128 registers a thread
 // (17 warps would leave 96, too few for the code of every radius in one
 // kernel without spills).
-// N: narrow tiles (64 x 30) for grids at most 64 cells wide at R <= 2, where
-// a 128-wide tile would leave most consumer threads without cells.
+// N: tiles half as wide, at R <= 2, for grids that they cover with less waste
+// (b1_best_us).  At R = 2 64 x 60 with two rows per thread: a plane of one takes
+// 0.62 us, as of a 128 x 30 one, while 64 x 30 with one row per thread took
+// 0.41 for half the cells (225 x 93 x 42: 4 tiles' 1.65 us -> 1.24; 32 x 163 x
+// 176: 12 wide tiles' 7.4 us -> 5.6).
 template <int R, bool N = false> struct B1S;
 template <> struct B1S<1, false> { static constexpr int TX = 128, TY = 15, RY = 1, NS = 16; };
 template <> struct B1S<2, false> { static constexpr int TX = 128, TY = 30, RY = 2, NS = 8; };
 template <> struct B1S<3, false> { static constexpr int TX = 128, TY = 15, RY = 1, NS = 8; };
 template <> struct B1S<4, false> { static constexpr int TX = 128, TY = 15, RY = 1, NS = 8; };
 template <> struct B1S<1, true> { static constexpr int TX = 64, TY = 30, RY = 1, NS = 16; };
-template <> struct B1S<2, true> { static constexpr int TX = 64, TY = 30, RY = 1, NS = 16; };
+template <> struct B1S<2, true> { static constexpr int TX = 64, TY = 60, RY = 2, NS = 8; };
 template <int R, bool N = false>
 using B1Shape = StreamShape<R, B1S<R, N>::TX, B1S<R, N>::TY, B1S<R, N>::RY, B1S<R, N>::NS>;
 
@@ -490,11 +493,21 @@ double b1_sweep_us(const Geom &g, int dims, bool narrow, int k) {
                                                 : 1.03 * rows * chunks / (k * kB1Threads);
         return busy * row[R] + first[R];
     }
-    static const double plane[5] = {0, 0.359, 0.621, 0.419, 0.459}, plane_narrow[3] = {0, 0.373, 0.413};
+    static const double plane[5] = {0, 0.359, 0.621, 0.419, 0.459}, plane_narrow[3] = {0, 0.373, 0.621};
     int tx, ty, tiles_x, tiles_y, zchunk, items;
     b1_tile(g, narrow, &tx, &ty);
     stream3d_plan(g, tx, ty, k, &tiles_x, &tiles_y, &zchunk, &items);
     return (double)((items + k - 1) / k) * (zchunk * (narrow ? plane_narrow : plane)[R] + 0.5) + 3.0;
+}
+
+// The faster tile's time, and which.
+double b1_best_us(const Geom &g, int dims, int k, int *narrow) {
+    const double wide_us = b1_sweep_us(g, dims, false, k);
+    *narrow = 0;
+    if (dims == 2 || g.radius > 2) return wide_us;
+    const double narrow_us = b1_sweep_us(g, dims, true, k);
+    *narrow = narrow_us < wide_us;
+    return std::min(narrow_us, wide_us);
 }
 
 struct B1Cost {
@@ -506,9 +519,10 @@ struct B1Cost {
 // When the last grid ends, by the kernel's own schedule: each team takes its
 // tier's next grid (`order`: largest work first) when it is free, and splits
 // for the next tier once that queue is empty.  While the grids being swept do
-// not fit the L2 together, the 2-D ones take up to 1.65 times as long (1.5 to
-// 1.7 measured; the 3-D ones 1.03 to 1.1, left out): many large grids on small
-// teams lose to few on large ones.  *last is the grid that ends last.
+// not fit the L2 together, the 2-D ones take 1.65 times as long, and more the
+// more bytes they have (R = 1 1.6 at 150 MB, 1.75 at 300, 2.1 at 1200; the 3-D
+// ones 1.03 to 1.1, left out): many large grids on small teams lose to few on
+// large ones.  *last is the grid that ends last.
 double b1_schedule(const std::vector<int> &ladder, const std::vector<B1Cost> &cost, const std::vector<int> &order,
                    const std::vector<int> &tier_of, int *last) {
     constexpr double kOutside = 1.65, kFits = 70, kSpills = 125;  // MB of the L2's 129
@@ -545,7 +559,8 @@ double b1_schedule(const std::vector<int> &ladder, const std::vector<B1Cost> &co
             }
         }
         if (busy[0].empty() && busy[1].empty()) return now[0];
-        const double slow = 1 + (kOutside - 1) * std::min(1.0, std::max(0.0, (mb - kFits) / (kSpills - kFits)));
+        const double slow = mb > kSpills ? kOutside + 0.12 * std::log2(mb / kSpills)
+                                         : 1 + (kOutside - 1) * std::max(0.0, (mb - kFits) / (kSpills - kFits));
         const double d0 = busy[0].empty() ? 1e300 : busy[0][0].until - now[0];
         const double d1 = busy[1].empty() ? 1e300 : (busy[1][0].until - now[1]) * slow;
         const int k = d1 < d0;
@@ -569,12 +584,12 @@ double b1_schedule(const std::vector<int> &ladder, const std::vector<B1Cost> &co
 // the sweeps of a grid nor how many grids share the GPU.  GB300, milliseconds
 // a launch by the rule -> by this, the model's figures in brackets: 36 2-D
 // (64 to 2048 a side, R = 1) and 12 3-D grids (32 to 256, R = 2), 100 to 500
-// sweeps 19.7 -> 14.8 (20.4 -> 13.9); 23 and 7 grids 7.95 -> 2.58; 14 and 4
-// 4.55 -> 2.52; 26 and 2 3.45 -> 1.38; 40 and 11 9.10 -> 9.22; 11 and 15 13.2
-// -> 12.1; 384 and 128 with 20 sweeps 11.46 -> 10.95; the 512-grid benchmark
-// batch keeps the rule's plan (2592 ms, 2603 by the model).  The search takes
-// 0.15 ms of host time at 48 grids, 0.8 ms at 512; from 4096 grids on, which
-// leave little to gain at the end, there is none.
+// sweeps 21.1 -> 14.2 (20.0 -> 13.1); 23 and 7 grids 7.95 -> 2.66; 14 and 4
+// 4.55 -> 2.53; 26 and 2 3.45 -> 1.39; 40 and 11 9.10 -> 7.81; 384 and 128
+// 145.0 -> 130.4 (140.8 -> 125.9), with 20 sweeps 11.33 -> 10.84.  11 and 15
+// (10.6 ms) and the 512-grid benchmark batch (2508 ms, 2462 by the model) keep
+// the rule's plan.  The search takes 0.2 ms of host time at 48 grids, 1.2 ms at
+// 512; from 4096 grids on, which leave little to gain at the end, there is none.
 void plan_tiers(const std::vector<int> &ladder, const std::vector<B1Cost> &cost, const std::vector<int> &order,
                 const std::vector<char> &fixed, std::vector<int> *tier_of) {
     const int L = (int)ladder.size(), n = (int)order.size();
@@ -716,26 +731,12 @@ int batch1_prepare(const stencil_batch_job *jobs, int njobs, void *d_workspace,
         while (ladder[t] > want) ++t;
         tier_of[i] = t;
         work[i] = (double)cells * b.iterations;
-        J.narrow = p.dims == 3 && p.radius <= 2 && p.nx <= 64;
-        if (p.dims == 3) {
-            int tx = 0, ty = 0;
-            b1_tile(g, J.narrow, &tx, &ty);
-            CUtensorMap m[2];
-            const long long dims[3] = {g.nx, g.ny, g.nz};
-            const int box[3] = {tx + 2 * ((p.radius + 3) & ~3), ty + 2 * p.radius, 1};
-            rc = make_tensor_map(&m[0], J.a, 3, dims, box, g.sy, true);
-            if (!rc) rc = make_tensor_map(&m[1], J.b, 3, dims, box, g.sy, true);
-            if (rc) return rc;
-            J.map_pair = (int)(maps.size() / 2);
-            maps.push_back(m[0]);
-            maps.push_back(m[1]);
-        } else if ((long long)(g.sy / 4) * (g.ny - 2 * g.radius) >= (1LL << 31)) {
+        if (p.dims == 2 && (long long)(g.sy / 4) * (g.ny - 2 * g.radius) >= (1LL << 31))
             return fail(STENCIL_EUNSUPPORTED, "job %d: 2-D grid of 2^31 or more chunk-rows", i);
-        }
         if (!by_rule) {
             cost[i].mb = 8e-6 * (double)J.rows * g.sy;
             cost[i].rows = p.dims == 2;
-            for (int k : ladder) cost[i].us.push_back(b.iterations * b1_sweep_us(g, p.dims, J.narrow, k));
+            for (int k : ladder) cost[i].us.push_back(b.iterations * b1_best_us(g, p.dims, k, &J.narrow));
         }
     }
     // largest work first, then by tier: the job table's order
@@ -748,9 +749,20 @@ int batch1_prepare(const stencil_batch_job *jobs, int njobs, void *d_workspace,
         B1Job &J = table[i];
         const int team = ladder[tier_of[i]];
         if (J.dims == 3) {
+            const Geom &g = J.g;
             int tx = 0, ty = 0;
-            b1_tile(J.g, J.narrow, &tx, &ty);
-            stream3d_plan(J.g, tx, ty, team, &J.tiles_x, &J.tiles_y, &J.zchunk, &J.items);
+            b1_best_us(g, 3, team, &J.narrow);
+            b1_tile(g, J.narrow, &tx, &ty);
+            stream3d_plan(g, tx, ty, team, &J.tiles_x, &J.tiles_y, &J.zchunk, &J.items);
+            CUtensorMap m[2];
+            const long long dims[3] = {g.nx, g.ny, g.nz};
+            const int box[3] = {tx + 2 * ((g.radius + 3) & ~3), ty + 2 * g.radius, 1};
+            rc = make_tensor_map(&m[0], J.a, 3, dims, box, g.sy, true);
+            if (!rc) rc = make_tensor_map(&m[1], J.b, 3, dims, box, g.sy, true);
+            if (rc) return rc;
+            J.map_pair = (int)(maps.size() / 2);
+            maps.push_back(m[0]);
+            maps.push_back(m[1]);
         } else {
             rows2d_plan(J.g, (long long)team * kB1Threads, &J.hb, &J.nblk);
         }
