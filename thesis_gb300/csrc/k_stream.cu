@@ -174,7 +174,8 @@ namespace {
 
 // Persistent sweeps at R >= 3, which are issue-bound: the shape whose busiest
 // CTA takes least time over its planes, at the time of a plane measured for
-// each (us on one CTA per SM, within 5 % over 64^3 to 768^3).  Two rows per
+// each (us on one CTA per SM, a chunk's 2R halo planes counting as four; within
+// 5 % over 256^3 to 768^3), and by 3 % or more.  Two rows per
 // thread share their y-neighbours' loads and keep two chains of sums in
 // flight, so a row costs 20 % less than with one, but the taller tiles fill
 // small or odd grids worse.  GB300, us a sweep, 128 x 16 / two rows 128 wide /
@@ -185,15 +186,15 @@ namespace {
 // 53.6.
 int wide_shape(const Geom &g, int ctas) {
     static const struct { int shape; double plane_us[2]; } kShapes[3] = {
-        {4, {0.47, 0.49}}, {7, {0.69, 0.62}}, {8, {0.70, 0.62}}};
+        {4, {0.458, 0.48}}, {7, {0.672, 0.59}}, {8, {0.685, 0.59}}};
     int best = 4;
     double least = 1e300;
     for (const auto &c : kShapes) {
         const StreamKernel k = pick(g.radius, c.shape);
         int tiles_x, tiles_y, zchunk, items;
         stream3d_plan(g, k.tx, k.ty, ctas, &tiles_x, &tiles_y, &zchunk, &items);
-        const double us = (double)((items + ctas - 1) / ctas) * (zchunk + 1) * c.plane_us[g.radius - 3];
-        if (us < least) { least = us; best = c.shape; }
+        const double us = (double)((items + ctas - 1) / ctas) * (zchunk + 4) * c.plane_us[g.radius - 3];
+        if (us < 0.97 * least) { least = us; best = c.shape; }
     }
     return best;
 }
