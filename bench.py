@@ -396,7 +396,7 @@ def bench_c1(S, lib, torch, steps=5):
     O.run(h.copy(), h.copy(), R, O.JACOBI, sweeps, 1)
     cpu_s = time.perf_counter() - t0
     return {"workload": "2D 256^2 FP32 R=1 Jacobi, 1000 sweeps (one cooperative launch, tiles and "
-                        "halos in shared memory, exchanged through L2 every few sweeps)",
+                        "halos on chip, exchanged through L2 every few sweeps)",
             "value": round(ups / min(times) / 1e9, 3), "unit": "GCell-updates/s",
             "ms_per_solve": round(min(times) * 1e3, 4), "us_per_sweep": round(min(times) / sweeps * 1e6, 3),
             "engine": engine, "gpu_launches": launches,

@@ -37,6 +37,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <array>
 #include <mutex>
 #include <vector>
 
@@ -718,32 +719,51 @@ bool ir2_make_plan(const Geom &g, int t, int tx, int ty, int max_ctas, Ir2Plan *
 // best): an exchange costs 1060 cycles plus 4.16 per halo quad, a sweep 278
 // cycles plus 1.33 per 8-cell chunk of its region and 136 per further chunk
 // slot of a thread.
-double ir2_cost(const Geom &g, const Ir2Plan &p) {
-    const int R = g.radius, ni = ir2_items(p);
+double ir2_sweep_cost(const Geom &g, int tx, int ty, int ext) {
+    const int chunks = (tx + 2 * roundup8(ext)) / 8, rows = ty + 2 * ext;
+    return 278.0 + 1.33 * chunks * rows;
+}
+// sweeps: ir2_sweep_cost of the plan's T sweeps
+double ir2_cost(const Ir2Plan &p, double sweeps) {
     const long long ring = ((long long)p.pw * p.ph - (long long)p.tx * p.ty) / 4;
-    double c = 1060.0 + 4.16 * ring;
-    for (int k = 1; k <= p.t; ++k) {
-        const int ext = (p.t - k) * R;
-        const int chunks = (p.tx + 2 * roundup8(ext)) / 8, rows = p.ty + 2 * ext;
-        c += 278.0 + 136.0 * (ni - 1) + 1.33 * chunks * rows;
-    }
-    return c / p.t;
+    return (1060.0 + 4.16 * ring + sweeps) / p.t + 136.0 * (ir2_items(p) - 1);
+}
+double ir2_cost(const Geom &g, const Ir2Plan &p) {
+    double sweeps = 0;
+    for (int k = 0; k < p.t; ++k) sweeps += ir2_sweep_cost(g, p.tx, p.ty, k * g.radius);
+    return ir2_cost(p, sweeps);
 }
 
+// The cheapest plan, kept by sizes as the FP32 engine's is (at most 256 of
+// them).  In the search a tile's depths share the sum of their sweeps' costs
+// and end at the first that does not fit: 18 us of host time, 50 with each
+// depth on its own.
 bool ir2_choose(const Geom &g, int m, int temporal, int tile_x, int tile_y, int max_ctas,
                 Ir2Plan *out) {
     const int tmax = std::max(1, std::min(m, kIr2MaxT - 1));
+    typedef std::array<int, 8> Key;
+    static std::mutex mu;
+    static std::vector<std::pair<Key, Ir2Plan>> cache;
+    const Key key = {g.nx, g.ny, g.radius, tmax, temporal, tile_x, tile_y, max_ctas};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        for (const auto &c : cache)
+            if (c.first == key) { *out = c.second; return true; }
+    }
     bool found = false;
     double best = 1e30;
-    for (int t = 1; t <= tmax; ++t) {
-        if (temporal > 0 && t != std::min(temporal, tmax)) continue;
-        for (int tx : {16, 24, 32, 40, 48, 64, 80, 96, 128, 256}) {
-            if (tile_x > 0 && tx != tile_x) continue;
-            for (int ty : {4, 8, 12, 16, 20, 24, 32, 40, 48, 56, 64, 128}) {
-                if (tile_y > 0 && ty != tile_y) continue;
+    for (int tx : {16, 24, 32, 40, 48, 64, 80, 96, 128, 256}) {
+        if (tile_x > 0 && tx != tile_x) continue;
+        for (int ty : {4, 8, 12, 16, 20, 24, 32, 40, 48, 56, 64, 128}) {
+            if (tile_y > 0 && ty != tile_y) continue;
+            if ((long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) > max_ctas) continue;
+            double sweeps = 0;
+            for (int t = 1; t <= tmax; ++t) {
+                sweeps += ir2_sweep_cost(g, tx, ty, (t - 1) * g.radius);
                 Ir2Plan q;
-                if (!ir2_make_plan(g, t, tx, ty, max_ctas, &q)) continue;
-                const double c = std::min(ir2_cost(g, q), ir2_reg_plan(g.radius, q).cost);
+                if (!ir2_make_plan(g, t, tx, ty, max_ctas, &q)) break;  // nor does a deeper one
+                if (temporal > 0 && t != std::min(temporal, tmax)) continue;
+                const double c = std::min(ir2_cost(q, sweeps), ir2_reg_plan(g.radius, q).cost);
                 if (c < best - 1e-9) {
                     best = c;
                     *out = q;
@@ -755,6 +775,11 @@ bool ir2_choose(const Geom &g, int m, int temporal, int tile_x, int tile_y, int 
     if (!found && tile_x > 0 && tile_y > 0)
         found = ir2_make_plan(g, temporal > 0 ? std::min(temporal, tmax) : 1, tile_x, tile_y,
                               max_ctas, out);
+    if (found) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (cache.size() >= 256) cache.clear();
+        cache.emplace_back(key, *out);
+    }
     return found;
 }
 
