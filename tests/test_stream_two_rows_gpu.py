@@ -1,4 +1,4 @@
-"""3-D sweeps at R = 3 and 4 on the tiles with two rows per thread, 128 or 64
+"""3-D sweeps at R = 2, 3 and 4 on the tiles with two rows per thread, 128 or 64
 cells wide, and on the narrow ones beside them: bit for bit the oracle's."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 # tile wide, few long and many short chunks
 GRIDS = [((60, 181, 128), 3, 3), ((61, 331, 132), 3, 4), ((90, 301, 64), 3, 2), ((300, 121, 68), 3, 2),
          ((200, 90, 252), 3, 3), ((31, 500, 124), 3, 5), ((61, 331, 132), 4, 4), ((90, 301, 64), 4, 3),
-         ((300, 121, 68), 4, 2), ((200, 88, 252), 4, 3), ((33, 500, 124), 4, 5), ((250, 221, 192), 4, 2)]
+         ((300, 121, 68), 4, 2), ((200, 88, 252), 4, 3), ((33, 500, 124), 4, 5), ((250, 221, 192), 4, 2),
+         ((90, 301, 64), 2, 3), ((130, 61, 56), 2, 4), ((130, 55, 144), 2, 3), ((200, 121, 60), 2, 2)]
 
 
 @pytest.mark.parametrize("case", GRIDS, ids=lambda c: "x".join(map(str, c[0])) + "_r%d_i%d" % c[1:])
@@ -35,7 +36,7 @@ def test_two_row_tiles_match_oracle(cuda, case, mode):
     assert S.device_status() == 0
 
 
-@pytest.mark.parametrize("shape,radius", [((61, 331, 129), 3), ((90, 301, 63), 4), ((160, 200, 126), 4)])
+@pytest.mark.parametrize("shape,radius", [((150, 179, 59), 2), ((61, 331, 129), 3), ((90, 301, 63), 4), ((160, 200, 126), 4)])
 def test_two_row_tiles_on_pitched_copies(cuda, shape, radius):
     import torch
     from thesis_gb300 import stencil as S

@@ -93,10 +93,10 @@ StreamKernel sk() {
 // per thread (more warps, fewer registers each); 3 = a 16-slot ring (more
 // planes in flight, one CTA per SM); 4 (R >= 3) = 128 x 16, one row per
 // thread, 16 consumer warps in one CTA; 5 (R <= 2) = 128 x 32, two rows per
-// thread (half the y-halo rows per output row); 7 and 8 (R >= 3) = two rows
-// per thread, as many as 12 (R = 4) or 16 warps (R = 3) take with 168 and 128
-// registers a thread, 128 or 64 cells wide.  The persistent form exists for
-// the shapes it uses (R = 1: 3, R = 2: 5 and 6, R >= 3: 4, 7 and 8).
+// thread (half the y-halo rows per output row); 7 and 8 = two rows per
+// thread, as many as 12 (R = 4) or 16 warps take with 168 and 128 registers a
+// thread, 128 (7, R >= 3) or 64 cells wide (8, R >= 2).  The persistent form
+// exists for the shapes it uses (R = 1: 3, R = 2: 5, 6 and 8, R >= 3: 4, 7 and 8).
 StreamKernel pick(int r, int shape) {
     // shape 6: the persistent-form shape of the radius with x neighbours by
     // warp shuffles (A/B against the shared-memory reads)
@@ -111,7 +111,7 @@ StreamKernel pick(int r, int shape) {
     }
     switch (r) {
         case 1: return shape == 5 ? sk<1, 128, 32, 2, 8>() : shape == 3 ? sk<1, 128, 16, 1, 16, true>() : shape == 2 ? sk<1, 128, 16, 1, 8>() : shape == 1 ? sk<1, 64, 32, 2, 8>() : sk<1, 128, 16, 2, 8>();
-        case 2: return shape == 5 ? sk<2, 128, 32, 2, 8, true>() : shape == 3 ? sk<2, 128, 16, 1, 16>() : shape == 2 ? sk<2, 128, 16, 1, 8>() : shape == 1 ? sk<2, 64, 32, 2, 8>() : sk<2, 128, 16, 2, 8>();
+        case 2: return shape == 8 ? sk<2, 64, 60, 2, 8, true>() : shape == 5 ? sk<2, 128, 32, 2, 8, true>() : shape == 3 ? sk<2, 128, 16, 1, 16>() : shape == 2 ? sk<2, 128, 16, 1, 8>() : shape == 1 ? sk<2, 64, 32, 2, 8>() : sk<2, 128, 16, 2, 8>();
         case 3: return shape == 7 ? sk<3, 128, 30, 2, 8, true>() : shape == 8 ? sk<3, 64, 60, 2, 8, true>() : shape == 4 ? sk<3, 128, 16, 1, 8, true>() : shape == 2 ? sk<3, 128, 8, 1, 8>() : shape == 1 ? sk<3, 64, 32, 2, 8>() : sk<3, 128, 16, 2, 8>();
         case 4: return shape == 7 ? sk<4, 128, 22, 2, 8, true>() : shape == 8 ? sk<4, 64, 44, 2, 8, true>() : shape == 4 ? sk<4, 128, 16, 1, 8, true>() : shape == 3 ? sk<4, 128, 16, 2, 16>() : shape == 2 ? sk<4, 128, 8, 1, 8>() : shape == 1 ? sk<4, 64, 32, 2, 8>() : sk<4, 128, 16, 2, 8>();
         default: return {nullptr, nullptr, 0, 0, 0, 0};
@@ -172,29 +172,34 @@ bool stream3d_supported(const Geom &g) {
 
 namespace {
 
-// Persistent sweeps at R >= 3, which are issue-bound: the shape whose busiest
-// CTA takes least time over its planes, at the time of a plane measured for
-// each (us on one CTA per SM, a chunk's 2R halo planes counting as four; within
-// 5 % over 256^3 to 768^3), and by 3 % or more.  Two rows per
-// thread share their y-neighbours' loads and keep two chains of sums in
-// flight, so a row costs 20 % less than with one, but the taller tiles fill
-// small or odd grids worse.  GB300, us a sweep, 128 x 16 / two rows 128 wide /
-// two rows 64 wide: R = 3 64^3 4.7 / 5.6 / 5.3, 128^3 7.0 / 7.7 / 8.1, 300^3
-// 58.0 / 45.4 / 40.9, 512^3 215.7 / 178.4 / 181.3, 768^3 694 / 583 / 594; R = 4
-// 64^3 5.2 / 5.4 / 4.9, 128^3 7.3 / 6.9 / 7.1, 300^3 61.1 / 57.6 / 50.9, 512^3
-// 223.4 / 211.5 / 211.7, 768^3 735 / 640 / 668, 600 x 64 x 600 45.1 / 42.4 /
-// 53.6.
+// Persistent sweeps at R >= 3, and at R = 2 below 2^25 cells, which are
+// issue-bound: the shape whose busiest CTA takes least time over its planes, at
+// the time of a plane measured for each (us on one CTA per SM, a chunk's 2R halo
+// planes counting as four; within 5 % over 256^3 to 768^3), and by 3 % or more;
+// grids beyond the L2 take the 5.1 TB/s (R = 2; else 6.0) that they reach.  Two
+// rows per thread share their y-neighbours' loads and keep two chains of sums
+// in flight, so at R >= 3 a row costs 20 % less than with one, but the taller
+// tiles fill small or odd grids worse.  GB300, us a sweep, 128 x 16 / two rows
+// 128 wide / two rows 64 wide: R = 3 64^3 4.7 / 5.6 / 5.3, 128^3 7.0 / 7.7 / 8.1,
+// 300^3 58.0 / 45.4 / 40.9, 512^3 215.7 / 178.4 / 181.3, 768^3 694 / 583 / 594; R
+// = 4 64^3 5.2 / 5.4 / 4.9, 128^3 7.3 / 6.9 / 7.1, 300^3 61.1 / 57.6 / 50.9,
+// 512^3 223.4 / 211.5 / 211.7, 768^3 735 / 640 / 668, 600 x 64 x 600 45.1 / 42.4
+// / 53.6.  R = 2, 128 x 32 / 64 x 60: 64 x 317 x 282 17.7 / 12.0, 56 x 111 x 315
+// 11.1 / 7.7, 140 x 361 x 511 57.8 / 50.7, 160^3 10.7 / 10.0, 300^3 42.8 / 43.2.
 int wide_shape(const Geom &g, int ctas) {
-    static const struct { int shape; double plane_us[2]; } kShapes[3] = {
-        {4, {0.458, 0.48}}, {7, {0.672, 0.59}}, {8, {0.685, 0.59}}};
-    int best = 4;
+    static const struct { int shape[3]; double plane_us[3]; } kShapes[3] = {
+        {{5, 4, 4}, {0.60, 0.458, 0.48}}, {{0, 7, 7}, {0, 0.672, 0.59}}, {{8, 8, 8}, {0.60, 0.685, 0.59}}};
+    const int at = g.radius - 2;
+    const double bytes = 8.0 * g.sz * g.nz, memory_us = bytes > 129e6 ? bytes / (at ? 6.0e6 : 5.1e6) : 0;
+    int best = 0;
     double least = 1e300;
     for (const auto &c : kShapes) {
-        const StreamKernel k = pick(g.radius, c.shape);
+        if (!c.shape[at]) continue;
+        const StreamKernel k = pick(g.radius, c.shape[at]);
         int tiles_x, tiles_y, zchunk, items;
         stream3d_plan(g, k.tx, k.ty, ctas, &tiles_x, &tiles_y, &zchunk, &items);
-        const double us = (double)((items + ctas - 1) / ctas) * (zchunk + 4) * c.plane_us[g.radius - 3];
-        if (us < 0.97 * least) { least = us; best = c.shape; }
+        const double us = std::max(memory_us, (double)((items + ctas - 1) / ctas) * (zchunk + 4) * c.plane_us[at]);
+        if (us < 0.97 * least) { least = us; best = c.shape[at]; }
     }
     return best;
 }
@@ -220,7 +225,7 @@ int stream_shape(const Geom &g, int tile_x, int tile_y, int shape_hint, bool per
     // shared-memory reads win: 525 vs 605 at 256^3, 258 vs 301 at 128^3).
     const bool big = (long long)g.nx * g.ny * g.nz >= (1LL << 25);
     if (persistent && !(shape_hint >= 1 && shape_hint <= 6))
-        shape = R == 1 ? 3 : (R == 2 ? (big ? 6 : 5) : wide_shape(g, ctas));
+        shape = R == 1 ? 3 : (R == 2 && big ? 6 : wide_shape(g, ctas));
     return shape;
 }
 
