@@ -112,9 +112,11 @@ STENCIL_API int stencil_params_check(const stencil_params *p);
  * Runs asynchronously on `stream` and writes to *d_result (if non-NULL) which
  * of d_u1 / d_u2 holds the state after the last sweep.  Allocates nothing,
  * except that the 2-D temporally blocked engine (COOP or AUTO on small 2-D
- * grids) keeps a per-device exchange buffer, grown on first use (outside a
- * CUDA graph capture: run such a dispatch once before capturing it) and freed
- * by stencil_release().
+ * grids) keeps exchange buffers, one for each of up to 16 launches in flight,
+ * made on first use (outside a CUDA graph capture: run such a dispatch once
+ * before capturing it) and freed by stencil_release().  A captured launch's
+ * buffer, and the grid-barrier counter of any persistent launch, belong to the
+ * graph until it and its executables are destroyed.
  * Both buffers must be 16-byte aligned (cudaMalloc gives 256). */
 STENCIL_API int stencil_dispatch_ex(const stencil_params *p, float *d_u1, float *d_u2,
                         stencil_stream_t stream, float **d_result);

@@ -342,8 +342,9 @@ int stencil_dispatch_ex(const stencil_params *p, float *d_u1, float *d_u2,
         float *res = nullptr;
         rc = run_tb2d(g, cur, nxt, p->iterations, p->temporal,
                       p->block_x * std::max(p->coarsen_x, 1), p->block_y, s, &res);
-        // its exchange buffer cannot be made inside a graph capture: rows that
-        // are not 16-byte aligned go to the rows kernel then, which needs none
+        // a graph capture of a grid larger than any swept before is refused (its
+        // exchange buffer is allocated outside): rows that are not 16-byte
+        // aligned go to the rows kernel then, which needs none
         if (rc != STENCIL_EUNSUPPORTED || !rows2d_any_supported(g, 2)) {
             if (rc) return rc;
             if (d_result) *d_result = res;
@@ -670,7 +671,7 @@ int stencil_device_status(int *status) {
 }
 
 int stencil_release(void) {
-    tb2d_release();
+    release_slots();
     std::lock_guard<std::mutex> lock(g_ws_mu);
     const int dev = current_device();
     if (dev < 0 || dev >= 64) return STENCIL_OK;

@@ -68,17 +68,30 @@ void stream3d_plan(const Geom &g, int tx, int ty, int resident, int *tiles_x, in
                    int *zchunk, int *items);
 int run_tb3d(const Geom &g, float *a, float *b, int iters, int temporal, cudaStream_t s,
              float **res);
-// A zeroed grid-barrier counter for one persistent launch on stream s
-// (round-robin over a fixed device array; k_stream.cu).
-int grid_bar_slot(cudaStream_t s, unsigned **slot);
+// Zeroed device memory of one persistent launch on stream s, the launch's own
+// until it has ended or, captured, as long as its graph lives
+// (launch_slots.cu): a grid-barrier counter or the 2-D engine's exchange
+// buffer.  Made on the stack before the launch; its destructor marks the
+// launch's end, so it goes out of scope after the launch is enqueued.
+// release_slots frees what the current device's pools hold.
+struct LaunchSlot {
+    void *pool = nullptr, *slot = nullptr;
+    cudaStream_t stream = nullptr;
+    LaunchSlot() = default;
+    LaunchSlot(const LaunchSlot &) = delete;
+    LaunchSlot &operator=(const LaunchSlot &) = delete;
+    ~LaunchSlot();
+    void *mem() const;
+};
+int take_barrier(cudaStream_t s, LaunchSlot *slot);
+int take_exchange(cudaStream_t s, size_t bytes, LaunchSlot *slot);
+void release_slots();
 // Small 2-D grids: all sweeps in one cooperative launch, one tile per CTA,
 // `temporal` sweeps per exchange through global memory (k_tb2d.cu).
-// tile_x/tile_y/temporal 0 = chosen by the library.  tb2d_release frees the
-// current device's exchange buffers.
+// tile_x/tile_y/temporal 0 = chosen by the library.
 bool tb2d_supported(const Geom &g, int dims);
 int run_tb2d(const Geom &g, float *a, float *b, int iters, int temporal, int tile_x, int tile_y,
              cudaStream_t s, float **res);
-void tb2d_release();
 // Larger 2-D grids: all sweeps in one cooperative launch, a grid-wide barrier
 // between sweeps, register-queue columns (k_rows2d.cu).
 // max_ctas > 0 caps the CTAs of the launch; rows2d_capacity = the CTAs of the

@@ -951,19 +951,10 @@ int plan_phases(BatchPlan *plan) {
             c.clear();
         }
     if (!alone.queue[0].empty()) plan->phases.push_back(alone);
-    // A phase's launches take consecutive grid-barrier counters (a ring of
-    // 256): at most 128 jobs per phase keeps the counters of lanes running at
-    // once distinct.
-    constexpr size_t kPhaseJobs = 128;
-    std::vector<std::vector<int>> parts;
+    bool shared = false;
     for (auto &c : byclass) {
         if (c.empty()) continue;
         std::stable_sort(c.begin(), c.end(), [&](int x, int y) { return work(x) > work(y); });
-        for (size_t k = 0; k < c.size(); k += kPhaseJobs)
-            parts.emplace_back(c.begin() + k, c.begin() + std::min(c.size(), k + kPhaseJobs));
-    }
-    bool shared = false;
-    for (auto &c : parts) {
         const StreamedJob &j0 = plan->streamed[c[0]];
         const int nl = std::min<int>(j0.dims == 2 ? lanes2 : lanes, (int)c.size());
         int ctas = 0;

@@ -311,9 +311,10 @@ int run_ragged3d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, f
     if (resident < 1) return fail(STENCIL_EUNSUPPORTED, "ragged stream kernel does not fit on an SM");
     int tiles_x = 0, tiles_y = 0, zchunk = 0, items = 0;
     stream3d_plan(g, k.tx, k.ty, resident, &tiles_x, &tiles_y, &zchunk, &items);
-    unsigned *bar = nullptr;
-    rc = grid_bar_slot(s, &bar);
+    LaunchSlot slot;
+    rc = take_barrier(s, &slot);
     if (rc) return rc;
+    unsigned *bar = static_cast<unsigned *>(slot.mem());
     Geom gg = g;
     int sw = iters;
     void *args[] = {&a, &b, &gg, &tiles_x, &tiles_y, &zchunk, &items, &sw, &bar};

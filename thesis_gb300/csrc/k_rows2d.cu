@@ -168,9 +168,10 @@ int run_rows2d_any(const Geom &g, float *a, float *b, int iters, cudaStream_t s,
     hb = std::min(hb, rows);
     int nblk = (rows + hb - 1) / hb;
     const int grid = (int)std::min<long long>(ctas, ((long long)cols * nblk + kRowsThreads - 1) / kRowsThreads);
-    unsigned *bar = nullptr;
-    int rc = grid_bar_slot(s, &bar);
+    LaunchSlot slot;
+    int rc = take_barrier(s, &slot);
     if (rc) return rc;
+    unsigned *bar = static_cast<unsigned *>(slot.mem());
     Geom gg = g;
     int n = iters;
     void *args[] = {&a, &b, &gg, &hb, &nblk, &n, &bar};
@@ -192,9 +193,10 @@ int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, flo
     rows2d_plan(g, (long long)ctas * kRowsThreads, &hb, &nblk);
     const int items = nch * nblk;
     const int grid = (int)std::max<long long>(1, std::min<long long>(ctas, (items + kRowsThreads - 1) / kRowsThreads));
-    unsigned *bar = nullptr;
-    int rc = grid_bar_slot(s, &bar);
+    LaunchSlot slot;
+    int rc = take_barrier(s, &slot);
     if (rc) return rc;
+    unsigned *bar = static_cast<unsigned *>(slot.mem());
     Geom gg = g;
     int hb_ = hb, nb_ = nblk, n = iters;
     void *args[] = {&a, &b, &gg, &hb_, &nb_, &n, &bar};

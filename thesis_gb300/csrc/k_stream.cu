@@ -28,7 +28,6 @@
 // sequence number fixes each plane's slot and mbarrier phase.  No CTA-wide
 // barrier is used after set-up, and every mbarrier wait is bounded.
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 #include <vector>
 #include <cmath>
@@ -117,25 +116,6 @@ StreamKernel pick(int r, int shape) {
         default: return {nullptr, nullptr, 0, 0, 0, 0};
     }
 }
-
-}  // namespace
-
-// Grid-barrier counters of the persistent launches: a fixed device array (no
-// allocation, so a launch can be captured in a CUDA graph), one slot per
-// launch taken round-robin and zeroed on the launch's stream just before it.
-constexpr int kGridBarSlots = 256;
-__device__ unsigned g_grid_bar[kGridBarSlots];
-
-int grid_bar_slot(cudaStream_t s, unsigned **slot) {
-    static std::atomic<unsigned> next{0};
-    unsigned *base = nullptr;
-    ST_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&base), g_grid_bar));
-    *slot = base + (next.fetch_add(1) % kGridBarSlots);
-    ST_CUDA(cudaMemsetAsync(*slot, 0, sizeof(unsigned), s));
-    return STENCIL_OK;
-}
-
-namespace {
 
 // Sets the kernel's shared-memory limit and returns its resident CTAs per SM,
 // once per kernel and device (later calls, e.g. inside a CUDA graph capture,
@@ -314,9 +294,10 @@ int run_stream3d(const Geom &g, float *a, float *b, int iters, int tile_x, int t
         // One cooperative launch (every CTA resident, as the grid barrier
         // needs): sweep k reads maps[k & 1] and writes the other buffer.
         if (iters > 0) {
-            unsigned *bar = nullptr;
-            rc = grid_bar_slot(s, &bar);
+            LaunchSlot slot;
+            rc = take_barrier(s, &slot);
             if (rc) return rc;
+            unsigned *bar = static_cast<unsigned *>(slot.mem());
             float *d0 = b, *d1 = a;
             int sw = iters;
             void *args[] = {&maps[0], &maps[1], &d0, &d1, &gg, &tx_, &ty_, &zchunk, &it_, &sw, &bar};

@@ -36,7 +36,6 @@
 // over every SM and exchanging once per T sweeps is what makes it fast (one
 // cluster of 16 SMs is issue-bound on the same grid).
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -746,43 +745,6 @@ bool choose_plan(const Geom &g, int iters, int temporal, int tile_x, int tile_y,
     return found;
 }
 
-// Exchange buffers: per device a few slots taken round-robin (so launches on
-// different streams do not share one), all grown together outside any graph
-// capture and zeroed on the launch's stream just before each launch.
-constexpr int kTb2XchSlots = 4;
-struct XchPool {
-    unsigned long long *buf[kTb2XchSlots] = {};
-    size_t bytes = 0;
-    unsigned next = 0;
-};
-std::mutex g_xch_mu;
-XchPool g_xch[64];
-
-int xch_slot(cudaStream_t s, size_t bytes, unsigned long long **out) {
-    const int dev = current_device();
-    if (dev < 0 || dev >= 64) return fail(STENCIL_ECUDA, "no current device");
-    std::lock_guard<std::mutex> lock(g_xch_mu);
-    XchPool &pool = g_xch[dev];
-    if (pool.bytes < bytes) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        ST_CUDA(cudaStreamIsCapturing(s, &cs));
-        if (cs != cudaStreamCaptureStatusNone)
-            return fail(STENCIL_EUNSUPPORTED,
-                        "2-D temporal blocking: run the dispatch once outside the graph capture "
-                        "(its exchange buffer is allocated then)");
-        for (auto &b : pool.buf) {
-            cudaFree(b);  // waits for the device
-            b = nullptr;
-        }
-        pool.bytes = 0;
-        for (auto &b : pool.buf) ST_CUDA(cudaMalloc(reinterpret_cast<void **>(&b), bytes));
-        pool.bytes = bytes;
-    }
-    *out = pool.buf[pool.next++ % kTb2XchSlots];
-    ST_CUDA(cudaMemsetAsync(*out, 0, bytes, s));
-    return STENCIL_OK;
-}
-
 // CTAs of the launch that can be resident at once (one per SM), checked once
 // per radius and device with the largest shared-memory size the plans use
 // (which is also set as each kernel's dynamic shared-memory limit).
@@ -826,17 +788,6 @@ int tb2_max_ctas(int r) {
 
 }  // namespace
 
-void tb2d_release() {
-    const int dev = current_device();
-    if (dev < 0 || dev >= 64) return;
-    std::lock_guard<std::mutex> lock(g_xch_mu);
-    for (auto &b : g_xch[dev].buf) {
-        cudaFree(b);
-        b = nullptr;
-    }
-    g_xch[dev].bytes = 0;
-}
-
 bool tb2d_supported(const Geom &g, int dims) {
     if (dims != 2 || g.radius < 1 || g.radius > 4) return false;
     const int ctas = tb2_max_ctas(g.radius);
@@ -864,9 +815,10 @@ int run_tb2d(const Geom &g, float *a, float *b, int iters, int temporal, int til
                             : reinterpret_cast<const void *>(tb2_fn(g.radius, g.legacy != 0, plan_items(p)));
     const int grid = p.tiles_x * p.tiles_y, threads = reg.lw ? reg.threads : kTb2Threads;
     const size_t smem = reg.lw ? (size_t)reg.smem : 2ull * p.pw * p.ph * sizeof(float);
-    unsigned long long *xch = nullptr;
-    int rc = xch_slot(s, 2ull * grid * p.tx * p.ty * sizeof(unsigned long long), &xch);
+    LaunchSlot slot;
+    int rc = take_exchange(s, 2ull * grid * p.tx * p.ty * sizeof(unsigned long long), &slot);
     if (rc) return rc;
+    unsigned long long *xch = static_cast<unsigned long long *>(slot.mem());
     Geom gg = g;
     int n = iters;
     void *args[] = {&a, &b, &gg, &p, &n, &xch};
