@@ -433,7 +433,12 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
             first[i * hrow + tid] = S[i];
             last[i * hrow + tid] = S[RW - R + i];
         }
-        __syncthreads();
+        // The warps of a CTA that has rows outside the grid meet here from two
+        // instantiations.  PTX barriers are met by number, each warp at its own
+        // instruction; __syncthreads() is not allowed where warps differ.  (GB300,
+        // 256^2 0.311 us a sweep; one barrier before the branch 0.316, one branch
+        // for the CTA 0.334.)
+        asm volatile("barrier.sync.aligned 1;" ::: "memory");
         float4 up[R], dn[R];  // rows -R .. -1 and RW .. RW+R-1
 #pragma unroll
         for (int i = 0; i < R; ++i) {
