@@ -209,7 +209,7 @@ STENCIL_API int stencil_batch_prepare(const stencil_batch_job *jobs, int njobs, 
  * ragged jobs in (one kernel), one
  * persistent cluster launch over a device work queue (every cluster the
  * device can hold) for the jobs that a cluster sweeps (on clusters of one CTA,
- * before it, a launch for the 2-D JACOBI grids of R = 1 with at most 133 rows
+ * beside it, a launch for the 2-D JACOBI grids of R = 1 with at most 133 rows
  * of up to 128 cells or 265 of up to 64, each in the registers of one CTA),
  * then, for each job too
  * large for a cluster's shared memory, one persistent launch of its own, and

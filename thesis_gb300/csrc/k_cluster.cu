@@ -745,6 +745,7 @@ struct BatchHeader {
     int cluster_size;
     int clusters;
     int reg_jobs;        // of the njobs, the last ones: grids of k_reg2d
+    int reg_first;       // k_reg2d's launch comes before k_cluster's
     unsigned reg_queue;
 };
 
@@ -822,7 +823,7 @@ __global__ void __launch_bounds__(kStageThreads)
 // one prepared workspace: mid-size 3-D jobs run side by side, one lane on
 // the caller's stream and the others here, each lane a queue of jobs on its
 // share of the CTAs the device holds (a whole-GPU launch of one of them is
-// latency-bound).
+// latency-bound); so do k_reg2d and k_cluster.
 constexpr int kLanes = 8;
 struct Lanes {
     cudaStream_t s[kLanes - 1] = {};
@@ -847,7 +848,7 @@ struct BatchPlan {
     // n queues side by side, each job with at most `ctas` CTAs
     struct Phase { int ctas; std::vector<std::vector<int>> queue; };
     std::vector<Phase> phases;
-    std::shared_ptr<Lanes> lanes;     // set when some phase has two lanes or more
+    std::shared_ptr<Lanes> lanes;     // set where launches run side by side
 };
 
 // Launch plan of each prepared workspace (set by prepare, read by launch).
@@ -920,6 +921,18 @@ bool stream_job(const StreamedJob &j) {
 
 long long job_cells(const StreamedJob &j) { return (long long)j.g.nx * j.g.ny * j.g.nz; }
 
+int make_lanes(BatchPlan *plan) {
+    if (plan->lanes) return STENCIL_OK;
+    auto ln = std::make_shared<Lanes>();
+    ST_CUDA(cudaEventCreateWithFlags(&ln->fork, cudaEventDisableTiming));
+    for (int k = 0; k < kLanes - 1; ++k) {
+        ST_CUDA(cudaStreamCreateWithFlags(&ln->s[k], cudaStreamNonBlocking));
+        ST_CUDA(cudaEventCreateWithFlags(&ln->join[k], cudaEventDisableTiming));
+    }
+    plan->lanes = ln;
+    return STENCIL_OK;
+}
+
 // Orders the whole-GPU jobs into phases.  First every job that runs alone,
 // in the given order; then, per kernel (radius, arithmetic, shape class: the
 // grids' CTAs are then interchangeable on an SM, so all lanes' CTAs fit on
@@ -990,16 +1003,7 @@ int plan_phases(BatchPlan *plan) {
         plan->phases.push_back(ph);
         shared = true;
     }
-    if (shared) {
-        auto ln = std::make_shared<Lanes>();
-        ST_CUDA(cudaEventCreateWithFlags(&ln->fork, cudaEventDisableTiming));
-        for (int k = 0; k < kLanes - 1; ++k) {
-            ST_CUDA(cudaStreamCreateWithFlags(&ln->s[k], cudaStreamNonBlocking));
-            ST_CUDA(cudaEventCreateWithFlags(&ln->join[k], cudaEventDisableTiming));
-        }
-        plan->lanes = ln;
-    }
-    return STENCIL_OK;
+    return shared ? make_lanes(plan) : STENCIL_OK;
 }
 
 // One whole-GPU job on stream s.
@@ -1218,7 +1222,14 @@ extern "C" int stencil_batch_prepare_engine(const stencil_batch_job *jobs, int n
     for (int i = 0; i < nc; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work[x] > work[y]; });
     // On clusters of one CTA the small 2-D grids go to k_reg2d, a launch of
-    // its own, last in the table.
+    // its own, last in the table.  It runs beside k_cluster's: both take grids
+    // from queues, one CTA on an SM, so whatever SMs one leaves the other
+    // fills.  First comes the launch with the longest single grid (a CTA of
+    // k_reg2d sweeps about five times the cells of k_cluster's), which would end
+    // last.  GB300, milliseconds, every grid in the cluster launch / the two in a
+    // row / side by side: 40 + 40 3-D grids 23.7 / 26.0 / 23.7, 4 long ones
+    // + 300 2-D of R = 2 46.5 / 15.8 / 10.2, 600 + one long R = 2 18.7 / 18.3 / 14.1,
+    // 152 + 152 9.4 / 5.86 / 5.85.
     auto in_regs = [&](int i) { return csize == 1 && reg2d_takes(table[i]); };
     const auto reg0 = std::stable_partition(order.begin(), order.end(), [&](int i) { return !in_regs(i); });
     std::vector<ClusterJob> sorted(nc);
@@ -1227,6 +1238,12 @@ extern "C" int stencil_batch_prepare_engine(const stencil_batch_job *jobs, int n
     h.queue = 0;
     h.reg_queue = 0;
     h.reg_jobs = (int)(order.end() - reg0);
+    const double longest = reg0 == order.begin() ? 0.0 : work[order.front()];
+    h.reg_first = h.reg_jobs && work[*reg0] > 5.0 * longest;
+    if (h.reg_jobs && h.reg_jobs < nc) {
+        int rc = make_lanes(&plan);
+        if (rc) return rc;
+    }
     h.njobs = nc;
     h.cluster_size = csize;
     h.clusters = max_active_clusters(csize);
@@ -1262,16 +1279,29 @@ extern "C" int stencil_batch_launch(const void *d_workspace, stencil_stream_t st
         const ClusterJob *table = reinterpret_cast<const ClusterJob *>(static_cast<const char *>(d_workspace) + hb);
         BatchHeader *dh = reinterpret_cast<BatchHeader *>(const_cast<void *>(d_workspace));
         const int nc = h.njobs - h.reg_jobs;
-        if (h.reg_jobs) {
-            ST_CUDA(cudaMemsetAsync(&dh->reg_queue, 0, sizeof(unsigned), s));
-            k_reg2d<<<std::min(h.reg_jobs, num_sms()), kRegThreads, kRegSmem, s>>>(table + nc, h.reg_jobs,
-                                                                                      &dh->reg_queue);
-            ST_CUDA(cudaGetLastError());
+        auto regs = [&](cudaStream_t on) -> int {
+            ST_CUDA(cudaMemsetAsync(&dh->reg_queue, 0, sizeof(unsigned), on));
+            k_reg2d<<<std::min(h.reg_jobs, num_sms()), kRegThreads, kRegSmem, on>>>(table + nc, h.reg_jobs,
+                                                                                       &dh->reg_queue);
+            return cuda_fail(cudaGetLastError(), "batch launch");
+        };
+        auto clusters = [&](cudaStream_t on) {
+            return launch_cluster_jobs(table, nc, &dh->queue, std::min(h.clusters, nc), h.cluster_size, on);
+        };
+        int rc = STENCIL_OK;
+        if (h.reg_jobs && nc) {
+            const Lanes &ln = *plan.lanes;
+            ST_CUDA(cudaEventRecord(ln.fork, s));
+            ST_CUDA(cudaStreamWaitEvent(ln.s[0], ln.fork, 0));
+            rc = h.reg_first ? regs(s) : clusters(s);
+            if (!rc) rc = h.reg_first ? clusters(ln.s[0]) : regs(ln.s[0]);
+            // joined even after a failure, so that a capture stays well formed
+            ST_CUDA(cudaEventRecord(ln.join[0], ln.s[0]));
+            ST_CUDA(cudaStreamWaitEvent(s, ln.join[0], 0));
+        } else {
+            rc = nc ? clusters(s) : regs(s);
         }
-        if (nc) {
-            int rc = launch_cluster_jobs(table, nc, &dh->queue, std::min(h.clusters, nc), h.cluster_size, s);
-            if (rc) return rc;
-        }
+        if (rc) return rc;
     }
     for (const BatchPlan::Phase &ph : plan.phases) {
         if (ph.queue.size() == 1) {

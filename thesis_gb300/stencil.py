@@ -303,8 +303,8 @@ class Batch:
 
     def kernel_launches(self):
         """Kernel launches of one ``launch`` (one replay of its CUDA graph):
-        1 for the one-launch engine; for the phased one the cluster launch,
-        one per whole-GPU job, and the two copy kernels of jobs whose nx is
+        1 for the one-launch engine; for the phased one the cluster launch
+        (on clusters of one CTA, one more for small 2-D grids), one per whole-GPU job, and the two copy kernels of jobs whose nx is
         not a multiple of 4."""
         n = ctypes.c_int()
         _lib.check(_lib.load().stencil_batch_launches(self.ws, ctypes.byref(n)), "stencil_batch_launches")
