@@ -243,20 +243,25 @@ static int choose_variant(const stencil_params &p) {
     if (p.dims == 2 && p.iterations >= 8 &&
         (tb2d_supported(g, 2) || rows2d_supported(g, 2) || rows2d_any_supported(g, 2)))
         return STENCIL_VARIANT_COOP;
-    // 3-D grids whose planes one cluster of 16 CTAs sweeps faster than the
-    // streaming sweeps over every SM, which take 3.7 (R = 1), 4.5 (R = 2, 3) or
-    // 4.7 us (R = 4) up to about 2^18 cells; the cluster's sweep goes with the
-    // cells of its busiest CTA.  GB300, us a sweep, cells (cluster): R = 1 32^3
-    // 2048 (1.83), 40^3 4800 (2.13), 48^3 6912 (3.94), 9 x 100^2 10000 (5.07);
-    // R = 2 40^3 (2.71), 48^3 (4.21), 32 x 64^2 8192 (4.73); R = 4 32^3 (2.40),
-    // 48^3 (4.05), 52^3 8112 (6.84).  Rows of more than 128 cells: 20 x 20 x 200
-    // R = 3 4.91 cluster, 4.73 streaming.
+    // Grids that one cluster of 16 CTAs holds in shared memory: alone, the
+    // streaming sweeps over every SM are faster for the largest of the 3-D ones
+    // (64^3 R = 1 3.80 us a sweep, 4.88 on a cluster; 56^3 R = 2 4.69 / 5.43), but
+    // nine clusters run side by side where one such launch takes the whole GPU:
+    // from two streams on the cluster is ahead (64^3 R = 1, us a sweep and grid on
+    // 2 / 4 / 8 streams: 2.44 / 1.23 / 0.76, streaming 3.71 / 3.71 / 3.71).
+    if (p.iterations >= 8 && cluster_resident(g, p.dims)) return STENCIL_VARIANT_CLUSTER;
+    // Other 3-D grids whose planes one cluster sweeps faster from the L2 than the
+    // streaming sweeps, which take 3.7 (R = 1), 4.5 (R = 2, 3) or 4.7 us (R = 4)
+    // up to about 2^18 cells; the cluster's sweep goes with the cells of its
+    // busiest CTA.  GB300, us a sweep, cells (cluster): R = 2 40^3 4800 (2.71), 32
+    // x 64^2 8192 (4.73); R = 4 32^3 2048 (2.40), 48^3 6912 (4.05), 52^3 8112
+    // (6.84).  Rows of more than 128 cells: 20 x 20 x 200 R = 3 4.91 cluster, 4.73
+    // streaming.
     if (p.dims == 3 && p.iterations >= 8 && stream3d_supported(g)) {
         const long long busiest = (long long)(g.nz - 2 * g.radius + 15) / 16 * g.nx * g.ny;
-        return cluster_shape_ok(3, (int)g.sy, g.ny, g.radius) && g.nx <= 128 && busiest <= (g.radius == 1 ? 6500 : 7000)
-                   ? STENCIL_VARIANT_CLUSTER : STENCIL_VARIANT_SMEM_REGISTER;
+        if (cluster_shape_ok(3, (int)g.sy, g.ny, g.radius) && g.nx <= 128 && busiest <= (g.radius == 1 ? 6500 : 7000))
+            return STENCIL_VARIANT_CLUSTER;
     }
-    if (p.iterations >= 8 && cluster_resident(g, p.dims)) return STENCIL_VARIANT_CLUSTER;
     if (p.dims == 3 && stream3d_supported(g)) return STENCIL_VARIANT_SMEM_REGISTER;
     return STENCIL_VARIANT_BASE;
 }
