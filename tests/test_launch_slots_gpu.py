@@ -89,15 +89,17 @@ def test_a_long_launch_beside_hundreds_of_short_ones(cuda):
     """The long launch's barrier counter is nobody else's while it runs."""
     import torch
     from thesis_gb300 import stencil as S
-    u, a, b = grid((33, 61, 57), 1)
-    v, c, d = grid((12, 13, 14), 2)
+    u, a, b = grid((33, 61, 57), 1)  # both persistent
+    v, c, d = grid((45, 46, 47), 2)
     s, t = torch.cuda.Stream(), torch.cuda.Stream()
     torch.cuda.synchronize()
     with torch.cuda.stream(s):
         S.sweep(a, b, 1, 4000, stream=s)
+    assert S.last_dispatch() == ("ragged3d-persistent", 1)
     for _ in range(700):
         with torch.cuda.stream(t):
             S.sweep(c, d, 1, 4, stream=t)
+    assert S.last_dispatch() == ("ragged3d-persistent", 1)
     torch.cuda.synchronize()
     assert bits_equal(a.cpu().numpy(), oracle_pair(u, u, 1, 4000, O.JACOBI)[0])
     assert bits_equal(c.cpu().numpy(), oracle_pair(v, v, 1, 2800, O.JACOBI)[0])
@@ -109,7 +111,7 @@ def test_threads_on_shared_streams(cuda):
     import torch
     from thesis_gb300 import stencil as S
     streams = [torch.cuda.Stream() for _ in range(2)]
-    work = [[grid(shape, 20 + k) for shape in ((66, 71), (130, 128), (21, 35, 33))] for k in range(4)]
+    work = [[grid(shape, 20 + k) for shape in ((66, 71), (130, 128), (45, 46, 47))] for k in range(4)]
     torch.cuda.synchronize()
     errors = []
 

@@ -426,11 +426,11 @@ int stencil_dispatch_ex(const stencil_params *p, float *d_u1, float *d_u2,
         return STENCIL_OK;
     }
     if (auto_pick && ragged3d_supported(g, p->dims) &&
-        (p->iterations >= 4 || cell_count(*p) >= (1LL << 22))) {
+        ((p->iterations >= 4 && cell_count(*p) >= ragged3d_least_cells(p->radius)) || cell_count(*p) >= (1LL << 22))) {
         // 3-D rows that are not 16-byte aligned, left to the library; a few
         // sweeps of a small grid are launched one by one (the persistent
         // launch costs about 6 us more: 101 x 99 x 97 R = 2, one sweep 25 us
-        // against 19, 20 sweeps 8.5 us each against 16).
+        // against 19, 20 sweeps 8.5 us each against 16), as are the smallest.
         float *res = nullptr;
         rc = run_ragged3d(g, cur, nxt, p->iterations, s, &res);
         if (rc) return rc;

@@ -109,6 +109,8 @@ int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, flo
 // 3-D grids whose rows are not 16-byte aligned (nx % 4 != 0, R <= 4): all
 // sweeps in one cooperative launch (k_ragged.cu).
 bool ragged3d_supported(const Geom &g, int dims);
+// Grids of fewer cells are swept faster by a launch per sweep.
+long long ragged3d_least_cells(int radius);
 int run_ragged3d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res);
 // Resident CTAs of a kernel on the whole device; sets its shared-memory limit
 // (k_stream.cu).

@@ -301,6 +301,16 @@ bool ragged3d_supported(const Geom &g, int dims) {
     return dims == 3 && g.nx % 4 != 0 && g.sy == g.nx && g.radius >= 1 && g.radius <= 4;
 }
 
+// A launch per sweep takes 4.2 to 6.3 us a sweep up to about 10^5 cells, the
+// persistent sweeps 5.6 (R = 1), 5.5, 6.4 or 7.4 us (R = 4) as soon as the CTAs
+// have a plane each.  GB300, us a sweep in a call of 8 sweeps, a launch each /
+// persistent: R = 1 37^3 5.95 / 6.20, 45^3 6.47 / 6.22, 61^3 8.45 / 6.21; R = 2
+// 33^3 5.45 / 6.00, 37^3 6.44 / 5.95; R = 3 45^3 6.48 / 7.00, 49^3 8.52 / 7.06; R =
+// 4 33^3 6.45 / 7.98, 17 x 65 x 129 6.49 / 8.25, 61^3 9.72 / 8.09.
+long long ragged3d_least_cells(int radius) {
+    return radius == 1 ? 80000 : radius == 2 ? 45000 : radius == 3 ? 110000 : 150000;
+}
+
 int run_ragged3d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res) {
     if (res) *res = (iters & 1) ? b : a;
     if (iters <= 0) return STENCIL_OK;
