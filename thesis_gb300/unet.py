@@ -151,23 +151,24 @@ class UNet:
             n += -(-P[k].numel() // 128) * 128
         self._flat = {k: torch.zeros(n, device=self.device) for k in ("w", "d", "m", "v")}
         self._flat["wb"] = torch.zeros(n, dtype=torch.bfloat16, device=self.device)
-        self._views = []  # (dict, key, tensor) of every view of a flat tensor
+        self._views = []  # (dict, key, flat tensor's name, byte offset) of every view
         for (P, k), o in zip(tensors, offsets):
             shape, size = P[k].shape, P[k].numel()
             self._flat["w"][o:o + size].copy_(P[k].reshape(-1))
             for flat, key in (("w", k), ("d", "d" + k), ("m", "m" + k), ("v", "v" + k), ("wb", "wb")):
                 if flat != "wb" or (k == "w" and P is not self.head):
                     P[key] = self._flat[flat][o:o + size].view(shape)
-                    self._views.append((P, key, P[key]))
+                    self._views.append((P, key, flat, o * self._flat[flat].element_size()))
         self.head_w, self.head_b = self.head["w"], self.head["b"]
         for name, cin, cout in LAYERS:
             self.params[name]["wt"] = torch.empty((cin, 9, cout), dtype=torch.bfloat16, device=self.device)
         self.sync_bf16()
 
     def _whole(self):
-        """Whether every tensor is still the view made above (a caller may
-        have put its own in the dicts)."""
-        return all(P[key] is t for P, key, t in self._views)
+        """Whether every tensor still lies where the view made above does (a
+        caller may have put others in the dicts or behind them)."""
+        base = {k: t.data_ptr() for k, t in self._flat.items()}
+        return all(P[key].data_ptr() == base[flat] + o for P, key, flat, o in self._views)
 
     def sync_bf16(self, stream=None):
         s = _stream(stream)
