@@ -82,9 +82,9 @@ UNET_API int unet_conv3x3_wgrad_dil(const unet_act *x, const unet_act *dy, float
 UNET_API int unet_wgrad_workspace_bytes(const unet_act *x, const unet_act *dy, size_t *bytes);
 /* The weight gradient on a chosen engine: 1 = tcgen05 (TMEM accumulator,
  * TMA-fed operands; asks for w % 32 == 0 and a 256-byte aligned workspace of
- * unet_wgrad_workspace_bytes, which it no longer uses), 2 = mma.sync, 0 =
- * tcgen05 for any width (workspace may be NULL) where the channels are
- * multiples of 32 and the dilation is below about 20, else mma.sync.
+ * unet_wgrad_workspace_bytes, which it does not use), 2 = mma.sync, 0 =
+ * tcgen05 for any width and dilation (workspace may be NULL) where the
+ * channels are multiples of 32, else mma.sync.
  * Same accumulation contract as unet_conv3x3_wgrad_dil (FP32 atomics). */
 UNET_API int unet_conv3x3_wgrad_engine(const unet_act *x, const unet_act *dy, float *dw, float *db,
                                        int dilation, int engine, void *workspace,

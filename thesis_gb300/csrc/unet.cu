@@ -618,6 +618,8 @@ struct WgradRows {
     int stages;      // steps in flight
     int lag;         // steps between a row's arrival and its last use
     int dslot;       // bytes of a step of dy
+    int march;       // dil: a row serves three output rows; 0: its three rows are loaded with each
+    int xrows;       // rows of x in shared memory
 };
 
 __device__ __forceinline__ uint64_t umma_desc_mn64(uint32_t saddr, uint32_t block_bytes) {
@@ -634,8 +636,9 @@ __global__ void __launch_bounds__(192, 2)
     __shared__ float bsum[4][128];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(wr_smem) + 1023) & ~static_cast<uintptr_t>(1023));
-    const int tile = p.wp * 64, dil = p.dil, rs = p.rs, nst = p.stages, nx = nst + p.lag;
-    unsigned char *xring = base, *dring = base + (size_t)((nx + p.lag) * rs + dil) * tile;
+    const int tile = p.wp * 64, dil = p.dil, rs = p.rs, nst = p.stages, nx = nst + p.lag, march = p.march;
+    const int xstep = march ? rs : 3 * rs, xend = march ? nx * rs : 1 << 30;  // ring rows of a step; where they wrap
+    unsigned char *xring = base, *dring = base + (size_t)p.xrows * tile;
     uint64_t *full = reinterpret_cast<uint64_t *>(dring + (size_t)nst * p.dslot);
     uint64_t *empty = full + nst, *accd = empty + nst;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(accd + 1);
@@ -673,7 +676,9 @@ __global__ void __launch_bounds__(192, 2)
     // stays in one image's column (output rows y0 .. y1 - 1) is one march.
     // Its step g brings input rows y0 - dil + g * rs ... and dy's rows that
     // these complete, y0 - 2 * dil + g * rs ..., of which the ones in the
-    // march are used.
+    // march are used.  Where the rows of one march do not fit shared memory
+    // (wide dilations) a step brings its rs rows of dy and the three times rs
+    // input rows that they meet, one after the other.
     if (warp == 4) {
         const uint32_t on = elect_lane(), xs = smem_u32(xring), ds = smem_u32(dring), fb = smem_u32(full);
         RingPos q;
@@ -682,15 +687,19 @@ __global__ void __launch_bounds__(192, 2)
         for (int r = r0; r < r1 && ok;) {
             const int img = r / p.H, y0 = r - img * p.H, y1 = min(p.H, y0 + (r1 - r));
             const int im = img % p.n, w0 = img / p.n * p.wp, xw = w0 + (shift - 1) * dil;
-            for (int row = y0 - dil; row < y1 + dil; row += rs) {
+            for (int row = y0 - march; row < y1 + march; row += rs) {
                 if (wrap && !warp_wait_bounded(&empty[q.slot], q.parity ^ 1)) { ok = false; break; }
                 if (bias) fence_proxy_async();  // the bias warps' reads of the slot before the TMA write
-                const uint32_t bar = fb + 8 * q.slot;
+                const uint32_t bar = fb + 8 * q.slot, to = xs + xslot * xstep * tile;
                 const bool twice = xslot < p.lag;
-                expect_tx_if(on, bar, p.dslot + (twice ? 2 : 1) * rs * tile);
-                tma_load_4d_if(on, xs + xslot * rs * tile, &xmap, bar, ci0, xw, row, im);
-                tma_load_5d_if(on, ds + q.slot * p.dslot, &gmap, bar, 0, w0, co0 / 32, row - dil, im);
-                if (twice) tma_load_4d_if(on, xs + (nx + xslot) * rs * tile, &xmap, bar, ci0, xw, row, im);
+                expect_tx_if(on, bar, p.dslot + (march ? twice ? 2 : 1 : 3) * rs * tile);
+                tma_load_4d_if(on, to, &xmap, bar, ci0, xw, march ? row : row - dil, im);
+                tma_load_5d_if(on, ds + q.slot * p.dslot, &gmap, bar, 0, w0, co0 / 32, row - march, im);
+                if (!march) {
+                    tma_load_4d_if(on, to + rs * tile, &xmap, bar, ci0, xw, row, im);
+                    tma_load_4d_if(on, to + 2 * rs * tile, &xmap, bar, ci0, xw, row + dil, im);
+                }
+                if (twice) tma_load_4d_if(on, to + nx * rs * tile, &xmap, bar, ci0, xw, row, im);
                 if (++xslot == nx) xslot = 0;
                 q.next(nst);
                 wrap |= q.slot == 0;
@@ -702,7 +711,7 @@ __global__ void __launch_bounds__(192, 2)
         // D FP32, A and B BF16, both MN-major, N = ncols, M = 128
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-        const uint64_t adesc = umma_desc_mn64(smem_u32(xring), dil * tile), bdesc = umma_desc_mn64(smem_u32(dring), tile);
+        const uint64_t adesc = umma_desc_mn64(smem_u32(xring), (march ? dil : rs) * tile), bdesc = umma_desc_mn64(smem_u32(dring), tile);
         const uint32_t astep = tile >> 4, ks = p.wp / 16, on = elect_lane(), fb = smem_u32(empty);
         RingPos q;
         int xslot = 0;
@@ -711,9 +720,10 @@ __global__ void __launch_bounds__(192, 2)
         for (int r = r0; r < r1 && ok;) {
             const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
             int first = xslot * rs;  // ring row of input row y - dil
-            for (int i = -2 * dil; i < np; i += rs) {
+            for (int i = -2 * march; i < np; i += rs) {
                 if (!warp_wait_bounded(&full[q.slot], q.parity)) { ok = false; break; }
                 tc_fence_after();
+                if (!march) first = xslot * xstep;
                 uint64_t b = bdesc + q.slot * (p.dslot >> 4);
                 for (int j = i; j < i + rs; ++j, b += drow >> 4) {
                     if (j < 0 || j >= np) continue;
@@ -723,7 +733,7 @@ __global__ void __launch_bounds__(192, 2)
                         mma_f16_if(on, tmem, a + k * 64, b + k * 64, idesc, acc);
                         acc = 1;
                     }
-                    if (++first == nx * rs) first = 0;
+                    if (++first == xend) first = 0;
                 }
                 tc_commit_if(on, fb + 8 * q.slot);
                 if (++xslot == nx) xslot = 0;
@@ -744,7 +754,7 @@ __global__ void __launch_bounds__(192, 2)
             bool ok = true;
             for (int r = r0; r < r1 && ok;) {
                 const int y0 = r % p.H, np = min(p.H - y0, r1 - r);
-                for (int i = -2 * dil; i < np; i += rs) {
+                for (int i = -2 * march; i < np; i += rs) {
                     if (!warp_wait_bounded(&full[q.slot], q.parity)) { ok = false; break; }
                     for (int j = max(i, 0); j < min(i + rs, np); ++j) {
                         if ((y0 + j) % 3 != shift) continue;
@@ -1588,23 +1598,28 @@ extern "C" int unet_flip_weights(const void *w, void *wt, int cout, int cin, ste
 
 namespace {
 
-// The row-marching weight gradient's plan for a layer; false where the rows
-// of one march do not fit shared memory in segments of 16 pixels (dilations
-// beyond about 20).  Two CTAs share an SM where the rings allow it.
+// The row-marching weight gradient's plan for a layer; false where its channels
+// are not multiples of 32.  Two CTAs share an SM where the rings allow it.
+// Dilations beyond about 20, of which no march fits shared memory in segments
+// of 16 pixels, load their input rows three times (64 x 128^2, 32 -> 32 channels,
+// dilation 32: 86 us; mma.sync 1026; dilation 1, marching, 91).
 constexpr int WR_SMEM = 107 * 1024, WR_SMEM_MAX = 218 * 1024;
 bool wgrad_rows_plan(const unet_act *x, const unet_act *dy, int dil, WgradRows *p) {
     if (x->c % 32 || dy->c % 32 || (long long)x->n * x->h * ((x->w + 15) / 16) >= (1LL << 31)) return false;
     const int nb = std::min(dy->c, 128) / 32;
-    for (int budget : {WR_SMEM, WR_SMEM_MAX})
+    for (int n = 0; n < 4; ++n)
         for (int wp : {128, 64, 32, 16}) {
+            const int budget = n % 2 ? WR_SMEM_MAX : WR_SMEM, march = n < 2 ? dil : 0;
+            if ((long long)march * 128 > WR_SMEM_MAX) continue;
             // the shortest segment that covers a row, else the longest that fits
             if (wp > 16 && wp / 2 >= x->w) continue;
             wp = std::min(wp, (x->w + 15) / 16 * 16);
-            const int rs = std::max(1, 256 / (wp * nb)), tile = wp * 64, lag = (2 * dil + rs - 1) / rs;
-            const int dslot = rs * nb * tile, fixed = (2 * lag * rs + dil) * tile;
-            const int stages = std::min(8, (budget - fixed) / (dslot + rs * tile));
+            const int rs = std::max(1, 256 / (wp * nb)), tile = wp * 64, lag = (2 * march + rs - 1) / rs;
+            const int dslot = rs * nb * tile, fixed = 2 * lag * rs + march, xstep = march ? rs : 3 * rs;
+            const int stages = std::min(8, (budget - fixed * tile) / (dslot + xstep * tile));
             if (stages < 3) continue;
-            *p = {x->c, dy->c, x->n, x->h, x->w, dil, wp, rs, (x->w + wp - 1) / wp * x->n * x->h, 1, stages, lag, dslot};
+            *p = {x->c, dy->c, x->n, x->h, x->w, dil, wp, rs, (x->w + wp - 1) / wp * x->n * x->h, 1, stages, lag, dslot,
+                  march, stages * xstep + fixed};
             // Slices of the rows.  The tensor core truncates: a sum of k
             // steps of 16 pixels ends about 1.5e-8 k below its exact value
             // (measured, positive activations), so few slices cost accuracy
@@ -1649,8 +1664,7 @@ int launch_wgrad_rows(const unet_act *x, const unet_act *dy, float *dw, float *d
     rc = make_tensor_map_general(&gm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, static_cast<const bf16 *>(dy->ptr) + dy->c_off,
                                  gd, gs, gb, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
-    const int xrows = (p.stages + 2 * p.lag) * p.rs + p.dil;
-    const int smem = xrows * p.wp * 64 + p.stages * p.dslot + 1024 + (2 * p.stages + 1) * 8 + 16;
+    const int smem = p.xrows * p.wp * 64 + p.stages * p.dslot + 1024 + (2 * p.stages + 1) * 8 + 16;
     k_wgrad_rows<<<dim3(p.slices, 3 * (p.cin / 32), (p.cout + 127) / 128), 192, smem, s>>>(xm, gm, dw, db, p);
     return cuda_fail(cudaGetLastError(), "wgrad (tcgen05) launch");
 }
@@ -1679,7 +1693,7 @@ extern "C" int unet_conv3x3_wgrad_engine(const unet_act *x, const unet_act *dy, 
                       workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
     if (engine == 1 && !fits)
         return fail(STENCIL_EINVAL, "tcgen05 weight gradient needs W %% 32 == 0 and a %zu-byte workspace", need);
-    // tcgen05 wherever the rows of a march fit shared memory
+    // tcgen05 wherever the channels allow it
     WgradRows p;
     if (engine != 2 && wgrad_rows_plan(x, dy, dilation, &p)) return launch_wgrad_rows(x, dy, dw, db, p, STREAM(s));
     return unet_conv3x3_wgrad_dil(x, dy, dw, db, dilation, s);
