@@ -77,7 +77,7 @@ using RowsFn = void (*)(float *, float *, Geom, int, int, int, unsigned *);
 // chunks), legal because every read of another CTA's writes follows the grid
 // barrier's acquire and a CTA barrier; STENCIL_ROWS_L1=0 (read at each
 // launch) selects ld.global.cg.
-RowsFn rows_fn(int r, bool l1 = false) {
+RowsFn rows_fn(int r, bool l1) {
     switch (r * 2 + (l1 ? 1 : 0)) {
         case 2: return k_rows2d<1, false>;
         case 3: return k_rows2d<1, true>;
@@ -101,23 +101,21 @@ bool rows_l1() {
     return !(e && e[0] == '0');
 }
 
-// Resident CTAs of the radius-r kernel (once per kernel and device).
-int rows_ctas(int r, bool any = false) {
+// Resident CTAs of the kernel that is launched (once per kernel and device).
+int rows_ctas(RowsFn fn) {
     static std::mutex mu;
-    static std::vector<std::pair<int, int>> cache;  // (device * 16 + 8 * any + r, ctas)
+    static std::vector<std::pair<std::pair<RowsFn, int>, int>> cache;
     const int dev = current_device();
     std::lock_guard<std::mutex> lock(mu);
-    const int key = dev * 16 + 8 * any + r;
     for (auto &c : cache)
-        if (c.first == key) return c.second;
+        if (c.first.first == fn && c.first.second == dev) return c.second;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void *>(any ? rows_any_fn(r) : rows_fn(r)),
-                                                      kRowsThreads, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void *>(fn), kRowsThreads, 0) != cudaSuccess) {
         cudaGetLastError();
         n = 0;
     }
     const int ctas = n * num_sms();
-    cache.push_back({key, ctas});
+    cache.push_back({{fn, dev}, ctas});
     return ctas;
 }
 
@@ -125,17 +123,17 @@ int rows_ctas(int r, bool any = false) {
 
 bool rows2d_supported(const Geom &g, int dims) {
     return dims == 2 && g.sy % 4 == 0 && g.radius >= 1 && g.radius <= 4 &&
-           (long long)(g.sy / 4) * (g.ny - 2 * g.radius) < (1LL << 31) && rows_ctas(g.radius) > 0;
+           (long long)(g.sy / 4) * (g.ny - 2 * g.radius) < (1LL << 31) && rows_ctas(rows_fn(g.radius, rows_l1())) > 0;
 }
 
 // Rows that are not 16-byte aligned: fewer than 2^31 (column, row) pairs, and
 // row offsets that the kernel's 64-bit products hold.
 bool rows2d_any_supported(const Geom &g, int dims) {
     return dims == 2 && g.sy % 4 != 0 && g.radius >= 1 && g.radius <= 4 &&
-           (long long)g.nx * g.ny < (1LL << 31) && rows_ctas(g.radius, true) > 0;
+           (long long)g.nx * g.ny < (1LL << 31) && rows_ctas(rows_any_fn(g.radius)) > 0;
 }
 
-int rows2d_capacity(const Geom &g) { return rows_ctas(g.radius); }
+int rows2d_capacity(const Geom &g) { return rows_ctas(rows_fn(g.radius, rows_l1())); }
 
 // Row blocks of a rows sweep of g on `threads` threads: the height, at most
 // 64 rows and at least 4 (R = 1) or 8, that costs the busiest thread the
@@ -162,7 +160,7 @@ void rows2d_plan(const Geom &g, long long threads, int *hb, int *nblk) {
 int run_rows2d_any(const Geom &g, float *a, float *b, int iters, cudaStream_t s, float **res) {
     if (res) *res = (iters & 1) ? b : a;
     if (iters <= 0) return STENCIL_OK;
-    const int ctas = rows_ctas(g.radius, true);
+    const int ctas = rows_ctas(rows_any_fn(g.radius));
     const int cols = g.nx - 2 * g.radius, rows = g.ny - 2 * g.radius;
     int hb = (int)std::min<long long>(64, std::max<long long>(4, (long long)cols * rows / (4LL * ctas * kRowsThreads)));
     hb = std::min(hb, rows);
@@ -187,7 +185,8 @@ int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, flo
         return fail(STENCIL_EUNSUPPORTED, "persistent 2-D rows kernel: row pitch %% 4 == 0, R <= 4");
     if (res) *res = (iters & 1) ? b : a;
     if (iters <= 0) return STENCIL_OK;
-    const int ctas = max_ctas > 0 ? std::min(max_ctas, rows_ctas(g.radius)) : rows_ctas(g.radius);
+    const RowsFn fn = rows_fn(g.radius, rows_l1());
+    const int resident = rows_ctas(fn), ctas = max_ctas > 0 ? std::min(max_ctas, resident) : resident;
     const int nch = (int)(g.sy / 4);
     int hb = 0, nblk = 0;
     rows2d_plan(g, (long long)ctas * kRowsThreads, &hb, &nblk);
@@ -200,8 +199,7 @@ int run_rows2d(const Geom &g, float *a, float *b, int iters, cudaStream_t s, flo
     Geom gg = g;
     int hb_ = hb, nb_ = nblk, n = iters;
     void *args[] = {&a, &b, &gg, &hb_, &nb_, &n, &bar};
-    ST_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(rows_fn(g.radius, rows_l1())), dim3(grid),
-                                        dim3(kRowsThreads), args, 0, s));
+    ST_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fn), dim3(grid), dim3(kRowsThreads), args, 0, s));
     note_launches("rows2d-persistent", 1);
     return STENCIL_OK;
 }
