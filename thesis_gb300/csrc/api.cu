@@ -19,6 +19,7 @@ namespace st {
 int launch_init_uniform(float *u, size_t count, uint64_t seed, cudaStream_t s);
 size_t residual_scratch_bytes();
 int launch_residual(const Geom &g, int dims, const float *u, double *scratch, cudaStream_t s);
+int residual_launches(const Geom &g, int dims);
 bool stream3d_supported(const Geom &g);
 bool tile_supported(const Geom &g, int dims);
 bool tb3d_supported(const Geom &g);
@@ -601,7 +602,7 @@ int stencil_solve(const stencil_params *p, float *d_u1, float *d_u2, double tol,
         if (rc) return rc;
         ++checks;
     }
-    t_launches = launches + 2LL * checks;
+    t_launches = launches + (long long)residual_launches(make_geom(*p), p->dims) * checks;
     result->sweeps = done;
     result->checks = checks;
     result->rel_residual = rel;

@@ -30,6 +30,7 @@ namespace st {
 
 size_t residual_scratch_bytes();
 int launch_residual(const Geom &g, int dims, const float *u, double *scratch, cudaStream_t s);
+int residual_launches(const Geom &g, int dims);
 // The TMA-fed correction sweep for 3-D grids (k_lpstream.cu): eo = M e + rhs
 // over the update region.  eo's border band must hold zeros (at R = 4 the
 // sweep's block stores write them there again); e and rhs are read only.
@@ -423,7 +424,7 @@ int ir_loop(const stencil_params &p, const stencil_ir_params &ir, float *u, char
         if ((ir.tol > 0.0 && (ir.check_every <= 1 || outer % ir.check_every == 0)) || last) {
             int rc = ir_check(g, p.dims, u, resid, s, &rel);
             if (rc) return rc;
-            launches += 2;
+            launches += residual_launches(g, p.dims);
             if (ir.tol > 0.0 && rel < ir.tol) break;
         }
     }

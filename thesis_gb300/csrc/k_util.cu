@@ -363,11 +363,19 @@ int launch_init_uniform(float *u, size_t count, uint64_t seed, cudaStream_t s) {
 // scratch: >= residual_scratch_bytes() of device memory, 8-byte aligned.
 size_t residual_scratch_bytes() { return (2 * kResidBlocks + 2) * sizeof(double); }
 
+// Whether the streaming pass takes the grid.
+static bool residual_streams(const Geom &g, int dims) {
+    return dims == 3 && g.nx % 4 == 0 && g.radius <= 4 && (long long)g.nx * g.ny * g.nz >= kResidStreamCells;
+}
+
+// Kernels of one launch_residual.
+int residual_launches(const Geom &g, int dims) { return residual_streams(g, dims) ? 3 : 2; }
+
 // Stage 1 over `blocks` blocks (any count: rows are handed out round-robin).
 int launch_residual_partial(const Geom &g, int dims, const float *u, double *part, int blocks,
                             cudaStream_t s) {
     const bool vec = g.nx % 4 == 0 && g.radius <= 4;
-    if (vec && dims == 3 && (long long)g.nx * g.ny * g.nz >= kResidStreamCells)
+    if (residual_streams(g, dims))
         switch (g.radius) {
             case 1: return launch_residual_stream<1>(g, u, part, blocks, s);
             case 2: return launch_residual_stream<2>(g, u, part, blocks, s);
