@@ -270,37 +270,63 @@ __global__ void __launch_bounds__(kTb2Threads, 1)
         // Read the halo ring from the neighbours' tiles, waiting for block
         // blk: every pair of a thread is requested before any is checked, and
         // again those that have not arrived, so the wait is that of the
-        // slowest (about two L2 round trips).
+        // slowest (about two L2 round trips).  At R = 3 with eight pairs a
+        // thread that spills (32 bytes): there they are asked for again one by one
+        // (GB300, LEGACY, us a sweep: 1488 x 188 1.63 / 1.76 together, 303 x 1328
+        // 2.02 / 2.15; JACOBI 198 x 1276 1.60 / 1.65, 423 x 616 1.71 / 1.69).
+        constexpr bool ONE_BY_ONE = R == 3 && NI == 4;
         bool ok = true;
         {
             unsigned long long a[NP], b[NP];
             unsigned want = 0;
             uint64_t t0 = 0;
+            auto request = [&](int i) {
+                asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a[i]), "=l"(b[i]) : "l"(slot + ring_w[i]) : "memory");
+            };
+            auto arrived = [&](int i) { return (unsigned)(a[i] >> 32) == blk && (unsigned)(b[i] >> 32) == blk; };
+            auto put = [&](int i) {
+                *reinterpret_cast<float2 *>(Sw + ring_s[i]) =
+                    make_float2(__uint_as_float((unsigned)a[i]), __uint_as_float((unsigned)b[i]));
+            };
+            auto in_time = [&]() {
+                const uint64_t t = globaltimer_ns();
+                if (!t0) t0 = t;
+                else if (t - t0 > kWaitLimitNs) {
+                    report_status(kStatusTimeout);
+                    ok = false;
+                }
+            };
+            if constexpr (ONE_BY_ONE) {
 #pragma unroll
-            for (int i = 0; i < NP; ++i)
-                if (ring_w[i] >= 0) want |= 1u << i;
-            while (want && ok) {
+                for (int i = 0; i < NP; ++i) {
+                    a[i] = b[i] = 0;
+                    if (ring_w[i] >= 0) request(i);
+                }
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    if (ring_w[i] < 0) continue;
+                    t0 = 0;
+                    while (ok && !arrived(i)) {
+                        in_time();
+                        request(i);
+                    }
+                    put(i);
+                }
+            } else {
 #pragma unroll
                 for (int i = 0; i < NP; ++i)
-                    if ((want >> i) & 1u)
-                        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
-                                     : "=l"(a[i]), "=l"(b[i])
-                                     : "l"(slot + ring_w[i])
-                                     : "memory");
+                    if (ring_w[i] >= 0) want |= 1u << i;
+                while (want && ok) {
 #pragma unroll
-                for (int i = 0; i < NP; ++i)
-                    if (((want >> i) & 1u) && (unsigned)(a[i] >> 32) == blk && (unsigned)(b[i] >> 32) == blk) {
-                        want &= ~(1u << i);
-                        *reinterpret_cast<float2 *>(Sw + ring_s[i]) =
-                            make_float2(__uint_as_float((unsigned)a[i]), __uint_as_float((unsigned)b[i]));
-                    }
-                if (want) {
-                    const uint64_t t = globaltimer_ns();
-                    if (!t0) t0 = t;
-                    else if (t - t0 > kWaitLimitNs) {
-                        report_status(kStatusTimeout);
-                        ok = false;
-                    }
+                    for (int i = 0; i < NP; ++i)
+                        if ((want >> i) & 1u) request(i);
+#pragma unroll
+                    for (int i = 0; i < NP; ++i)
+                        if (((want >> i) & 1u) && arrived(i)) {
+                            want &= ~(1u << i);
+                            put(i);
+                        }
+                    if (want) in_time();
                 }
             }
         }
