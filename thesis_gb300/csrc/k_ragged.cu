@@ -4,7 +4,7 @@
 // tensor maps cannot describe).
 //
 // The structure is the stream kernel's (stream_body.cuh): a CTA owns an x-y
-// tile and a chunk of z-planes, one producer warp streams plane tiles with
+// tile and a chunk of z-planes, producer warps stream plane tiles with
 // their halo into a ring of shared-memory slots (full/empty mbarriers), the
 // consumers keep the z-neighbours in a register queue, and between sweeps the
 // CTAs meet at a bounded grid barrier.  What differs:
@@ -21,12 +21,12 @@
 // bound by HBM at R = 1 and by instruction issue at larger radii (about twice
 // the instructions per cell of the stream kernel's 4-cell vectors).  GB300, us
 // per sweep, against a launch per sweep of one thread per cell: 509 x 511 x 510
-// R = 1 194 (1303; the stream kernel's 512^3: 185), 205 x 301 x 253 R = 2 33.4
-// (177), 99 x 505 x 205 R = 3 32.3 (157), 511 x 510 x 509 R = 4 313 (2033), 61^3
-// R = 1 5.6 (7.9).  Packed sums against scalar ones: R = 4 313 / 342, R = 2 33.4 /
-// 35.1; one CTA per SM against two at R = 2 (whose 56 registers spill): 205 x
-// 301 x 253 33.4 / 35.7, 511 x 510 x 509 259 / 249 (with four producer warps 30.9
-// and 230).
+// R = 1 194 (1303; the stream kernel's 512^3: 182), 205 x 301 x 253 R = 2 30.7
+// (177), 99 x 505 x 205 R = 3 32.5 (157), 511 x 510 x 509 R = 4 313 (2033), 61^3
+// R = 1 5.5 (7.9).  With two producer warps at every radius: packed sums
+// against scalar ones R = 4 313 / 342, R = 2 33.4 / 35.1; one CTA per SM against
+// two at R = 2 (whose 56 registers spill) 205 x 301 x 253 33.4 / 35.7, 511 x 510 x
+// 509 259 / 249 (one CTA with four producer warps 30.9 and 230).
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -58,12 +58,11 @@ template <int R, int WX, int M>
 __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R, WX, M>::MIN_BLOCKS)
     k_ragged3d(float *a, float *b, Geom g, int tiles_x, int tiles_y, int zchunk, int items, int sweeps, unsigned *grid_bar) {
     using S = RaggedShape<R, WX, M>;
-    constexpr bool PK = true;  // packed sums of row pairs
     constexpr int C = 6 * R, QN = 2 * R + 1, RY = S::RY, NS = S::NS, PW = S::PW;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float *ring = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + NS * S::SLOT), *empty = full + NS;
-    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int ntiles = tiles_x * tiles_y;
     const long long total = g.sz * g.nz;
     if (tid == 0) {
@@ -82,12 +81,11 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
         // addresses stay in uniform registers (a lane per row made a plane of
         // 20 rows cost 2000 cycles).
         const int wp = warp - S::WARPS;
-        uint32_t on;
-        asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on));
+        const uint32_t on = elect_lane();
         uint32_t q = 0;
         for (int sw = 0; sw < sweeps; ++sw) {
-            // sweep sw reads what every CTA wrote in sweep sw - 1; every lane
-            // issues copies, so every lane acquires
+            // sweep sw reads what every CTA wrote in sweep sw - 1: the elected
+            // lane's acquire and fence (in the wait) come before its copies
             if (sw > 0 && !__all_sync(0xffffffffu, grid_wait_bounded(grid_bar, (unsigned)sw * gridDim.x))) return;
             const float *src = (sw & 1) ? b : a;
             for (int item = blockIdx.x; item < items; item += gridDim.x) {
@@ -99,7 +97,7 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
                 for (int p = 0; p < np; ++p, ++q) {
                     const int s = q & (NS - 1);
                     const uint32_t use = q / NS;
-                    if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (use - 1) & 1))) return;
+                    if (use > 0 && !warp_wait_bounded(&empty[s], (use - 1) & 1)) return;
                     fence_proxy_async();  // the consumers' reads of the slot before the copies
                     const long long plane = (long long)(z0 - R + p) * g.sz;
                     // cell (x, row r) sits at slot + shift + r * PW + x - x0 + R,
@@ -126,11 +124,7 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
                         from += 4ull * S::PW_WARPS * g.nx;
                         to += 4u * S::PW_WARPS * PW;
                     }
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
-                        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
-                        "r"(sum), "r"(on)
-                        : "memory");
+                    expect_tx_if(on, bar, sum);
                 }
             }
         }
@@ -195,7 +189,7 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
                             col[k] = cb[(k - R) * PW];
                         }
                     }
-                    // sums of two rows at a time along x and z (add_pair), started
+                    // sums of two rows at a time along x and z (fadd2), started
                     // from the first term (div_slow_from_first)
                     float2 acc[RY / 2];
 #pragma unroll
@@ -204,12 +198,12 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
                         acc[r] = make_float2(c0r[-R], c1r[-R]);
 #pragma unroll
                         for (int o = -R + 1; o <= R; ++o)
-                            if (o) acc[r] = add_pair<PK>(acc[r], make_float2(c0r[o], c1r[o]));
+                            if (o) acc[r] = fadd2(acc[r], make_float2(c0r[o], c1r[o]));
 #pragma unroll
                         for (int o = -R; o <= R; ++o)
                             if (o) acc[r].x += col[2 * r + R + o], acc[r].y += col[2 * r + 1 + R + o];
 #pragma unroll
-                        for (int o = -R; o <= -1; ++o) acc[r] = add_pair<PK>(acc[r], qz[r][(ph + R + o + QN) % QN]);
+                        for (int o = -R; o <= -1; ++o) acc[r] = fadd2(acc[r], qz[r][(ph + R + o + QN) % QN]);
                     }
                     release(sc);
                     {
@@ -226,7 +220,7 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
 #pragma unroll
                     for (int r = 0; r < RY / 2; ++r)
 #pragma unroll
-                        for (int o = 1; o <= R; ++o) acc[r] = add_pair<PK>(acc[r], qz[r][(ph + R + o) % QN]);
+                        for (int o = 1; o <= R; ++o) acc[r] = fadd2(acc[r], qz[r][(ph + R + o) % QN]);
                     // correctly rounded division by 6R: the fast path where every
                     // stored sum lies in its range, else the warp divides
                     float lo = 0x1p-100f, hi = 0x1p+120f;
@@ -239,7 +233,7 @@ __global__ void __launch_bounds__(RaggedShape<R, WX, M>::THREADS, RaggedShape<R,
                         }
                     if (__all_sync(0xffffffffu, lo >= 0x1p-100f && hi <= 0x1p+120f)) {
 #pragma unroll
-                        for (int r = 0; r < RY / 2; ++r) acc[r] = div_pair<PK, C>(acc[r]);
+                        for (int r = 0; r < RY / 2; ++r) acc[r] = div_fast2<C>(acc[r]);
                     } else {
 #pragma unroll
                         for (int r = 0; r < RY / 2; ++r)
