@@ -178,3 +178,44 @@ def test_graphs_give_their_buffers_back(cuda):
     gc.collect()
     # two slots of 8 bytes a cell each time would be 250 MB
     assert before - torch.cuda.mem_get_info()[0] < 100 << 20
+
+
+def test_launches_in_other_threads_during_a_capture(cuda):
+    """A capture does not stop other threads' calls, nor do they end it."""
+    import ctypes
+    import torch
+    from thesis_gb300 import lib, stencil as S
+    lib.check(lib.load().stencil_release(), "stencil_release")
+    u, a, b = grid((66, 71), 1)
+    S.sweep(a, b, 1, 10)
+    a.copy_(torch.from_numpy(u)), b.copy_(torch.from_numpy(u))
+    other = [grid(shape, 30 + k) for k, shape in enumerate([(301, 304), (401, 399), (45, 46, 47), (90, 91, 92), (66, 71)])]
+    torch.cuda.synchronize()
+    s, g, errors = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+
+    def run():
+        try:
+            t = torch.cuda.Stream()
+            for _, x, y in other[:4]:
+                for _ in range(3):
+                    with torch.cuda.stream(t):
+                        S.sweep(x, y, 1, 10, stream=t)
+            _, x, y = other[4]  # the thread's own default stream
+            p = lib.make_params((66, 71), 1, 30, lib.MODE_JACOBI)
+            lib.check(lib.load().stencil_dispatch_ex(ctypes.byref(p), ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()),
+                                                     ctypes.c_void_p(2), None), "dispatch")
+        except Exception as e:
+            errors.append(e)
+
+    with torch.cuda.graph(g, stream=s):
+        S.sweep(a, b, 1, 10, stream=s)
+        t = threading.Thread(target=run)
+        t.start(), t.join()
+        S.sweep(a, b, 1, 10, stream=s)
+    assert not errors, errors
+    g.replay()
+    torch.cuda.synchronize()
+    assert bits_equal(a.cpu().numpy(), oracle_pair(u, u, 1, 20, O.JACOBI)[0])
+    for v, x, _ in other:
+        assert bits_equal(x.cpu().numpy(), oracle_pair(v, v, 1, 30, O.JACOBI)[0])
+    assert S.device_status() == 0

@@ -49,7 +49,7 @@ int launch_tile_sweep(const Geom &g, int dims, const float *src, float *dst, int
 
 // Multi-sweep drivers: run `iters` sweeps ping-ponging between a and b
 // starting from a; *res receives the buffer holding the final state.
-// shape_hint (block_z of the parameters): 0 = by tile fields, 1..3 = a shape.
+// shape_hint (block_z of the parameters): 0 = by tile fields, 1..6 = a shape.
 // Records kernel launches of the current dispatch (stencil_last_dispatch).
 void note_launches(const char *engine, long long n);
 bool stream3d_supported(const Geom &g);

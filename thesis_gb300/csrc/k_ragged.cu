@@ -300,7 +300,9 @@ bool ragged3d_supported(const Geom &g, int dims) {
 // have a plane each.  GB300, us a sweep in a call of 8 sweeps, a launch each /
 // persistent: R = 1 37^3 5.95 / 6.20, 45^3 6.47 / 6.22, 61^3 8.45 / 6.21; R = 2
 // 33^3 5.45 / 6.00, 37^3 6.44 / 5.95; R = 3 45^3 6.48 / 7.00, 49^3 8.52 / 7.06; R =
-// 4 33^3 6.45 / 7.98, 17 x 65 x 129 6.49 / 8.25, 61^3 9.72 / 8.09.
+// 4 33^3 6.45 / 7.98, 17 x 65 x 129 6.49 / 8.25, 61^3 9.72 / 8.09.  (On four
+// streams at once, us a sweep and grid: 49^3 R = 2 2.66 / 1.56, 101 x 99 x 97 R = 2
+// 12.3 / 6.3, but 63 x 65 x 67 R = 4 5.0 / 6.8, alone 10.4 / 6.9.)
 long long ragged3d_least_cells(int radius) {
     return radius == 1 ? 80000 : radius == 2 ? 45000 : radius == 3 ? 110000 : 150000;
 }

@@ -92,10 +92,11 @@ StreamKernel sk() {
 // per thread (more warps, fewer registers each); 3 = a 16-slot ring (more
 // planes in flight, one CTA per SM); 4 (R >= 3) = 128 x 16, one row per
 // thread, 16 consumer warps in one CTA; 5 (R <= 2) = 128 x 32, two rows per
-// thread (half the y-halo rows per output row); 7 and 8 = two rows per
-// thread, as many as 12 (R = 4) or 16 warps take with 168 and 128 registers a
-// thread, 128 (7, R >= 3) or 64 cells wide (8, R >= 2).  The persistent form
+// thread (half the y-halo rows per output row); 6 below; 7 and 8 = two rows
+// per thread, as many as 12 (R = 4) or 16 warps take with 168 and 128 registers
+// a thread, 128 (7, R >= 3) or 64 cells wide (8, R >= 2).  The persistent form
 // exists for the shapes it uses (R = 1: 3, R = 2: 5, 6 and 8, R >= 3: 4, 7 and 8).
+// Callers choose among 1 to 6 (block_z); 7 and 8 are the library's.
 StreamKernel pick(int r, int shape) {
     // shape 6: the persistent-form shape of the radius with x neighbours by
     // warp shuffles (A/B against the shared-memory reads)
@@ -187,22 +188,20 @@ int wide_shape(const Geom &g, int ctas) {
 // The shape run_stream3d sweeps with (see there) on `ctas` CTAs.
 int stream_shape(const Geom &g, int tile_x, int tile_y, int shape_hint, bool persistent, int ctas) {
     const int R = g.radius;
-    // Defaults measured fastest at 512^3 on GB300 (a launch per sweep,
-    // GCell/s): R <= 2 one row per thread with the 16-slot ring (R = 1: 701
-    // vs 634 with 8 slots and 613 with two rows per thread; R = 2: 692 vs
-    // 674 with 8 slots, 616 with 128 x 32 tiles and 581 with two rows), R >= 3
-    // one row per thread in 16 warps (R = 3: 574 vs 533 with two rows per
-    // thread; R = 4: 542 vs 531 with 8 warps and 491 with two rows).  In the
-    // persistent form R = 2 uses 128 x 32 tiles: 709 GCell/s at 512^3 with
-    // either shape, and neither wins across 96^3 to 384^3 (within 10 %
-    // either way).
+    // A launch per sweep: the fastest at 512^3 on GB300 (GCell/s): R <= 2 one
+    // row per thread with the 16-slot ring (R = 1: 701 vs 634 with 8 slots and
+    // 613 with two rows per thread; R = 2: 692 vs 674 with 8 slots, 616 with 128 x
+    // 32 tiles and 581 with two rows), R >= 3 one row per thread in 16 warps (R =
+    // 3: 574 vs 533 with two rows in 8 warps; R = 4: 542 vs 531 with 8 warps of
+    // one row and 491 with two rows).
     int shape = (!tile_x && !tile_y) ? (R <= 2 ? 3 : 4)
                                      : (tile_y == 1 ? 2 : ((tile_x && tile_x < 128) || tile_y > 16 ? 1 : 0));
     if (shape_hint >= 1 && shape_hint <= 6) shape = shape_hint;
-    // Persistent default per radius; at R = 2 on large grids (2^25 cells and
-    // up) the same shape with x neighbours by warp shuffles (GB300, same box:
-    // 512^3 694 vs 631 GCell/s, 384^3 653 vs 636; on 256^3 and smaller the
-    // shared-memory reads win: 525 vs 605 at 256^3, 258 vs 301 at 128^3).
+    // The persistent form: R = 1 as above; R = 2 from 2^25 cells on 128 x 32
+    // tiles with x neighbours by warp shuffles (GB300, same box: 512^3 694 vs 631
+    // GCell/s from shared memory, 384^3 653 vs 636; on 256^3 and smaller the
+    // shared-memory reads win: 525 vs 605 at 256^3, 258 vs 301 at 128^3); else by
+    // wide_shape.
     const bool big = (long long)g.nx * g.ny * g.nz >= (1LL << 25);
     if (persistent && !(shape_hint >= 1 && shape_hint <= 6))
         shape = R == 1 ? 3 : (R == 2 && big ? 6 : wide_shape(g, ctas));
